@@ -54,9 +54,7 @@ __host__ __device__ constexpr int min_ctas_per_sm(int bits, int mt, bool grouped
     return ring == 8 ? 2 : ((bits == 4 && grouped) ? (mt == 1 ? 3 : 2) : (mt == 1 ? AFB_DECODE_MT1_CTAS : AFB_DECODE_MT2_CTAS));
 }
 
-// ZP (int8 only): zero-points cost one more packed subtraction per pair of weights; int4 zero-points ride on the constant the
-// unpack subtracts anyway, so those instances take them without a switch.
-template <int BITS, int MT, bool GROUPED, bool ZP, int RING>
+template <int BITS, int MT, bool GROUPED, int RING>
 // resident CTAs per SM the register budget is cut for: the group-scaled int4 kernels want more registers than the others (16 rows:
 // about 118, 12 % faster with two CTAs and no spills than with three squeezed into 80; 8 rows: 80, 3 to 8 % faster with three
 // CTAs than with four at 64); the other kernels gain nothing or lose (measured)
@@ -76,9 +74,7 @@ decode_kernel(const DecodeParams p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
     const uint32_t wk_count = kWarps / p.wr;
     const uint32_t wr = warp / wk_count, wk = warp % wk_count;
-    // int8: the constant of the sign half of the unpack carries the encoding (dequant.cuh), so offset-binary storage costs no instruction
-    const uint32_t hi8 = p.enc == AFB_ENC_OFFSET_BINARY ? 0xC380C380u : 0xC300C300u;
-    const uint32_t magic4 = p.enc == AFB_ENC_OFFSET_BINARY ? 0x43004300u : 0x43084308u;
+    const uint32_t flip = BITS == 8 ? flip8(p.enc) : flip4(p.enc);
     const uint32_t groups_per_row = GROUPED ? (p.k >> p.group_shift) : 0;
     const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem) + warp * (kRing * kStageBytes) + lane * 16;
     const uint32_t act_row_bytes = p.pass_k * 2 + 16;   // +16: consecutive rows land in different bank groups
@@ -147,20 +143,19 @@ decode_kernel(const DecodeParams p) {
     const size_t sc_ia = (size_t)(ok_a ? row_a : 0) * groups_per_row, sc_ib = (size_t)(ok_b ? row_b : 0) * groups_per_row;
     uint32_t sc_k = ks + wk * CH;            // k of the chunk whose scales are fetched next
     const uint32_t sc_kstep = wk_count * CH;
-    // zero-points of this lane's two channels, as the packed-bf16 constants the unpack subtracts (dequant.cuh)
-    uint32_t z_a = 0u, z_b = 0u;                             // int8 (ZP instances): the decoded zero
-    uint32_t sub_a = 0x43084308u, sub_b = 0x43084308u;       // int4: 136 + the decoded zero
-    uint32_t z_a_nxt = 0u, z_b_nxt = 0u, sub_a_nxt = 0x43084308u, sub_b_nxt = 0x43084308u;
-    auto load_zeros = [&](size_t ia, size_t ib, uint32_t& za, uint32_t& zb, uint32_t& sa4, uint32_t& sb4) {
-        if (BITS == 8) { if (ZP) { za = zero8_const(p.zero[ia], p.enc); zb = zero8_const(p.zero[ib], p.enc); } }
-        else if (p.zero) { sa4 = zero4_const(p.zero[ia], p.enc); sb4 = zero4_const(p.zero[ib], p.enc); }
+    // the unpack's addends for this lane's two channels: they carry the zero-points (dequant.cuh)
+    uint32_t add_a = unpack_add(BITS, 0), add_b = add_a, add_a_nxt = add_a, add_b_nxt = add_a;
+    auto load_zeros = [&](size_t ia, size_t ib, uint32_t& za, uint32_t& zb) {
+        if (!p.zero) return;
+        za = unpack_add(BITS, BITS == 8 ? decode_zero8(p.zero[ia], p.enc) : decode_zero4(p.zero[ia], p.enc));
+        zb = unpack_add(BITS, BITS == 8 ? decode_zero8(p.zero[ib], p.enc) : decode_zero4(p.zero[ib], p.enc));
     };
-    if (!GROUPED) load_zeros(ok_a ? row_a : 0, ok_b ? row_b : 0, z_a, z_b, sub_a, sub_b);
-    auto load_group_scales = [&](float& sa, float& sb, uint32_t& za, uint32_t& zb, uint32_t& sa4, uint32_t& sb4) {
+    if (!GROUPED) load_zeros(ok_a ? row_a : 0, ok_b ? row_b : 0, add_a, add_b);
+    auto load_group_scales = [&](float& sa, float& sb, uint32_t& za, uint32_t& zb) {
         const uint32_t grp = sc_k >> p.group_shift;
         if (p.scale_dtype == AFB_SCALE_BF16) { sa = bf16_to_f32(sc_h[sc_ia + grp]); sb = bf16_to_f32(sc_h[sc_ib + grp]); }
         else { sa = sc_f[sc_ia + grp]; sb = sc_f[sc_ib + grp]; }
-        load_zeros(sc_ia + grp, sc_ib + grp, za, zb, sa4, sb4);
+        load_zeros(sc_ia + grp, sc_ib + grp, za, zb);
         sc_k += sc_kstep;
     };
 
@@ -171,7 +166,7 @@ decode_kernel(const DecodeParams p) {
         cp_async_commit();
     }
     float sc_a = 0.f, sc_b = 0.f, sc_a_nxt = 0.f, sc_b_nxt = 0.f;
-    if (GROUPED && my_chunks) load_group_scales(sc_a, sc_b, z_a, z_b, sub_a, sub_b);
+    if (GROUPED && my_chunks) load_group_scales(sc_a, sc_b, add_a, add_b);
     if (!dependency_met) { grid_dependency_wait(); dependency_met = true; }   // so far only B, scales and zero-points were read
 
     uint32_t i = 0;   // chunks this warp has consumed
@@ -256,16 +251,15 @@ decode_kernel(const DecodeParams p) {
             for (int j = 0; j < 4; ++j) {
                 if (BITS == 8) {
                     uint32_t a0, a1, a2, a3;
-                    s8x4_enc_to_bf16_strided(wav[j], hi8, a0, a2);
-                    s8x4_enc_to_bf16_strided(wbv[j], hi8, a1, a3);
-                    if (ZP) { a0 = bf16x2_sub(a0, z_a); a2 = bf16x2_sub(a2, z_a); a1 = bf16x2_sub(a1, z_b); a3 = bf16x2_sub(a3, z_b); }
+                    s8x4_to_bf16(wav[j], flip, kSel8Strided02, kSel8Strided13, kMulByte, add_a, a0, a2);
+                    s8x4_to_bf16(wbv[j], flip, kSel8Strided02, kSel8Strided13, kMulByte, add_b, a1, a3);
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt)
                         mma_bf16(GROUPED ? part[mt] : acc[mt], a0, a1, a2, a3, s[mt][2 * j], s[mt][2 * j + 1]);
                 } else {
                     uint32_t qa[4], qb[4];
-                    s4x8_to_bf16_strided(wav[j], magic4, qa, sub_a);
-                    s4x8_to_bf16_strided(wbv[j], magic4, qb, sub_b);
+                    s4x8_to_bf16_strided(wav[j], flip, add_a, qa);
+                    s4x8_to_bf16_strided(wbv[j], flip, add_b, qb);
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt) {
                         mma_bf16(GROUPED ? part[mt] : acc[mt], qa[0], qb[0], qa[1], qb[1], s[mt][4 * j], s[mt][4 * j + 1]);
@@ -280,7 +274,7 @@ decode_kernel(const DecodeParams p) {
                     acc[mt][2] = fmaf(sc_b, part[mt][2], acc[mt][2]); acc[mt][3] = fmaf(sc_b, part[mt][3], acc[mt][3]);
                 }
                 sc_a = sc_a_nxt; sc_b = sc_b_nxt;
-                z_a = z_a_nxt; z_b = z_b_nxt; sub_a = sub_a_nxt; sub_b = sub_b_nxt;
+                add_a = add_a_nxt; add_b = add_b_nxt;
             }
         };
         uint32_t cl = wk;
@@ -294,7 +288,7 @@ decode_kernel(const DecodeParams p) {
                 for (int u = 0; u < kRing; ++u) {
                     if (issued < my_chunks) issue_to(ring + ((u + kRing - 1) & (kRing - 1)) * kStageBytes);
                     cp_async_commit();
-                    if (GROUPED && i + 1 < my_chunks) load_group_scales(sc_a_nxt, sc_b_nxt, z_a_nxt, z_b_nxt, sub_a_nxt, sub_b_nxt);
+                    if (GROUPED && i + 1 < my_chunks) load_group_scales(sc_a_nxt, sc_b_nxt, add_a_nxt, add_b_nxt);
                     consume(ring + u * kStageBytes, chunk_off, (u & 1) ? par1 : par0);
                     ++i; chunk_off += chunk_step;
                 }
@@ -302,7 +296,7 @@ decode_kernel(const DecodeParams p) {
             } else {
                 if (issued < my_chunks) issue();
                 cp_async_commit();
-                if (GROUPED && i + 1 < my_chunks) load_group_scales(sc_a_nxt, sc_b_nxt, z_a_nxt, z_b_nxt, sub_a_nxt, sub_b_nxt);
+                if (GROUPED && i + 1 < my_chunks) load_group_scales(sc_a_nxt, sc_b_nxt, add_a_nxt, add_b_nxt);
                 consume(ring + (i & (kRing - 1)) * kStageBytes, chunk_off, BITS == 8 ? ((cl & 1u) << 5) : 0u);
                 ++i; chunk_off += chunk_step; cl += wk_count;
             }
@@ -326,9 +320,9 @@ decode_kernel(const DecodeParams p) {
     if (!dependency_met) grid_dependency_wait();
 }
 
-template <int BITS, int MT, bool GROUPED, bool ZP, int RING>
+template <int BITS, int MT, bool GROUPED, int RING>
 cudaError_t launch_one(const DecodeParams& p, dim3 grid, bool pdl, cudaStream_t s) {
-    auto kern = decode_kernel<BITS, MT, GROUPED, ZP, RING>;
+    auto kern = decode_kernel<BITS, MT, GROUPED, RING>;
     static DeviceOnce attr_set;   // per template instance
     int dev = 0;
     cudaGetDevice(&dev);
@@ -354,7 +348,7 @@ int resident_one() {
     cudaGetDevice(&dev);
     int n = cached[dev & 31].load(std::memory_order_acquire);
     if (n == 0) {
-        auto kern = decode_kernel<BITS, MT, GROUPED, false, RING>;
+        auto kern = decode_kernel<BITS, MT, GROUPED, RING>;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess) return 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kThreads, smem_bytes(MT, RING)) != cudaSuccess) return 0;
         cached[dev & 31].store(n, std::memory_order_release);
@@ -372,9 +366,7 @@ int resident_ctas(uint32_t bits, int mt, bool grouped) {   // of the 4-stage ins
 
 template <int BITS, int MT, bool GROUPED>
 cudaError_t launch_cfg(const DecodeParams& p, dim3 grid, bool deep_ring, bool pdl, cudaStream_t s) {
-    const bool zp = BITS == 8 && p.zero != nullptr;
-    if (deep_ring) return zp ? launch_one<BITS, MT, GROUPED, BITS == 8, 8>(p, grid, pdl, s) : launch_one<BITS, MT, GROUPED, false, 8>(p, grid, pdl, s);
-    return zp ? launch_one<BITS, MT, GROUPED, BITS == 8, 4>(p, grid, pdl, s) : launch_one<BITS, MT, GROUPED, false, 4>(p, grid, pdl, s);
+    return deep_ring ? launch_one<BITS, MT, GROUPED, 8>(p, grid, pdl, s) : launch_one<BITS, MT, GROUPED, 4>(p, grid, pdl, s);
 }
 
 }  // namespace

@@ -1,13 +1,16 @@
 // In-register unpack of packed int8 / int4 weights to exact bf16 pairs.
 //
 // The reference kernel splices each byte into the mantissa of 2^23 and subtracts
-// 2^23 + 128 in fp32 (bf16gemm_kernel_gfx90a.s:18-27, constants :204-210).  bf16 has an
-// 8-bit significand, so on sm_100a the same idea is done directly in packed bf16:
-//   int8:  v = (v & 0x7f) - 128 * bit7.   0x4300 | (v & 0x7f) is the bf16 128 + (v & 0x7f)
-//          and 0xC300 | (v & 0x80) is the bf16 -128 (bit7 = 0) or -256 (bit7 = 1); their
-//          bf16 sum is the exact integer v.  Two weights per 32-bit lane operation.
-//   int4:  0x4300 | (q ^ 8) is the bf16 128 + (q + 8); subtracting 136 gives q exactly.
-// All results are integers of magnitude <= 128, exactly representable in bf16.
+// 2^23 + 128 in fp32 (bf16gemm_kernel_gfx90a.s:18-27, constants :204-210).  Here the splice costs nothing: a bf16 whose upper
+// byte is zero is its lower byte times 2^-133 (denormals, and up to 255 the binade above them, have the same step), so an
+// unsigned weight u merely zero-extended to 16 bits already IS the bf16 u * 2^-133, and ONE packed fused multiply-add,
+//     fma(u * 2^-133, 2^127, -(128 + zero) * 2^-6)  =  (u - 128 - zero) * 2^-6,
+// makes two exact weights of it (both operands and the result have at most 8 significant bits).  An int4 weight in the upper
+// half of a byte is 16 u * 2^-133 and takes 2^123.  Zero-points and the storage encoding live in the constants.
+// Every routine returns the weights times kUnpackFactor = 2^-6; the kernels multiply the finished fp32 sums by 64 (powers of
+// two: no bit of a result depends on it).  Cost per 4 int8 weights: 1 xor + 2 permutes + 2 fma (splice, sign and add: 8 in natural
+// order, 7 strided); per 8 int4 weights 10 in natural order, 9 strided (13, 11).  The unpack is what the decode kernels and the
+// converter warps of the prefill kernels issue most; see the figures there.
 #pragma once
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -20,26 +23,10 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
     return d;
 }
-// (a & b) | c
-__device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
 // (a & b) ^ c
 __device__ __forceinline__ uint32_t lop3_and_xor(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
     asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-__device__ __forceinline__ uint32_t bf16x2_add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-__device__ __forceinline__ uint32_t bf16x2_sub(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
 __device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
@@ -54,87 +41,104 @@ __device__ __forceinline__ uint32_t bf16x2_fma(uint32_t a, uint32_t b, uint32_t 
     return d;
 }
 
-// x holds two two's-complement int8 values in bits [0,8) and [16,24) (other bits ignored).
-// Returns the two exact bf16 values, low half = the value from bits [0,8).
-__device__ __forceinline__ uint32_t s8pair_to_bf16x2(uint32_t x) {
-    const uint32_t lo = lop3_and_or(x, 0x007f007fu, 0x43004300u);  // 128 + (v & 0x7f)
-    const uint32_t hi = lop3_and_or(x, 0x00800080u, 0xC300C300u);  // -128 - 128 * bit7
-    return bf16x2_add(lo, hi);
-}
+// What the unpack adds and multiplies.  kUnpackFactor * 64 = 1.
+constexpr float kUnpackInverse = 64.f;
+constexpr uint32_t kMulByte = 0x7F007F00u;       // 2^127 in both halves: weights in the low bits of their byte
+constexpr uint32_t kMulHighNibble = 0x7D007D00u; // 2^123: weights in bits [4,8) of their byte
+constexpr uint32_t kMulNibblePair = 0x7D007F00u; // low half from bits [0,4), high half from bits [4,8)
 
-// Four consecutive int8 (two's complement) of word w -> {k0,k1} and {k2,k3} as bf16x2.
-__device__ __forceinline__ void s8x4_to_bf16_natural(uint32_t w, uint32_t& p01, uint32_t& p23) {
-    p01 = s8pair_to_bf16x2(prmt(w, 0u, 0x4140u));
-    p23 = s8pair_to_bf16x2(prmt(w, 0u, 0x4342u));
-}
-// Same bytes, cheaper pairing: {k0,k2} and {k1,k3} (the consumer permutes its other operand).
-__device__ __forceinline__ void s8x4_to_bf16_strided(uint32_t w, uint32_t& p02, uint32_t& p13) {
-    p02 = s8pair_to_bf16x2(w);
-    p13 = s8pair_to_bf16x2(w >> 8);
-}
+// Stored integers to unsigned ones (value + 128 / value + 8): one xor per word, nothing to flip when they are stored that way.
+__host__ __device__ __forceinline__ uint32_t flip8(uint32_t enc) { return enc == AFB_ENC_OFFSET_BINARY ? 0u : 0x80808080u; }
+__host__ __device__ __forceinline__ uint32_t flip4(uint32_t enc) { return enc == AFB_ENC_OFFSET_BINARY ? 0u : 0x88888888u; }
 
-// The same for either storage encoding without a separate flip: `hi` = 0xC300C300 (two's complement) or 0xC380C380 (value + 128).
-// With value + 128 the top bit is inverted, so the sign half is -256 + 128 * bit7 = the bf16 pattern 0xC380 with bit 7 toggled off.
-__device__ __forceinline__ uint32_t s8pair_enc_to_bf16x2(uint32_t x, uint32_t hi) {
-    const uint32_t lo = lop3_and_or(x, 0x007f007fu, 0x43004300u);   // 128 + (v & 0x7f)
-    return bf16x2_add(lo, lop3_and_xor(x, 0x00800080u, hi));         // two's complement: -128 - 128 * bit7; offset: -256 + 128 * bit7
-}
-__device__ __forceinline__ void s8x4_enc_to_bf16_strided(uint32_t w, uint32_t hi, uint32_t& p02, uint32_t& p13) {
-    p02 = s8pair_enc_to_bf16x2(w, hi);
-    p13 = s8pair_enc_to_bf16x2(w >> 8, hi);
-}
+__device__ __forceinline__ uint32_t bf16_dup(uint16_t s) { return (uint32_t)s * 0x00010001u; }
+__device__ __forceinline__ uint32_t bf16_dup_rn(float v) { return bf16_dup(__bfloat16_as_ushort(__float2bfloat16_rn(v))); }
 
-// magic = 0x43084308 for two's-complement nibbles, 0x43004300 for offset-binary (+8) nibbles.
-// x holds two nibbles in bits [0,4) and [16,20) (other bits ignored) -> two exact bf16.
-// `sub` is the packed-bf16 constant that is subtracted: 136 without zero-points, 136 + zero with them (the same instruction).
-__device__ __forceinline__ uint32_t s4pair_to_bf16x2(uint32_t x, uint32_t magic, uint32_t sub = 0x43084308u) {
-    return bf16x2_sub(lop3_and_xor(x, 0x000f000fu, magic), sub);
-}
-// Eight consecutive nibbles of w (k0 in bits [0,4)) -> {k0,k1},{k2,k3},{k4,k5},{k6,k7}.
-__device__ __forceinline__ void s4x8_to_bf16_natural(uint32_t w, uint32_t magic, uint32_t p[4], uint32_t sub = 0x43084308u) {
-    const uint32_t sh = w >> 4;
-    p[0] = s4pair_to_bf16x2(prmt(w, sh, 0x0400u), magic, sub);
-    p[1] = s4pair_to_bf16x2(prmt(w, sh, 0x0501u), magic, sub);
-    p[2] = s4pair_to_bf16x2(prmt(w, sh, 0x0602u), magic, sub);
-    p[3] = s4pair_to_bf16x2(prmt(w, sh, 0x0703u), magic, sub);
-}
-// Cheaper pairing: {k0,k4},{k1,k5},{k2,k6},{k3,k7}.
-__device__ __forceinline__ void s4x8_to_bf16_strided(uint32_t w, uint32_t magic, uint32_t p[4], uint32_t sub = 0x43084308u) {
-    p[0] = s4pair_to_bf16x2(w, magic, sub);
-    p[1] = s4pair_to_bf16x2(w >> 4, magic, sub);
-    p[2] = s4pair_to_bf16x2(w >> 8, magic, sub);
-    p[3] = s4pair_to_bf16x2(w >> 12, magic, sub);
-}
-
-// Consecutive-k pairs {k0,k1},{k2,k3} of a word, whichever way the word is laid out: plain [k0,k1,k2,k3] needs two byte
-// permutes, the pre-packed order [k0,k2,k1,k3] (afb_prepack) is what the cheap routine reads as pairs.
-__device__ __forceinline__ void s8x4_to_bf16_pairs(uint32_t w, bool packed, uint32_t& p01, uint32_t& p23) {
-    if (packed) s8x4_to_bf16_strided(w, p01, p23);
-    else s8x4_to_bf16_natural(w, p01, p23);
-}
-__device__ __forceinline__ void s4x8_to_bf16_pairs(uint32_t w, uint32_t magic, bool packed, uint32_t p[4], uint32_t sub = 0x43084308u) {
-    if (packed) s4x8_to_bf16_strided(w, magic, p, sub);
-    else s4x8_to_bf16_natural(w, magic, p, sub);
-}
-// Zero-points: a byte in the weights' own encoding -> the packed-bf16 constant the unpack subtracts.
-//   int8: the decoded zero itself, both halves (one extra sub.bf16x2 per pair; |q - z| <= 255 is exact in bf16);
-//   int4: 136 + decoded zero, which takes the place of the 136 the unpack subtracts anyway (no extra instruction).
-__device__ __forceinline__ uint32_t zero8_const(uint32_t zbyte, uint32_t enc) {
-    const int z = enc == AFB_ENC_OFFSET_BINARY ? (int)zbyte - 128 : (int)(int8_t)zbyte;
-    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn((float)z)) * 0x00010001u;
-}
-__device__ __forceinline__ uint32_t zero4_const(uint32_t zbyte, uint32_t enc) {
+// The addend for a zero-point byte in the weights' own encoding (without zero-points: the byte that decodes to 0).
+__device__ __forceinline__ int decode_zero8(uint32_t zbyte, uint32_t enc) { return enc == AFB_ENC_OFFSET_BINARY ? (int)zbyte - 128 : (int)(int8_t)zbyte; }
+__device__ __forceinline__ int decode_zero4(uint32_t zbyte, uint32_t enc) {
     const int nib = (int)(zbyte & 0xFu);
-    const int z = enc == AFB_ENC_OFFSET_BINARY ? nib - 8 : ((nib ^ 8) - 8);
-    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn((float)(136 + z))) * 0x00010001u;
+    return enc == AFB_ENC_OFFSET_BINARY ? nib - 8 : ((nib ^ 8) - 8);
 }
+__device__ __forceinline__ uint32_t unpack_add(int bits, int zero) { return bf16_dup_rn((float)(-(bits == 8 ? 128 : 8) - zero) * 0.015625f); }
+
+// Two of the four bytes of `t` (flipped to unsigned) as bf16 pairs; the selectors say which: {k0,k1},{k2,k3} of a plain word, or
+// {b0,b2},{b1,b3}: the pre-packed order [k0,k2,k1,k3] read as consecutive k, or a plain word in strided pairs.
+constexpr uint32_t kSel8Natural01 = 0x4140u, kSel8Natural23 = 0x4342u, kSel8Strided02 = 0x4240u, kSel8Strided13 = 0x4341u;
+__device__ __forceinline__ void s8x4_to_bf16(uint32_t w, uint32_t flip, uint32_t sel0, uint32_t sel1, uint32_t mul, uint32_t add, uint32_t& p0, uint32_t& p1) {
+    const uint32_t t = w ^ flip;
+    p0 = bf16x2_fma(prmt(t, 0u, sel0), mul, add);
+    p1 = bf16x2_fma(prmt(t, 0u, sel1), mul, add);
+}
+
+// Eight nibbles of w in strided pairs: {n0,n4},{n1,n5},{n2,n6},{n3,n7} (consecutive k of a pre-packed word).
+__device__ __forceinline__ void s4x8_to_bf16_strided(uint32_t w, uint32_t flip, uint32_t add, uint32_t p[4]) {
+    const uint32_t h = w >> 8;
+    p[0] = bf16x2_fma(lop3_and_xor(w, 0x000f000fu, flip & 0x000f000fu), kMulByte, add);
+    p[1] = bf16x2_fma(lop3_and_xor(w, 0x00f000f0u, flip & 0x00f000f0u), kMulHighNibble, add);
+    p[2] = bf16x2_fma(lop3_and_xor(h, 0x000f000fu, flip & 0x000f000fu), kMulByte, add);
+    p[3] = bf16x2_fma(lop3_and_xor(h, 0x00f000f0u, flip & 0x00f000f0u), kMulHighNibble, add);
+}
+// Eight nibbles of w in either order, chosen by the constants of Nibbles: even nibbles and odd nibbles are masked out of the word
+// once each (odd ones stay in the upper half of their bytes) and a permute pairs the bytes; its sign-replicating selectors supply
+// the zero bytes (an even nibble's byte never has its top bit set).
+struct Nibbles { uint32_t sel[4], mul[2]; };
+__device__ __forceinline__ Nibbles nibbles(bool packed) {
+    Nibbles q;
+    q.sel[0] = packed ? 0x8280u : 0x8480u;   // {n0,n4} / {n0,n1}
+    q.sel[1] = packed ? 0x8684u : 0x9591u;   // {n1,n5} / {n2,n3}
+    q.sel[2] = packed ? 0x8381u : 0xA6A2u;   // {n2,n6} / {n4,n5}
+    q.sel[3] = packed ? 0x8785u : 0xB7B3u;   // {n3,n7} / {n6,n7}
+    q.mul[0] = packed ? kMulByte : kMulNibblePair;         // of pairs 0 and 2
+    q.mul[1] = packed ? kMulHighNibble : kMulNibblePair;   // of pairs 1 and 3
+    return q;
+}
+__device__ __forceinline__ void s4x8_to_bf16(uint32_t w, uint32_t flip, const Nibbles& q, uint32_t mul0, uint32_t mul1, uint32_t add, uint32_t p[4]) {
+    const uint32_t e = lop3_and_xor(w, 0x0f0f0f0fu, flip & 0x0f0f0f0fu), o = lop3_and_xor(w, 0xf0f0f0f0u, flip & 0xf0f0f0f0u);
+    p[0] = bf16x2_fma(prmt(e, o, q.sel[0]), mul0, add);
+    p[1] = bf16x2_fma(prmt(e, o, q.sel[1]), mul1, add);
+    p[2] = bf16x2_fma(prmt(e, o, q.sel[2]), mul0, add);
+    p[3] = bf16x2_fma(prmt(e, o, q.sel[3]), mul1, add);
+}
+
+// Group scales on weights that go to the tensor cores as bf16_rn(q * scale): the scale rides on the same multiply-add,
+//     fma(u * 2^-133, scale * 2^123, -128 * scale * 2^-10)  =  bf16_rn((u - 128) * scale) * 2^-10,
+// one rounding of the exact product, as a separate multiplication of the exact weight would round it.  Needs both constants to be
+// exact: 2^-100 < scale < 16 (or 0) and no zero-point ((128 + zero) * scale can have 16 significant bits); negative scales stay out
+// so that a zero weight keeps the sign that the product gives it.  Otherwise the weight
+// is unpacked as above and multiplied by scale * 2^-4, with the same factor of 2^-10 in the result.
+constexpr float kGroupInverse = 1024.f;
+struct GroupUnpack {
+    uint32_t mul0, mul1;   // multipliers of the unpack (int8 uses mul0)
+    uint32_t add;
+    uint32_t scale;        // scale * 2^-4 in both halves: second step when not folded, and the two-term mode
+};
+__device__ __forceinline__ bool group_folds(uint16_t s, bool has_zero) {
+    const float f = __uint_as_float((uint32_t)s << 16);
+    return !has_zero && ((f < 16.f && f > 7.9e-31f) || s == 0);
+}
+__device__ __forceinline__ GroupUnpack group_unpack(int bits, uint16_t s, int zero, bool folded, const Nibbles& q) {
+    const float f = __uint_as_float((uint32_t)s << 16);
+    GroupUnpack u;
+    u.scale = bf16_dup_rn(f * 0.0625f);
+    u.mul0 = bits == 8 ? kMulByte : q.mul[0];
+    u.mul1 = bits == 8 ? kMulByte : q.mul[1];
+    if (folded) {   // the multipliers above divided by 16, times the scale
+        const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16_rn(f * 0x1p123f)), hi = __bfloat16_as_ushort(__float2bfloat16_rn(f * 0x1p119f));
+        u.mul0 = ((u.mul0 & 0xffffu) == 0x7F00u ? lo : hi) | ((u.mul0 >> 16) == 0x7F00u ? lo : hi) << 16;
+        u.mul1 = ((u.mul1 & 0xffffu) == 0x7F00u ? lo : hi) | ((u.mul1 >> 16) == 0x7F00u ? lo : hi) << 16;
+        u.add = bf16_dup_rn(f * (bits == 8 ? -0.125f : -0.0078125f));   // -128 * 2^-10, -8 * 2^-10
+    } else {
+        u.add = unpack_add(bits, zero);
+    }
+    return u;
+}
+
 // Place of weight k inside its word in the pre-packed layout (int8: bytes [k0,k2,k1,k3]; int4: nibbles [k0,k2,k4,k6,k1,k3,k5,k7]).
 __host__ __device__ __forceinline__ uint32_t packed_pos(uint32_t bits, uint32_t k) {
     if (bits == 8) { const uint32_t i = k & 3u; return (k & ~3u) | ((i >> 1) | ((i & 1u) << 1)); }
     const uint32_t i = k & 7u;
     return (k & ~7u) | ((i >> 1) | ((i & 1u) << 2));
 }
-
-__device__ __forceinline__ uint32_t bf16_dup(uint16_t s) { return (uint32_t)s * 0x00010001u; }
 
 }  // namespace afb

@@ -124,9 +124,12 @@ int launch_naive(const afb_gemm_args& a, DeviceCtx*, cudaStream_t s) {
 // ---------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) dequant_dump_kernel(afb_gemm_args a, uint16_t* __restrict__ out) {
     const uint8_t* __restrict__ pb = reinterpret_cast<const uint8_t*>(a.ptr_b);
-    const uint32_t xormask = a.b_encoding == AFB_ENC_OFFSET_BINARY ? 0x80808080u : 0u;
-    const uint32_t magic4 = a.b_encoding == AFB_ENC_OFFSET_BINARY ? 0x43004300u : 0x43084308u;
+    const int bits = (int)a.b_bits;
     const bool packed = a.b_layout == AFB_LAYOUT_COL_PACKED;
+    const uint32_t flip = bits == 8 ? flip8(a.b_encoding) : flip4(a.b_encoding);
+    const uint32_t sel0 = packed ? kSel8Strided02 : kSel8Natural01, sel1 = packed ? kSel8Strided13 : kSel8Natural23;
+    const Nibbles nib = nibbles(packed);
+    const uint32_t unscale = bf16_dup_rn(kUnpackInverse), unscale_group = bf16_dup_rn(kGroupInverse);   // the unpack's factor, exact
     if (a.b_layout != AFB_LAYOUT_ROW) {
         const uint32_t per16 = a.b_bits == 8 ? 16u : 32u;  // weights per 16-byte piece
         const uint32_t pieces_per_row = a.k / per16;
@@ -141,16 +144,20 @@ __global__ void __launch_bounds__(256) dequant_dump_kernel(afb_gemm_args a, uint
             const uint8_t* pz = reinterpret_cast<const uint8_t*>(a.ptr_zero);
             const uint32_t zb = pz ? pz[a.group_size ? (size_t)n * groups + k0 / a.group_size : n] : 0u;
             const bool has_zero = pz != nullptr;
-            const uint32_t z8 = zero8_const(has_zero ? zb : (a.b_encoding == AFB_ENC_OFFSET_BINARY ? 128u : 0u), a.b_encoding);
-            const uint32_t sub4 = has_zero ? zero4_const(zb, a.b_encoding) : 0x43084308u;
-            uint32_t sc = 0;
+            const int zero = !has_zero ? 0 : (bits == 8 ? decode_zero8(zb, a.b_encoding) : decode_zero4(zb, a.b_encoding));
+            GroupUnpack up;
+            up.mul0 = bits == 8 ? kMulByte : nib.mul[0]; up.mul1 = nib.mul[1]; up.add = unpack_add(bits, zero); up.scale = unscale;
+            bool multiply = true;   // by up.scale: the group scale, or nothing but the inverse factor
             if (a.group_size) {
                 // a 16-byte piece never straddles a group (group_size is a multiple of 32)
                 const size_t si = (size_t)n * groups + k0 / a.group_size;
                 uint16_t sb;
                 if (a.scale_dtype == AFB_SCALE_BF16) sb = reinterpret_cast<const uint16_t*>(a.ptr_scale)[si];
                 else sb = __bfloat16_as_ushort(__float2bfloat16_rn(reinterpret_cast<const float*>(a.ptr_scale)[si]));
-                sc = bf16_dup(sb);
+                if (!((a.flags & AFB_FLAG_DUMP_DECODE_PAIRING) && !packed)) {
+                    multiply = !group_folds(sb, has_zero);
+                    up = group_unpack(bits, sb, zero, !multiply, nib);
+                }
             }
             uint32_t* o = reinterpret_cast<uint32_t*>(out + (size_t)n * a.k + k0);
             if ((a.flags & AFB_FLAG_DUMP_DECODE_PAIRING) && !packed) {
@@ -161,13 +168,15 @@ __global__ void __launch_bounds__(256) dequant_dump_kernel(afb_gemm_args a, uint
                 for (int j = 0; j < 4; ++j) {
                     if (a.b_bits == 8) {
                         uint32_t p02, p13;
-                        s8x4_to_bf16_strided(w[j] ^ xormask, p02, p13);
-                        if (has_zero) { p02 = bf16x2_sub(p02, z8); p13 = bf16x2_sub(p13, z8); }
+                        s8x4_to_bf16(w[j], flip, kSel8Strided02, kSel8Strided13, kMulByte, up.add, p02, p13);
+                        p02 = bf16x2_mul(p02, unscale); p13 = bf16x2_mul(p13, unscale);
                         o16[4 * j + 0] = (uint16_t)(p02 & 0xffff); o16[4 * j + 2] = (uint16_t)(p02 >> 16);
                         o16[4 * j + 1] = (uint16_t)(p13 & 0xffff); o16[4 * j + 3] = (uint16_t)(p13 >> 16);
                     } else {
                         uint32_t p[4];
-                        s4x8_to_bf16_strided(w[j], magic4, p, sub4);
+                        s4x8_to_bf16_strided(w[j], flip, up.add, p);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) p[i] = bf16x2_mul(p[i], unscale);
 #pragma unroll
                         for (int i = 0; i < 4; ++i) { o16[8 * j + i] = (uint16_t)(p[i] & 0xffff); o16[8 * j + 4 + i] = (uint16_t)(p[i] >> 16); }
                     }
@@ -178,18 +187,21 @@ __global__ void __launch_bounds__(256) dequant_dump_kernel(afb_gemm_args a, uint
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     uint32_t p01, p23;
-                    s8x4_to_bf16_pairs(w[j] ^ xormask, packed, p01, p23);
-                    if (has_zero) { p01 = bf16x2_sub(p01, z8); p23 = bf16x2_sub(p23, z8); }
-                    if (a.group_size) { p01 = bf16x2_mul(p01, sc); p23 = bf16x2_mul(p23, sc); }
+                    s8x4_to_bf16(w[j], flip, sel0, sel1, up.mul0, up.add, p01, p23);
+                    if (multiply) { p01 = bf16x2_mul(p01, up.scale); p23 = bf16x2_mul(p23, up.scale); }
+                    if (a.group_size) { p01 = bf16x2_mul(p01, unscale_group); p23 = bf16x2_mul(p23, unscale_group); }
                     o[2 * j] = p01; o[2 * j + 1] = p23;
                 }
             } else {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     uint32_t p[4];
-                    s4x8_to_bf16_pairs(w[j], magic4, packed, p, sub4);
+                    s4x8_to_bf16(w[j], flip, nib, up.mul0, up.mul1, up.add, p);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) o[4 * j + i] = a.group_size ? bf16x2_mul(p[i], sc) : p[i];
+                    for (int i = 0; i < 4; ++i) {
+                        if (multiply) p[i] = bf16x2_mul(p[i], up.scale);
+                        o[4 * j + i] = a.group_size ? bf16x2_mul(p[i], unscale_group) : p[i];
+                    }
                 }
             }
         }
@@ -201,9 +213,10 @@ __global__ void __launch_bounds__(256) dequant_dump_kernel(afb_gemm_args a, uint
         for (size_t id = blockIdx.x * (size_t)blockDim.x + threadIdx.x; id < total; id += (size_t)gridDim.x * blockDim.x) {
             const uint32_t k = (uint32_t)(id / n4);
             const uint32_t n0 = (uint32_t)(id % n4) * 4;
-            const uint32_t w = *reinterpret_cast<const uint32_t*>(pb + (size_t)k * a.ldb + n0) ^ xormask;
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(pb + (size_t)k * a.ldb + n0);
             uint32_t p02, p13;
-            s8x4_to_bf16_strided(w, p02, p13);
+            s8x4_to_bf16(w, flip, kSel8Strided02, kSel8Strided13, kMulByte, unpack_add(8, 0), p02, p13);
+            p02 = bf16x2_mul(p02, unscale); p13 = bf16x2_mul(p13, unscale);
             uint16_t v[4] = {(uint16_t)(p02 & 0xffff), (uint16_t)(p13 & 0xffff), (uint16_t)(p02 >> 16), (uint16_t)(p13 >> 16)};
 #pragma unroll
             for (int i = 0; i < 4; ++i) out[(size_t)k * a.n + n0 + i] = v[i];

@@ -224,7 +224,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                                 float sc[8];
                                 load_scale8(p.scale, p.scale_dtype, col, sc);  // same address in all lanes: one broadcast
 #pragma unroll
-                                for (int e = 0; e < 8; ++e) v[e] *= sc[e];
+                                for (int e = 0; e < 8; ++e) v[e] *= kUnpackInverse * sc[e];
+                            } else {
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) v[e] *= kUnpackInverse;
                             }
                             if (p.c_f32) {
                                 *reinterpret_cast<float4*>(crow32 + ch * 32 + q * 8) = make_float4(v[0], v[1], v[2], v[3]);
@@ -251,8 +254,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         const int cid = threadIdx.x - kFirstConvWarp * 32;   // 0..511
         constexpr int kPiecesPerRow = L::kRawRowBytes / 16;   // 4 (int8) or 2 (int4)
         constexpr int kItems = (BN * kPiecesPerRow + kConvWarps * 32 - 1) / (kConvWarps * 32);   // the last item may be empty for some threads
-        const uint32_t xormask = (BITS == 8 && p.enc == AFB_ENC_OFFSET_BINARY) ? 0x80808080u : 0u;
-        const uint32_t magic4 = p.enc == AFB_ENC_OFFSET_BINARY ? 0x43004300u : 0x43084308u;
+        const uint32_t flip = BITS == 8 ? flip8(p.enc) : flip4(p.enc), add = unpack_add(BITS, 0);
+        const uint32_t sel0 = p.packed ? kSel8Strided02 : kSel8Natural01, sel1 = p.packed ? kSel8Strided13 : kSel8Natural23;
+        const Nibbles nib = nibbles(p.packed != 0);
         const uint32_t groups_per_row = GROUPED ? p.k / p.group : 0;
         const uint32_t kb_per_group = GROUPED ? p.group / BK : 1;
         uint32_t sa = 0, pa = 0, sb = 0, pb = 0;
@@ -295,7 +299,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                         uint32_t o[8];
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            s8x4_to_bf16_pairs(w[j] ^ xormask, p.packed != 0, o[2 * j], o[2 * j + 1]);
+                            s8x4_to_bf16(w[j], flip, sel0, sel1, kMulByte, add, o[2 * j], o[2 * j + 1]);
                             if (GROUPED) { o[2 * j] = bf16x2_mul(o[2 * j], sc_cur[itx]); o[2 * j + 1] = bf16x2_mul(o[2 * j + 1], sc_cur[itx]); }
                         }
                         *reinterpret_cast<uint4*>(orow + (((2 * piece) ^ sw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -304,7 +308,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             uint32_t q[4];
-                            s4x8_to_bf16_pairs(w[j], magic4, p.packed != 0, q);
+                            s4x8_to_bf16(w[j], flip, nib, nib.mul[0], nib.mul[1], add, q);
                             if (GROUPED) {
 #pragma unroll
                                 for (int e = 0; e < 4; ++e) q[e] = bf16x2_mul(q[e], sc_cur[itx]);

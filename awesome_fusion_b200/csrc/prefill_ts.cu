@@ -279,9 +279,9 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
         const uint32_t q = (uint32_t)(warp & 3);             // TMEM lane quarter this warp may touch
         const uint32_t kq = (uint32_t)(warp - 2) >> 2;        // which part of the 64-wide K step / which part of the columns
         const uint32_t ch = q * 32 + lane;                    // channel (TMEM lane) of this thread inside the tile
-        const uint32_t xormask = (BITS == 8 && p.enc == AFB_ENC_OFFSET_BINARY) ? 0x80808080u : 0u;
-        const uint32_t magic4 = p.enc == AFB_ENC_OFFSET_BINARY ? 0x43004300u : 0x43084308u;
-        const bool packed = p.packed != 0;
+        const uint32_t flip = BITS == 8 ? flip8(p.enc) : flip4(p.enc);
+        const uint32_t sel0 = p.packed ? kSel8Strided02 : kSel8Natural01, sel1 = p.packed ? kSel8Strided13 : kSel8Natural23;
+        const Nibbles nib = nibbles(p.packed != 0);
         const uint32_t groups_per_row = GROUPED ? p.k / p.group : 0;
         const bool has_zero = p.zero != nullptr;
         // raw tile in shared memory: rows of 64 (int8) / 32 (int4) bytes, stored by TMA with the 64- / 32-byte swizzle
@@ -339,26 +339,34 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
             auto load_group = [&](uint32_t gidx, uint32_t& sc, uint32_t& zb) {
                 sc = 0; zb = 0;
                 if (nn >= p.n || gidx >= groups_per_row) return;
-                sc = bf16_dup(reinterpret_cast<const uint16_t*>(p.scale)[(size_t)nn * groups_per_row + gidx]);
+                sc = reinterpret_cast<const uint16_t*>(p.scale)[(size_t)nn * groups_per_row + gidx];
                 if (has_zero) zb = p.zero[(size_t)nn * groups_per_row + gidx];
             };
             uint32_t kpos = w.kb0 * BK + kq * kKPer;            // first k this thread converts in the coming step
             const uint32_t gstep = (GROUPED && p.group < (uint32_t)BK) ? BK / p.group : 1u;   // groups a 64-wide step advances by (2 for groups of 32)
             uint32_t gcur = GROUPED ? kpos / p.group : 0, gend = GROUPED ? (gcur + 1) * p.group : 0xffffffffu;
-            uint32_t z8 = 0u, sub4 = 0x43084308u;               // zero-point constants of the unpack (dequant.cuh)
+            // constants of the unpack (dequant.cuh): the zero-point, and with group scales the scale as well where it can be folded in
+            auto zero_of = [&](uint32_t zb) { return !has_zero ? 0 : (BITS == 8 ? decode_zero8(zb, p.enc) : decode_zero4(zb, p.enc)); };
+            GroupUnpack up;
+            bool folded = false;
+            auto set_group = [&] {
+                folded = __all_sync(0xffffffffu, group_folds((uint16_t)sc_cur, has_zero)) && !p.exact;
+                up = group_unpack(BITS, (uint16_t)sc_cur, zero_of(zb_cur), folded, nib);
+            };
             if (GROUPED) {
                 load_group(gcur, sc_cur, zb_cur);
                 load_group(gcur + gstep, sc_nxt, zb_nxt);
-            } else if (has_zero && nn < p.n) {
-                zb_cur = p.zero[nn];
+                set_group();
+            } else {
+                if (has_zero && nn < p.n) zb_cur = p.zero[nn];
+                up.mul0 = BITS == 8 ? kMulByte : nib.mul[0]; up.mul1 = nib.mul[1]; up.add = unpack_add(BITS, zero_of(zb_cur)); up.scale = 0;
             }
-            if (has_zero) { if (BITS == 8) z8 = zero8_const(zb_cur, p.enc); else sub4 = zero4_const(zb_cur, p.enc); }
             for (uint32_t kb = w.kb0; kb < w.kb1; ++kb, kpos += BK) {
                 if (GROUPED && kpos >= gend) {
                     gcur += gstep; gend += gstep * p.group;
                     sc_cur = sc_nxt; zb_cur = zb_nxt;
                     load_group(gcur + gstep, sc_nxt, zb_nxt);
-                    if (has_zero) { if (BITS == 8) z8 = zero8_const(zb_cur, p.enc); else sub4 = zero4_const(zb_cur, p.enc); }
+                    set_group();
                 }
                 const bool two_terms = GROUPED && p.exact;
                 if (!wait_or_abort(bar_full(st), ph, abort_flag) || !wait_or_abort(bar_empty_a(sa), pa ^ 1u, abort_flag) ||
@@ -384,11 +392,10 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
 #pragma unroll
                 for (int j = 0; j < kWords; ++j) {
                     if (BITS == 8) {
-                        s8x4_to_bf16_pairs(w[j] ^ xormask, packed, o[2 * j], o[2 * j + 1]);
-                        if (has_zero) { o[2 * j] = bf16x2_sub(o[2 * j], z8); o[2 * j + 1] = bf16x2_sub(o[2 * j + 1], z8); }
+                        s8x4_to_bf16(w[j], flip, sel0, sel1, up.mul0, up.add, o[2 * j], o[2 * j + 1]);
                     } else {
                         uint32_t qv[4];
-                        s4x8_to_bf16_pairs(w[j], magic4, packed, qv, sub4);
+                        s4x8_to_bf16(w[j], flip, nib, up.mul0, up.mul1, up.add, qv);
                         o[4 * j] = qv[0]; o[4 * j + 1] = qv[1]; o[4 * j + 2] = qv[2]; o[4 * j + 3] = qv[3];
                     }
                 }
@@ -397,14 +404,14 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
                     uint32_t lo[kOut];
 #pragma unroll
                     for (int j = 0; j < kOut; ++j) {
-                        const uint32_t hi = bf16x2_mul(o[j], sc_cur);
-                        lo[j] = bf16x2_fma(o[j], sc_cur, hi ^ 0x80008000u);   // q * s - hi: the fused product is exact, the difference fits bf16
+                        const uint32_t hi = bf16x2_mul(o[j], up.scale);
+                        lo[j] = bf16x2_fma(o[j], up.scale, hi ^ 0x80008000u);   // q * s - hi: the fused product is exact, the difference fits bf16
                         o[j] = hi;
                     }
                     ptx::tmem_st_cols(taddr + 32, lo);
-                } else if (GROUPED) {
+                } else if (GROUPED && !folded) {
 #pragma unroll
-                    for (int j = 0; j < kOut; ++j) o[j] = bf16x2_mul(o[j], sc_cur);
+                    for (int j = 0; j < kOut; ++j) o[j] = bf16x2_mul(o[j], up.scale);
                 }
                 ptx::tmem_st_cols(taddr, o);
                 ptx::tmem_st_wait();
@@ -427,10 +434,10 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
             }
             ptx::tc_fence_after_sync();
             count_pending();   // the previous tile of this CTA (pipelined reduce-scatter only)
-            float scale = 1.f;
+            float scale = GROUPED ? kGroupInverse : 0.f;
             if (!GROUPED && nn < p.n)
-                scale = p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn] << 16)
-                                                       : reinterpret_cast<const float*>(p.scale)[nn];
+                scale = kUnpackInverse * (p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn] << 16)
+                                                       : reinterpret_cast<const float*>(p.scale)[nn]);
             if (p.push_on == 2 && !wait_or_abort(bar_tile_fwd, (it & 1u) ^ 1u, abort_flag)) {   // the previous tile has left
                 if (!*abort_flag) { report_timeout(p.status, 26, (int)t, -1); *abort_flag = 1; }
                 break;
@@ -533,13 +540,13 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
                     __threadfence();
                     const uint32_t tid = threadIdx.x - 64;                  // 0 .. 255 over the converter warps
                     const uint32_t c4 = tid & 31u, nv = n0 + c4 * 4;        // this thread's four channels (the same in every row)
-                    float sc4[4] = {1.f, 1.f, 1.f, 1.f};
+                    float sc4[4] = {kGroupInverse, kGroupInverse, kGroupInverse, kGroupInverse};
                     if (!GROUPED) {
 #pragma unroll
                         for (int e = 0; e < 4; ++e)
                             if (nv + e < p.n)
-                                sc4[e] = p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nv + e] << 16)
-                                                                         : reinterpret_cast<const float*>(p.scale)[nv + e];
+                                sc4[e] = kUnpackInverse * (p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nv + e] << 16)
+                                                                         : reinterpret_cast<const float*>(p.scale)[nv + e]);
                     }
                     const float* wst = p.tail_ws + (size_t)w.tail_r * p.tail_parts * BMA * BNW;
                     constexpr uint32_t kVecs = BMA * (BNW / 4), kMaxParts = 4, kU = 4;

@@ -66,6 +66,27 @@ def test_dequant_groups_and_int4(afb, oracle, bits, group, enc, scale_dtype):
     assert np.array_equal(got, oracle.dequant_bf16(case))
 
 
+@pytest.mark.parametrize("bits,enc", [(8, 0), (4, 0), (4, 1)])
+@pytest.mark.parametrize("factor", [1.0, 4096.0, -1.0, 2.0 ** -105])
+def test_group_scales_on_both_sides_of_the_folding_limits(afb, oracle, bits, enc, factor):
+    """Group scales are folded into the unpack's multiply-add while that is exact and multiplied separately otherwise: the dump bit for
+    bit, the GEMM with the oracle fed the same rounded weights (one row in four has its scales multiplied by `factor`)."""
+    case = T.make_case(24, 96, 512, bits=bits, group=128, enc=enc, scale_dtype=1, seed=19, scale_range=(0.005, 0.05))
+    case.scale[::4] = T.np_bf16_rne(T.np_bf16_to_f32(case.scale[::4]) * np.float32(factor))
+    d_b, d_s = afb.to_device(case.b), afb.to_device(case.scale)
+    d_o = afb.malloc(case.n * case.k * 2)
+    afb.dequant_dump(afb.make_args(d_o, d_b, d_b, d_s, 1, case.n, case.k, ldb=case.ldb, bits=bits, encoding=enc, layout=1, scale_dtype=1, group=128), d_o)
+    afb.device_sync()
+    dump = afb.to_host(d_o, (case.n, case.k), np.uint16)
+    for p in (d_b, d_s, d_o):
+        afb.free(p)
+    assert np.array_equal(dump, oracle.dequant_bf16(case))
+    got, _ = T.run_case(afb, case, variant=pkg.VARIANT_PREFILL, flags=pkg.FLAG_PREFILL_TMEM_A)
+    ref = oracle.gemm(case, threads=4, round_w=True)
+    for rows in (slice(0, None, 4), slice(1, None, 4)):   # rows of B = columns of C, compared at their own magnitude
+        check_close(oracle, np.ascontiguousarray(ref[:, rows]), np.ascontiguousarray(got[:, rows]), f"group scales times {factor}")
+
+
 @pytest.mark.parametrize("bits,enc", [(8, 0), (8, 1), (4, 0), (4, 1)])
 def test_dequant_decode_pairing_is_bit_exact(afb, oracle, bits, enc):
     """The decode kernel unpacks with the strided pairing ({k0,k2},{k1,k3} for int8, {k0,k4}..{k3,k7} for int4).  The dump runs
