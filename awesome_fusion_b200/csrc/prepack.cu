@@ -52,6 +52,63 @@ __global__ void __launch_bounds__(256) prepack_row_kernel(const uint8_t* __restr
     }
 }
 
+// The same for 16-byte aligned rows: a 128 (k) x 128 (n) tile per CTA.  A thread loads 16 channels of 4 consecutive k (four 16-byte
+// loads in flight), transposes 4 x 4 byte blocks in registers straight into packed words, and the tile crosses shared memory once in
+// words: both sides move whole 128-byte lines.  Word q of channel c lies at q ^ 4 * (c / 16 % 8), so that the transposing stores (8
+// channel groups x 4 words per warp) and the 16-byte loads that follow are free of bank conflicts.  Bound by HBM (one read and one write
+// of B): 4096 x 11008 18.4 us = 4.9 TB/s, the byte-wise kernel above 94 us.
+__global__ void __launch_bounds__(256) prepack_row_wide_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint32_t n, uint32_t k,
+                                                               uint32_t in_pitch, uint32_t out_pitch) {
+    __shared__ __align__(16) uint32_t tile[128][32];
+    const uint32_t n0 = blockIdx.x * 128, k0 = blockIdx.y * 128;
+    {
+        const uint32_t cg = threadIdx.x & 7, q = threadIdx.x >> 3;   // 16 channels from n0 + 16 cg, k from k0 + 4 q
+        const uint32_t nn = n0 + cg * 16, kk = k0 + q * 4;
+        uint32_t v[4][4] = {};   // [k][four channels]
+        if (kk < k && nn < n) {   // k is a multiple of 4: all four rows exist
+            const uint8_t* src = in + (size_t)kk * in_pitch + nn;
+            if (nn + 16 <= n) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint4 x = __ldcs(reinterpret_cast<const uint4*>(src + (size_t)i * in_pitch));
+                    v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int b = 0; b < 16; ++b)
+                        if (nn + b < n) v[i][b >> 2] |= (uint32_t)src[(size_t)i * in_pitch + b] << (8 * (b & 3));
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {   // packed word of a channel: bytes of k [0,2,1,3]
+            const uint32_t lo02 = prmt(v[0][b], v[2][b], 0x5140u), hi02 = prmt(v[0][b], v[2][b], 0x7362u);   // {k0,k2} of channels 0,1 / 2,3
+            const uint32_t lo13 = prmt(v[1][b], v[3][b], 0x5140u), hi13 = prmt(v[1][b], v[3][b], 0x7362u);
+            const uint32_t w[4] = {prmt(lo02, lo13, 0x5410u), prmt(lo02, lo13, 0x7632u), prmt(hi02, hi13, 0x5410u), prmt(hi02, hi13, 0x7632u)};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) tile[cg * 16 + b * 4 + e][q ^ (cg * 4)] = w[e];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t c = i * 32 + (threadIdx.x >> 3), piece = threadIdx.x & 7;
+        const uint32_t nn = n0 + c, kk = k0 + piece * 16;
+        if (nn >= n || kk >= k) continue;
+        const uint4 x = *reinterpret_cast<const uint4*>(&tile[c][(piece ^ ((c >> 4) & 7u)) * 4]);
+        uint8_t* dst = out + (size_t)nn * out_pitch + kk;
+        if (kk + 16 <= k) {
+            *reinterpret_cast<uint4*>(dst) = x;
+        } else {   // the last words of a row
+            const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (kk + e * 4 < k) *reinterpret_cast<uint32_t*>(dst + e * 4) = w[e];
+        }
+    }
+}
+
 // rows of two equally shaped byte matrices interleaved: dst row 2i = g row i, dst row 2i+1 = u row i
 __global__ void __launch_bounds__(256) interleave_rows_kernel(const uint8_t* __restrict__ g, const uint8_t* __restrict__ u, uint8_t* __restrict__ dst,
                                                               uint32_t rows, uint32_t row_bytes) {
@@ -89,6 +146,10 @@ extern "C" int afb_prepack(const afb_gemm_args* a, void* out_b, uint32_t out_ldb
     } else {
         dim3 grid((a->n + 31) / 32, (a->k + 31) / 32);
         if (grid.y > 65535) return AFB_ERR_UNSUPPORTED;
+        // rows of whole 16-byte pieces on both sides; other pitches and pointers take the byte-wise kernel (five times slower)
+        const bool wide = a->ldb % 16 == 0 && out_pitch % 16 == 0 && (uintptr_t)a->ptr_b % 16 == 0 && (uintptr_t)out_b % 16 == 0;
+        if (wide) prepack_row_wide_kernel<<<dim3((a->n + 127) / 128, (a->k + 127) / 128), 256, 0, s>>>(reinterpret_cast<const uint8_t*>(a->ptr_b), reinterpret_cast<uint8_t*>(out_b), a->n, a->k, a->ldb, out_pitch);
+        else
         prepack_row_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const uint8_t*>(a->ptr_b), reinterpret_cast<uint8_t*>(out_b), a->n, a->k, a->ldb, out_pitch);
     }
     count_launch();

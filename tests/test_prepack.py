@@ -106,3 +106,23 @@ def test_dequant_dump_reads_packed_weights(afb, oracle, bits, group):
     for p in (d_b, d_s, d_o):
         afb.free(p)
     assert np.array_equal(got, oracle.dequant_bf16(case))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,k,in_pitch,out_pitch", [(128, 128, 128, 128), (205, 132, 208, 144), (16, 4, 16, 16), (129, 260, 160, 272), (300, 516, 304, 528), (205, 132, 205, 144)])
+def test_transposing_prepack_at_tile_edges(afb, oracle, n, k, in_pitch, out_pitch):
+    """[K,N] input with 16-byte rows (a 128 x 128 tile per CTA) at the edges of tiles and pieces; the last shape has odd rows and
+    takes the byte-wise kernel.  The padding of the output is not written."""
+    case = T.make_case(1, n, k, layout=0, seed=n + k)
+    want = oracle.prepack(case, out_ldb=out_pitch).b
+    wide = np.full((k, in_pitch), 0x55, np.uint8)
+    wide[:, :n] = case.b
+    d_b, d_o = afb.to_device(wide), afb.to_device(np.full((n, out_pitch), 0xAA, np.uint8))
+    args = afb.make_args(d_o, d_b, d_b, d_b, 1, n, k, ldb=in_pitch, bits=8, layout=0)
+    afb.prepack(args, d_o, out_pitch)
+    afb.device_sync()
+    got = afb.to_host(d_o, (n, out_pitch), np.uint8)
+    for p in (d_b, d_o):
+        afb.free(p)
+    assert np.array_equal(got[:, :k], want[:, :k])
+    assert np.all(got[:, k:] == 0xAA)
