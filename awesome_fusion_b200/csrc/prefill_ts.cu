@@ -235,43 +235,48 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
         }
     } else if (warp == 1) {
         // ======================= MMA issuer =======================
-        if (lane == 0) {
-            constexpr uint32_t idesc = ptx::umma_idesc_bf16_f32(BNW, BMA);
-            uint32_t st = 0, ph = 0, sa = 0, pa = 0, it = 0;
-            bool ok = true;
-            Item w;
-            for (; ok && get_item(it, w); ++it) {
-                const uint32_t t = w.t;
-                if (!wait_or_abort(bar_acc_empty, (it & 1u) ^ 1u, abort_flag)) {   // the epilogue of the previous tile has drained the accumulator
-                    if (!*abort_flag) { report_timeout(p.status, 22, (int)t, -1); *abort_flag = 1; }
-                    break;
+        // The whole warp runs the loop and one elected lane issues: the operands of tcgen05.mma are then warp-uniform values.  With the
+        // loop under `if (lane == 0)` this warp set the pace: about 850 cycles per 64-wide step against 512 of tensor work (2048 x
+        // 28672 x 8192 int8 818 us, now 666; 4096 rows 1634, now 1464; 2048 x 11008 x 4096 146, now 138).
+        auto wait_all = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag)); };
+        constexpr uint32_t idesc = ptx::umma_idesc_bf16_f32(BNW, BMA);
+        constexpr uint32_t tmem0 = 0;   // all 512 columns are this CTA's: the allocation starts at column 0
+        const uint64_t desc0 = ptx::umma_desc_kmajor_sw128(smem_base + L::kOffAct);
+        const bool two_terms = GROUPED && p.exact;   // slots sa (hi) and sa + 1 (lo) move in lockstep
+        uint32_t st = 0, ph = 0, sa = 0, pa = 0, it = 0;
+        bool ok = true;
+        Item w;
+        for (; ok && get_item(it, w); ++it) {
+            const uint32_t t = w.t;
+            if (!wait_all(bar_acc_empty, (it & 1u) ^ 1u)) {   // the epilogue of the previous tile has drained the accumulator
+                if (!*abort_flag) { report_timeout(p.status, 22, (int)t, -1); *abort_flag = 1; }
+                break;
+            }
+            ptx::tc_fence_after_sync();
+            for (uint32_t kb = w.kb0; kb < w.kb1; ++kb) {
+                if (!wait_all(bar_full(st), ph) || !wait_all(bar_full_a(sa), pa) || (two_terms && !wait_all(bar_full_a(sa + 1), pa))) {
+                    if (!*abort_flag) { report_timeout(p.status, 23, (int)t, (int)kb); *abort_flag = 1; }
+                    ok = false; break;
                 }
                 ptx::tc_fence_after_sync();
-                for (uint32_t kb = w.kb0; kb < w.kb1; ++kb) {
-                    const bool two_terms = GROUPED && p.exact;   // slots sa (hi) and sa + 1 (lo) move in lockstep
-                    if (!wait_or_abort(bar_full(st), ph, abort_flag) || !wait_or_abort(bar_full_a(sa), pa, abort_flag) ||
-                        (two_terms && !wait_or_abort(bar_full_a(sa + 1), pa, abort_flag))) {
-                        if (!*abort_flag) { report_timeout(p.status, 23, (int)t, (int)kb); *abort_flag = 1; }
-                        ok = false; break;
-                    }
-                    ptx::tc_fence_after_sync();
-                    const uint64_t db = ptx::umma_desc_kmajor_sw128(smem_base + L::kOffAct + st * L::kActBytes);
-                    const uint32_t ta = tmem_base + L::kColA + sa * 32;
+                if (ptx::elect_one()) {
+                    const uint64_t db = desc0 + st * (uint32_t)(L::kActBytes >> 4);
+                    const uint32_t ta = tmem0 + L::kColA + sa * 32;
 #pragma unroll
                     for (int j = 0; j < BK / 16; ++j)   // 16 k per instruction: 8 TMEM columns of weights, 32 bytes of each activation row
-                        ptx::umma_bf16_ts(tmem_base, ta + 8 * j, db + 2u * j, idesc, ((kb - w.kb0) | (uint32_t)j) ? 1u : 0u);
+                        ptx::umma_bf16_ts(tmem0, ta + 8 * j, db + 2u * j, idesc, ((kb - w.kb0) | (uint32_t)j) ? 1u : 0u);
                     if (two_terms) {
 #pragma unroll
-                        for (int j = 0; j < BK / 16; ++j) ptx::umma_bf16_ts(tmem_base, ta + 32 + 8 * j, db + 2u * j, idesc, 1u);
+                        for (int j = 0; j < BK / 16; ++j) ptx::umma_bf16_ts(tmem0, ta + 32 + 8 * j, db + 2u * j, idesc, 1u);
                     }
                     ptx::umma_commit(bar_empty_act(st));
                     ptx::umma_commit(bar_empty_a(sa));
                     if (two_terms) ptx::umma_commit(bar_empty_a(sa + 1));
-                    if (++st == S) { st = 0; ph ^= 1u; }
-                    sa += two_terms ? 2 : 1;
-                    if (sa == kSlotsA) { sa = 0; pa ^= 1u; }
+                    if (kb + 1 == w.kb1) ptx::umma_commit(bar_acc_full);
                 }
-                if (ok) ptx::umma_commit(bar_acc_full);
+                if (++st == S) { st = 0; ph ^= 1u; }
+                sa += two_terms ? 2 : 1;
+                if (sa == kSlotsA) { sa = 0; pa ^= 1u; }
             }
         }
     } else if (warp < 2 + kWorkerWarps) {
