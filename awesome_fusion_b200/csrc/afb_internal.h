@@ -17,7 +17,7 @@ struct DeviceCtx {
     // Split-K workspaces (fp32 partial sums + arrival counters, used by decode K-slices, the balanced decode form and the
     // prefill tail split): one per stream that has launched such a GEMM, so that launches on different streams never share
     // one.  Slot 0 is allocated by afb_init, the others on a stream's first launch (outside any stream capture).
-    static constexpr int kMaxWorkspaces = 16;
+    static constexpr int kMaxWorkspaces = 64;
     struct Workspace {
         bool          assigned = false;
         cudaStream_t  stream = nullptr;
@@ -54,7 +54,8 @@ unsigned long long* phase_ts_if_enabled(DeviceCtx* ctx);   // ctx->phase_ts when
 
 DeviceCtx* current_ctx();           // nullptr when afb_init was not called on the current device
 // The split-K workspace of `s` on this device (allocates it on the stream's first use); nullptr + *rc on failure.
-const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* rc);
+// `optional`: the caller has a form that does without; nullptr with *rc = AFB_OK then means that it is to take that one.
+const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* rc, bool optional = false);
 int  cuda_fail(cudaError_t e);      // records e, returns AFB_ERR_CUDA
 void count_launch(unsigned n = 1);
 
@@ -74,6 +75,11 @@ int launch_prefill(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s);     
 // (environment variable AFB_SUB_AR_SMS, default 16: on 2 GPUs 1.03 ms for the down-projection with 16, 1.13 with 8)
 uint32_t sub_allreduce_sms();
 int launch_prefill_ts(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, const afb_fused_args* fused = nullptr);   // converted weights in tensor memory
+// Row tiles per group of a persistent kernel's tile order (tiles of bma rows x 128 channels).
+uint32_t pick_group_m(const afb_gemm_args& a, uint32_t m_tiles, uint32_t n_tiles, uint32_t bma, int sms);
+// The streaming form of the decode and prefill variants (stream.cu): launched where it takes the arguments and is the faster one
+// (*done = true, its status returned); otherwise nothing happens and the caller goes on to the other forms.
+int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, bool* done);
 int launch_prefill_ts_tiles(const afb_gemm_args& a, DeviceCtx* ctx, uint32_t* tile_done, cudaStream_t s);
 // The sum and broadcast of the pipelined reduce-scatter done inside the pushing GEMM, by two extra warps of every CTA (so that no
 // second kernel has to share SMs with the GEMM): where the finished rows go, the words of the closing signal round, the count

@@ -17,7 +17,9 @@ std::atomic<int> g_last_cuda_error{0};
 std::atomic<unsigned long long> g_launches{0};
 constexpr size_t kSplitKWorkspaceBytes = 32u << 20;
 constexpr size_t kSplitKCounters = 4096;
-constexpr int kPreallocatedWorkspaces = 4;
+constexpr int kPreallocatedWorkspaces = 8;
+constexpr int kReservedWorkspaces = 16;              // slots that only launches which cannot do without one may take ...
+constexpr int kReservedPreallocated = 4;             // ... and among them preallocated ones, for first launches inside a capture
 constexpr uint32_t kPrefillTsMinM = 128;   // measured: above 128 activation rows the tensor-memory form is 1.3x faster, at 128 it is slower
 }  // namespace
 
@@ -39,12 +41,31 @@ unsigned long long* phase_ts_if_enabled(DeviceCtx* ctx) {
     return on ? ctx->phase_ts : nullptr;
 }
 
-const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* rc) {
+const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* rc, bool optional) {
     std::lock_guard<std::mutex> lock(g_mutex);
-    DeviceCtx::Workspace* free_slot = nullptr;
+    DeviceCtx::Workspace* with_memory = nullptr;
+    DeviceCtx::Workspace* without = nullptr;
+    int free_slots = 0, free_with_memory = 0;
     for (auto& w : ctx->workspaces) {
         if (w.assigned && w.stream == s) return &w;
-        if (!w.assigned && (!free_slot || (w.ws && !free_slot->ws))) free_slot = &w;   // an unassigned slot that already has memory first
+        if (w.assigned) continue;
+        ++free_slots;
+        if (w.ws) { ++free_with_memory; if (!with_memory) with_memory = &w; }
+        else if (!without) without = &w;
+    }
+    DeviceCtx::Workspace* free_slot = with_memory ? with_memory : without;   // one that already has memory first
+    if (optional) {
+        // a launch that has another form to fall back on: it leaves the others what they had before it existed, and does not
+        // allocate inside a capture
+        *rc = AFB_OK;
+        if (free_slots <= kReservedWorkspaces) return nullptr;
+        if (free_with_memory <= kReservedPreallocated) {
+            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
+            if (capture != cudaStreamCaptureStatusNone) return nullptr;
+            free_slot = without;
+            if (!free_slot) return nullptr;
+        }
     }
     if (!free_slot) { *rc = AFB_ERR_TOO_LARGE; return nullptr; }   // more streams than workspaces
     if (!free_slot->ws) {
@@ -255,8 +276,15 @@ int afb_gemm_launch(const afb_gemm_args* args, void* stream) {
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     switch (v) {
-        case AFB_VARIANT_DECODE:  return launch_decode(*args, ctx, s);
+        case AFB_VARIANT_DECODE: {
+            bool done = false;
+            rc = stream_if_faster(*args, ctx, s, &done);
+            return done ? rc : launch_decode(*args, ctx, s);
+        }
         case AFB_VARIANT_PREFILL: {
+            bool done = false;
+            rc = stream_if_faster(*args, ctx, s, &done);
+            if (done) return rc;
             // two implementations of the prefill variant; a flag or AFB_PREFILL_IMPL=ss|ts overrides the default
             static const int env_ts = [] { const char* e = getenv("AFB_PREFILL_IMPL"); return e ? (e[0] == 't' ? 1 : 0) : -1; }();
             bool ts = env_ts == 1;

@@ -733,6 +733,8 @@ int ts_tmap_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint6
     return r == CUDA_SUCCESS ? AFB_OK : AFB_ERR_CUDA;
 }
 
+}  // namespace
+
 // Row tiles per group of the tile order, from a simple model of the HBM traffic.  One wave of CTAs covers g row tiles and
 // about sms / g channel tiles and re-reads both from HBM, unless the activations of the group (g * BMA * K * 2 bytes) are
 // small enough to stay in L2 over the whole group, in which case they are read once per group.
@@ -760,6 +762,8 @@ uint32_t pick_group_m(const afb_gemm_args& a, uint32_t m_tiles, uint32_t n_tiles
     if (const char* e = getenv("AFB_PREFILL_GROUP_M")) { const uint32_t v = (uint32_t)atoi(e); if (v >= 1 && v <= m_tiles) best_g = v; }
     return best_g;
 }
+
+namespace {
 
 template <int BITS, bool GROUPED, int BMA>
 int launch_ts_cfg(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, uint32_t* tile_done = nullptr, void* const* push = nullptr,

@@ -1,0 +1,784 @@
+// Streaming form of the decode and prefill variants (B in [N,K] layout): weights flow HBM -> shared memory -> registers -> tensor
+// memory -> tcgen05.mma in one pipeline that is deep enough to run at memory speed when M is small and at tensor-core speed when
+// M is large (reference counterpart of the whole kernel: bf16gemm_kernel_gfx90a.s:184-636).
+//
+// D[n, m] = sum_k W[n,k] * A[m,k]: a tile has 128 output channels (the TMEM lanes) and `rows` activation rows (a multiple of 16,
+// fitted to M).  One CTA per SM:
+//
+//   warp 0      (1 lane)  TMA: raw weight blocks, 128 channels x 128 bytes (128 k of int8, 256 k of int4), 128-byte swizzle
+//   warp 1      (1 lane)  TMA: activation slabs [rows x 64] bf16, 128-byte swizzle
+//   warp 2      (1 lane)  tcgen05.mma 128 x rows x 16, weights from TMEM, activations from shared memory
+//   warps 4-7             epilogue, one lane quarter each: accumulator -> scale -> bf16 -> C, or fp32 partial sums -> workspace
+//   warps 8-23            converters: four groups of four warps (one per lane quarter); group g takes every fourth 64-wide step,
+//                         so that four steps are being unpacked at any time.  A warp's chain wait -> load -> unpack -> tcgen05.st
+//                         -> arrive takes about 800 cycles; what bounds a form in which all converters share ONE step is that
+//                         chain, whatever M is.
+//
+// k goes by in parts (one converter group's work: 64 or 128 k) and steps (one hand-off to and from the issuing warp: one part, or
+// two where few rows make the hand-off the larger cost).  Weights and activations have rings of their own.
+// Work is dealt in units of one raw block: first every CTA takes the same number of units of the tiles that do not fill whole
+// waves (contiguous, so at most two of its tiles are shared with neighbours), then whole tiles, one wave after the other.
+// A shared tile is finished by the last CTA to arrive, which adds the fp32 partial sums in CTA order (= ascending K): the bits do
+// not depend on who that is, and no CTA waits for another.  Up to 16 rows the group scales multiply the fp32 sum of each group, in the
+// epilogue warps, while the next groups are being computed; above that they are folded into the bf16 weights.
+//
+// What bounds it: for few rows int8 the weight stream (28672 x 8192, 16 rows: 44.7 us = 5.3 TB/s of weights, 63.8 with decode.cu; the
+// stream, the hand-offs and the shared tiles alone, without unpack and MMAs, take 44.7 too), int4 the issue slots of the unpack and of
+// the hand-offs (53 against 63 us; 40 without unpack and MMAs); for 65 to 128 rows the activations through L2 (28672 x 8192 int4
+// group-128, 128 rows: 66 us, 82 with prefill.cu); for many rows the pace of the issuing warp next to the unpack.
+#include <cstdlib>
+#include "afb_internal.h"
+#include "dequant.cuh"
+#include "ptx_sm100.cuh"
+
+namespace afb {
+
+namespace {
+
+constexpr int kCh = 128;              // output channels per tile
+constexpr int kSlab = 64;             // k of one activation box (128 bytes, one swizzle span)
+constexpr int kRawBytes = kCh * 128;  // one raw block
+constexpr int kGroups = 4;            // converter groups
+constexpr int kFirstEpi = 4, kFirstConv = 8;
+constexpr int kThreads = 32 * (kFirstConv + 4 * kGroups);
+constexpr int kMaxRaw = 12, kMaxSlots = 8, kMaxAcc = 8;
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kSet = 2;            // kSums: group sums handed to the epilogue at a time
+constexpr int kBars = 2 * (kMaxRaw + kMaxSlots + kMaxAcc) + 3;
+constexpr int kOffMisc = kBars * 8, kOffOut = 1024;
+constexpr int kOutBytes = 16 * 32 * 2;                    // one block of the result: 16 rows x 32 channels
+constexpr int kOffRaw = kOffOut + 4 * 2 * kOutBytes;      // two blocks per epilogue warp
+constexpr int kRingBudget = 232448 - 1024 - kOffRaw;      // bytes for the two rings (1 KiB for the alignment of the base)
+static_assert(kOffMisc + 32 <= kOffOut && kOffRaw % 1024 == 0, "shared memory layout");
+
+enum Mode { kChannel = 0,   // per-channel scale on the finished sum
+            kFold = 1,      // group scale folded into the bf16 weight (more than 16 activation rows)
+            kSums = 2 };    // group scale on the fp32 sum of each group (up to 16 rows)
+
+struct StreamParams {
+    uint16_t* c;
+    const void* scale;
+    const uint8_t* zero;
+    uint32_t m, n, k, ldc;
+    uint32_t enc, scale_dtype, packed;
+    uint32_t group_shift;     // log2(group / k of a part)
+    uint32_t flush;           // kSums: parts per group sum
+    uint32_t acc_cols;        // TMEM columns handed to the epilogue at a time (kSums: kSet group sums)
+    uint32_t rows, m_tiles, n_tiles, group_m;
+    uint32_t blocks, parts;   // raw blocks and parts along K
+    uint32_t shared_tiles, whole_waves;   // tiles [0, shared_tiles) are dealt in units, the rest are whole tiles
+    uint32_t raw_stages, slots, accs;
+    uint32_t slot_first;      // converters wait for their slot before they wait for their raw block
+    uint32_t c_tma, c_vec;    // tile stores; 8-byte stores of finished shared tiles
+    uint32_t finish_late;     // shared tiles are finished by all warps at the CTA's end, not by the epilogue warps on the way
+    float* ws;                // [2 * CTA + (not the CTA's first shared tile)][row][channel]
+    uint32_t* counters;       // one per shared tile, zero on entry and on exit
+    int32_t* status;
+};
+
+__device__ __forceinline__ void report_timeout(int32_t* status, int where, int a, int b) {
+    if (atomicCAS(status, 0, AFB_ERR_TIMEOUT) == 0) { status[1] = where; status[2] = a; status[3] = b; }
+}
+__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
+    unsigned long long t0 = 0;
+    for (uint32_t tries = 0; !ptx::mbar_try_wait(bar, parity);) {
+        if ((++tries & 0x3fu) == 0) {   // the clock is read only here: reading %globaltimer takes longer than most waits
+            if (*abort_flag) return false;
+            const unsigned long long t = ptx::globaltimer();
+            if (t0 == 0) t0 = t;
+            else if (t - t0 > ptx::kWaitLimitNs) return false;
+        }
+    }
+    return true;
+}
+// The same for a converged warp: every lane gets the same answer, so that none is missing from the warp-wide instructions that follow.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
+    return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag));
+}
+// A position in a ring of runtime length.
+struct Ring {
+    uint32_t i, phase;
+    __device__ __forceinline__ void step(uint32_t by, uint32_t len) { i += by; if (i >= len) { i -= len; phase ^= 1u; } }   // by <= len
+    __device__ __forceinline__ void set(uint32_t count, uint32_t len) { const uint32_t w = count / len; i = count - w * len; phase = w & 1u; }
+};
+
+// The pieces of work of one CTA, in order; every role walks the same list.
+struct Piece { uint32_t t, kb0, kb1; };
+struct Walk {
+    uint32_t u, u_end, it;
+    __device__ __forceinline__ void start(const StreamParams& p) {
+        const uint32_t total = p.shared_tiles * p.blocks;
+        u = (uint32_t)((uint64_t)blockIdx.x * total / gridDim.x);
+        u_end = (uint32_t)((uint64_t)(blockIdx.x + 1) * total / gridDim.x);
+        it = 0;
+    }
+    __device__ __forceinline__ bool next(const StreamParams& p, Piece& x) {
+        if (u < u_end) {
+            x.t = u / p.blocks; x.kb0 = u - x.t * p.blocks;
+            x.kb1 = min(p.blocks, x.kb0 + (u_end - u));
+            u += x.kb1 - x.kb0;
+            return true;
+        }
+        if (it >= p.whole_waves) return false;
+        x.t = p.shared_tiles + blockIdx.x + it * gridDim.x; x.kb0 = 0; x.kb1 = p.blocks;
+        ++it;
+        return true;
+    }
+};
+// Groups of group_m row tiles; inside a group the channel tiles advance, row tile fastest.
+__device__ __forceinline__ void tile_origin(const StreamParams& p, uint32_t t, uint32_t& m0, uint32_t& n0) {
+    const uint32_t per_group = p.group_m * p.n_tiles;
+    const uint32_t g = t / per_group, r = t - g * per_group;
+    const uint32_t gsz = min(p.group_m, p.m_tiles - g * p.group_m);
+    const uint32_t nt = r / gsz;
+    n0 = nt * kCh;
+    m0 = (g * p.group_m + (r - nt * gsz)) * p.rows;
+}
+
+template <int BITS, int MODE, int KS, int PAIR>
+__global__ void __launch_bounds__(kThreads, 1)
+stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_w,
+              const __grid_constant__ CUtensorMap tmap_c, const StreamParams p) {
+    constexpr uint32_t SPB = (BITS == 8 ? 128 : 256) / KS;   // parts per raw block
+    constexpr uint32_t kPartCols = KS / 2, kSlotCols = PAIR * kPartCols;   // TMEM columns of the converted weights of a part, of a step
+    extern __shared__ uint8_t smem_raw_base[];
+    const uint32_t smem_base = (ptx::smem_u32(smem_raw_base) + 1023u) & ~1023u;
+    uint8_t* smem_gen = smem_raw_base + (smem_base - ptx::smem_u32(smem_raw_base));
+    auto bar = [&](uint32_t i) { return smem_base + 8u * i; };
+    auto raw_full = [&](uint32_t s) { return bar(s); };
+    auto raw_empty = [&](uint32_t s) { return bar(kMaxRaw + s); };
+    auto step_full = [&](uint32_t s) { return bar(2 * kMaxRaw + s); };                // converted weights in TMEM, activations in shared memory
+    auto step_empty = [&](uint32_t s) { return bar(2 * kMaxRaw + kMaxSlots + s); };   // the MMAs of the step are done with both
+    auto acc_full = [&](uint32_t s) { return bar(2 * (kMaxRaw + kMaxSlots) + s); };
+    auto acc_empty = [&](uint32_t s) { return bar(2 * (kMaxRaw + kMaxSlots) + kMaxAcc + s); };
+    // a shared tile: every epilogue warp has published its part; the count has been taken.  The end: the epilogue is through
+    const uint32_t bar_stored = bar(kBars - 3), bar_verdict = bar(kBars - 2), bar_finish = bar(kBars - 1);
+    volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + kOffMisc);   // TMEM base, abort flag, "arrived last", tiles to finish, their number
+    volatile uint32_t* abort_flag = misc + 1;
+    const uint32_t slab_bytes = p.rows * 128u, part_bytes = slab_bytes * (KS / kSlab), act_bytes = PAIR * part_bytes, off_act = kOffRaw + p.raw_stages * kRawBytes;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // see decode.cu: no-op without AFB_FLAG_PDL
+
+    // Warp 0 needs only its own barriers: it starts the weight stream while the others are still setting up.
+    if (warp == 0) {
+        if (lane == 0) {
+            for (uint32_t s = 0; s < p.raw_stages; ++s) { ptx::mbar_init(raw_full(s), 1); ptx::mbar_init(raw_empty(s), 4 * SPB); }
+            *abort_flag = 0;
+            ptx::fence_mbar_init();
+        }
+        __syncwarp();
+        asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
+    } else {
+        if (warp == 1 && lane == 0) {
+            for (uint32_t s = 0; s < p.slots; ++s) { ptx::mbar_init(step_full(s), 4 * PAIR + 1); ptx::mbar_init(step_empty(s), 1); }
+            for (uint32_t s = 0; s < p.accs; ++s) { ptx::mbar_init(acc_full(s), 1); ptx::mbar_init(acc_empty(s), 4); }
+            ptx::mbar_init(bar_stored, 4);
+            ptx::mbar_init(bar_verdict, 1);
+            ptx::mbar_init(bar_finish, 4);
+            ptx::fence_mbar_init();
+            ptx::prefetch_tmap(&tmap_act);
+            if (p.c_tma) ptx::prefetch_tmap(&tmap_c);
+        }
+        if (warp == 2) {
+            ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(misc)), kTmemCols);
+            ptx::tmem_relinquish();
+        }
+        __syncwarp();
+        ptx::tc_fence_before_sync();
+        asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+        ptx::tc_fence_after_sync();
+    }
+    constexpr uint32_t tmem_base = 0;   // all 512 columns are this CTA's: the allocation starts at column 0
+    const uint32_t slot_base = tmem_base + kTmemCols - p.slots * kSlotCols;   // accumulators from column 0, slots at the end
+
+    auto give_up = [&](int where, uint32_t a, uint32_t b) {
+        if (!*abort_flag) { report_timeout(p.status, where, (int)a, (int)b); *abort_flag = 1; }
+    };
+    Walk walk;
+    walk.start(p);
+    Piece x;
+    auto parts_of = [&](const Piece& q) { return min(q.kb1 * SPB, p.parts) - q.kb0 * SPB; };
+
+    // Adds the partial sums of shared tile t in CTA order, scales, rounds and stores it; `tid` of `threads` threads, four channels of
+    // one row at a time, up to eight 16-byte loads in flight per thread.
+    const uint32_t total_units = p.shared_tiles * p.blocks;
+    // the CTA holding unit u: the largest c with c * total / grid <= u
+    auto cta_of = [&](uint32_t u) { return (uint32_t)((((uint64_t)u + 1) * gridDim.x + total_units - 1) / total_units) - 1u; };
+    auto finish_tile = [&](uint32_t t, uint32_t tid, uint32_t threads) {
+        uint32_t m0, n0;
+        tile_origin(p, t, m0, n0);
+        const uint32_t first = cta_of(t * p.blocks), last = cta_of(t * p.blocks + p.blocks - 1);
+        const uint32_t valid = min(p.rows, p.m - m0), vecs = valid * (kCh / 4);
+        const uint32_t nn = n0 + (tid & 31u) * 4;   // threads is a multiple of 32: the same four channels in every turn
+        float sc[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            sc[e] = MODE == kSums ? kUnpackInverse : MODE == kFold ? kGroupInverse : nn + e >= p.n ? 0.f :
+                kUnpackInverse * (p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn + e] << 16)
+                                                                  : reinterpret_cast<const float*>(p.scale)[nn + e]);
+        // Only the first contributor can hold the tile as anything but its first shared tile (slot 1).
+        const uint32_t first_slot = 2 * first + ((uint32_t)((uint64_t)first * total_units / gridDim.x) / p.blocks != t ? 1u : 0u);
+        const size_t stride = (size_t)p.rows * kCh;
+        for (uint32_t v = tid; v < vecs; v += 2 * threads) {
+            float4 sum[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+            for (uint32_t c = first; c <= last; c += 4) {
+                float4 y[2][4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        y[h][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (c + i <= last && v + h * threads < vecs)
+                            y[h][i] = __ldcg(reinterpret_cast<const float4*>(p.ws + (size_t)(c + i == first ? first_slot : 2 * (c + i)) * stride) + v + h * threads);
+                    }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) { sum[h].x += y[h][i].x; sum[h].y += y[h][i].y; sum[h].z += y[h][i].z; sum[h].w += y[h][i].w; }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (v + h * threads >= vecs) break;
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(sum[h].x * sc[0], sum[h].y * sc[1]), hi = __floats2bfloat162_rn(sum[h].z * sc[2], sum[h].w * sc[3]);
+                uint16_t* dst = p.c + (size_t)(m0 + (v + h * threads) / (kCh / 4)) * p.ldc + nn;
+                if (p.c_vec && nn + 4 <= p.n) {
+                    *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                } else {
+                    const uint16_t o[4] = {__bfloat16_as_ushort(lo.x), __bfloat16_as_ushort(lo.y), __bfloat16_as_ushort(hi.x), __bfloat16_as_ushort(hi.y)};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) if (nn + e < p.n) dst[e] = o[e];
+                }
+            }
+        }
+    };
+
+    // Warps 0 to 2 run their loops as whole warps and elect a lane for the asynchronous instructions only: the operands are then
+    // warp-uniform values.  (With the loops under `if (lane == 0)` the issuing warp needed 900 cycles per 64-wide step, whatever M.)
+    if (warp == 0) {
+        // ======================= TMA: raw weights =======================
+        Ring r{0, 0};
+        uint32_t issued = 0, parity = 0;
+        bool ok = true;
+        while (ok && walk.next(p, x)) {
+            uint32_t m0, n0;
+            tile_origin(p, x.t, m0, n0);
+            for (uint32_t kb = x.kb0; kb < x.kb1; ++kb) {
+                if (!warp_wait(raw_empty(r.i), r.phase ^ 1u, abort_flag)) { give_up(31, x.t, kb); ok = false; break; }
+                if (ptx::elect_one()) {
+                    ptx::mbar_arrive_expect_tx(raw_full(r.i), kRawBytes);
+                    ptx::tma_load_2d(smem_base + kOffRaw + r.i * kRawBytes, &tmap_w, (int)(kb * 128u), (int)n0, raw_full(r.i));
+                }
+                issued |= 1u << r.i; parity = (parity & ~(1u << r.i)) | (r.phase << r.i);
+                r.step(1, p.raw_stages);
+            }
+        }
+        for (uint32_t s = 0; s < p.raw_stages; ++s)   // never leave with a bulk copy still writing this CTA's shared memory
+            if (issued & (1u << s)) ptx::mbar_wait(raw_full(s), (parity >> s) & 1u);
+    } else if (warp == 1) {
+        // ======================= TMA: activations =======================
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // everything before this line reads weights only
+        Ring r{0, 0};
+        uint32_t issued = 0, parity = 0;
+        bool ok = true;
+        while (ok && walk.next(p, x)) {
+            uint32_t m0, n0;
+            tile_origin(p, x.t, m0, n0);
+            const uint32_t k0 = x.kb0 * SPB, ns = parts_of(x);
+            for (uint32_t l = 0; l < ns; l += PAIR) {
+                if (!warp_wait(step_empty(r.i), r.phase ^ 1u, abort_flag)) { give_up(32, x.t, l); ok = false; break; }
+                if (ptx::elect_one()) {
+                    ptx::mbar_arrive_expect_tx(step_full(r.i), l + PAIR <= ns ? act_bytes : part_bytes);
+#pragma unroll
+                    for (int h = 0; h < PAIR * KS / kSlab; ++h)
+                        if (PAIR == 1 || h < KS / kSlab || l + 1 < ns)
+                            ptx::tma_load_2d(smem_base + off_act + r.i * act_bytes + h * slab_bytes, &tmap_act, (int)((k0 + l) * KS + h * kSlab), (int)m0, step_full(r.i));
+                }
+                issued |= 1u << r.i; parity = (parity & ~(1u << r.i)) | (r.phase << r.i);
+                r.step(1, p.slots);
+            }
+        }
+        for (uint32_t s = 0; s < p.slots; ++s)
+            if (issued & (1u << s)) ptx::mbar_wait(step_full(s), (parity >> s) & 1u);   // after an abort the converters' part may be missing: then the limit of the wait, far above the time of a copy
+    } else if (warp == 2) {
+        // ======================= MMA issuer =======================
+        const uint32_t idesc = ptx::umma_idesc_bf16_f32(kCh, p.rows);
+        const uint64_t desc0 = ptx::umma_desc_kmajor_sw128(smem_base + off_act);
+        const uint32_t slab_d = slab_bytes >> 4, act_d = act_bytes >> 4;   // in units of the descriptor's address field
+        Ring rs{0, 0}, rc{0, 0};
+        bool ok = true, ready = false;
+        while (ok && walk.next(p, x)) {
+            const uint32_t ns = parts_of(x);
+            uint32_t in_sum = 0, sum = 0;   // parts in the current sum; sums in the current accumulator (kSums)
+            for (uint32_t l = 0; l < ns; l += PAIR) {
+                if (in_sum == 0 && sum == 0 && !warp_wait(acc_empty(rc.i), rc.phase ^ 1u, abort_flag)) { give_up(33, x.t, l); ok = false; break; }
+                if (!__all_sync(0xffffffffu, ready) && !warp_wait(step_full(rs.i), rs.phase, abort_flag)) { give_up(34, x.t, l); ok = false; break; }
+                ptx::tc_fence_after_sync();
+                const uint64_t db = desc0 + rs.i * act_d;
+                const uint32_t ta = slot_base + rs.i * kSlotCols, td = tmem_base + rc.i * p.acc_cols, done = step_empty(rs.i), acc_done = acc_full(rc.i);
+                rs.step(1, p.slots);
+                ready = ptx::mbar_test_wait(step_full(rs.i), rs.phase);   // of the next step: the answer is back when this one has been issued
+                bool last = false;
+#pragma unroll
+                for (int h = 0; h < PAIR; ++h) {
+                    if (PAIR > 1 && h > 0 && l + h >= ns) break;
+                    if (ptx::elect_one()) {
+#pragma unroll
+                        for (int j = 0; j < KS / 16; ++j)
+                            ptx::umma_bf16_ts(td + sum * 16, ta + h * kPartCols + 8 * j, db + (uint32_t)(h * (KS / kSlab) + j / 4) * slab_d + 2u * (j % 4), idesc, (in_sum | (uint32_t)j) ? 1u : 0u);
+                    }
+                    ++in_sum;
+                    if (MODE == kSums && in_sum == p.flush) { in_sum = 0; ++sum; }
+                    last = l + h + 1 == ns || (MODE == kSums && sum == kSet);
+                }
+                if (ptx::elect_one()) {
+                    ptx::umma_commit(done);
+                    if (last) ptx::umma_commit(acc_done);
+                }
+                if (last) { rc.step(1, p.accs); in_sum = sum = 0; }
+            }
+        }
+    } else if (warp >= kFirstConv) {
+        // ======================= converters =======================
+        const uint32_t g = (uint32_t)(warp - kFirstConv) >> 2, quarter = (uint32_t)warp & 3u;
+        const uint32_t ch = quarter * 32 + lane;
+        const uint32_t flip = BITS == 8 ? flip8(p.enc) : flip4(p.enc);
+        const uint32_t sel0 = p.packed ? kSel8Strided02 : kSel8Natural01, sel1 = p.packed ? kSel8Strided13 : kSel8Natural23;
+        const Nibbles nib = nibbles(p.packed != 0);
+        const bool has_zero = p.zero != nullptr;
+        const uint32_t groups_per_row = MODE == kChannel ? 0 : (p.parts >> p.group_shift);
+        auto zero_of = [&](uint32_t zb) { return !has_zero ? 0 : (BITS == 8 ? decode_zero8(zb, p.enc) : decode_zero4(zb, p.enc)); };
+        GroupUnpack up;
+        up.mul0 = BITS == 8 ? kMulByte : nib.mul[0]; up.mul1 = nib.mul[1]; up.add = unpack_add(BITS, 0); up.scale = 0;
+        uint32_t steps_before = 0, blocks_before = 0;   // of the pieces walked so far (a step is PAIR parts, the last of a piece may lack one)
+        bool ok = true;
+        while (ok && walk.next(p, x)) {
+            uint32_t m0, n0;
+            tile_origin(p, x.t, m0, n0);
+            const uint32_t nn = n0 + ch, ns = parts_of(x), k0 = x.kb0 * SPB;
+            const size_t g0 = (size_t)nn * groups_per_row;
+            uint32_t sc = 0, zb = 0, sc_nxt = 0, zb_nxt = 0;
+            auto load_group = [&](uint32_t l, uint32_t& s, uint32_t& z) {
+                if (MODE == kChannel || nn >= p.n || l >= ns) return;
+                const size_t i = g0 + ((k0 + l) >> p.group_shift);
+                if (MODE == kFold) s = reinterpret_cast<const uint16_t*>(p.scale)[i];
+                if (has_zero) z = p.zero[i];
+            };
+            if (MODE == kChannel && has_zero) up.add = unpack_add(BITS, zero_of(nn < p.n ? p.zero[nn] : 0u));
+            uint32_t l = (g - steps_before * PAIR) & (kGroups - 1);
+            Ring rr, rs;
+            rr.set(blocks_before + l / SPB, p.raw_stages);
+            rs.set(steps_before + l / PAIR, p.slots);
+            load_group(l, sc_nxt, zb_nxt);
+            const uint32_t nv = (ns + PAIR - 1) / PAIR * PAIR;
+            for (; l < nv; l += kGroups) {
+                if (PAIR > 1 && l == ns) {
+                    // The part that the last step of this piece lacks: waited for and reported like the others.  A group that passed
+                    // over it would next look at a slot two uses later, where the parity of the barrier no longer tells it anything.
+                    if (!warp_wait(step_empty(rs.i), rs.phase ^ 1u, abort_flag)) { give_up(36, x.t, l); ok = false; break; }
+                    if (lane == 0) ptx::mbar_arrive(step_full(rs.i));
+                    continue;
+                }
+                const uint32_t sub = l % SPB, left = ns - (l - sub);   // `left`: parts of this block and all after it
+                if (MODE != kChannel) { sc = sc_nxt; zb = zb_nxt; load_group(l + kGroups, sc_nxt, zb_nxt); }
+                if (p.slot_first && !warp_wait(step_empty(rs.i), rs.phase ^ 1u, abort_flag)) { give_up(36, x.t, l); ok = false; break; }
+                if (!warp_wait(raw_full(rr.i), rr.phase, abort_flag)) { give_up(35, x.t, l); ok = false; break; }
+                const uint8_t* raw = smem_gen + kOffRaw + rr.i * kRawBytes + ch * 128;
+                constexpr int kWords = BITS == 8 ? 16 : 8;   // of 64 weights
+                bool folded = true;
+                if (MODE == kFold) {
+                    folded = __all_sync(0xffffffffu, group_folds((uint16_t)sc, has_zero));
+                    up = group_unpack(BITS, (uint16_t)sc, zero_of(zb), folded, nib);
+                } else if (MODE == kSums && has_zero) {
+                    up.add = unpack_add(BITS, zero_of(zb));
+                }
+#pragma unroll
+                for (int h = 0; h < KS / 64; ++h) {
+                    uint32_t w[kWords], o[32];
+#pragma unroll
+                    for (int i = 0; i < kWords / 4; ++i) {
+                        const uint4 v = *reinterpret_cast<const uint4*>(raw + ((((sub * (KS / 64) + h) * (kWords / 4) + i) ^ (ch & 7u)) << 4));
+                        w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+                    }
+#pragma unroll
+                    for (int j = 0; j < kWords; ++j) {
+                        if (BITS == 8) {
+                            s8x4_to_bf16(w[j], flip, sel0, sel1, up.mul0, up.add, o[2 * j], o[2 * j + 1]);
+                        } else {
+                            uint32_t qv[4];
+                            s4x8_to_bf16(w[j], flip, nib, up.mul0, up.mul1, up.add, qv);
+                            o[4 * j] = qv[0]; o[4 * j + 1] = qv[1]; o[4 * j + 2] = qv[2]; o[4 * j + 3] = qv[3];
+                        }
+                    }
+                    if (MODE == kFold && !folded) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) o[j] = bf16x2_mul(o[j], up.scale);
+                    }
+                    if (h == 0) {
+                        if (!p.slot_first && !warp_wait(step_empty(rs.i), rs.phase ^ 1u, abort_flag)) { give_up(36, x.t, l); ok = false; break; }
+                        ptx::tc_fence_after_sync();
+                    }
+                    ptx::tmem_st_32x32(slot_base + ((quarter * 32u) << 16) + rs.i * kSlotCols + (l % PAIR) * kPartCols + h * 32, o);
+                }
+                if (!ok) break;
+                ptx::tmem_st_wait();
+                ptx::tc_fence_before_sync();
+                __syncwarp();   // every lane's weights are in tensor memory
+                if (lane == 0) {
+                    ptx::mbar_arrive(step_full(rs.i));
+                    ptx::mbar_arrive_count(raw_empty(rr.i), left < SPB && sub + 1 == left ? 1 + SPB - left : 1u);   // a short last block: for its missing parts, too
+                }
+                rr.step(kGroups / SPB, p.raw_stages);   // four parts on
+                rs.step(kGroups / PAIR, p.slots);
+            }
+            steps_before += (ns + PAIR - 1) / PAIR;
+            blocks_before += x.kb1 - x.kb0;
+        }
+    } else if (warp >= kFirstEpi) {
+        // ======================= epilogue =======================
+        const uint32_t quarter = (uint32_t)warp & 3u, ch = quarter * 32 + lane;
+        const uint32_t lane_base = tmem_base + ((quarter * 32u) << 16);
+        const uint32_t first_tile = walk.u / p.blocks;
+        const uint32_t groups_per_row = MODE == kChannel ? 0 : (p.parts >> p.group_shift);
+        Ring rc{0, 0};
+        uint32_t meeting = 0, to_finish = 0;
+        uint32_t block = 0;   // staging block of the next tile store
+        bool ok = true;
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // workspace, counters and C belong to the predecessor until it has ended
+        while (ok && walk.next(p, x)) {
+            uint32_t m0, n0;
+            tile_origin(p, x.t, m0, n0);
+            const uint32_t nn = n0 + ch, ns = parts_of(x);
+            const uint32_t valid = min(p.rows, p.m - m0);
+            const bool whole = x.kb0 == 0 && x.kb1 == p.blocks;
+            const float scale = MODE == kSums ? kUnpackInverse : MODE == kFold ? kGroupInverse :
+                nn >= p.n ? 0.f : kUnpackInverse * (p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn] << 16)
+                                                                                    : reinterpret_cast<const float*>(p.scale)[nn]);
+            // 16 rows of this lane's channel, finished
+            auto store = [&](uint32_t c0, const float (&v)[16]) {
+                if (p.c_tma) {
+                    // through shared memory as a tile store (clipped at the edges of C); two blocks per warp take turns
+                    const uint32_t out = smem_base + kOffOut + (quarter * 2 + block) * kOutBytes;
+                    if (lane == 0) ptx::bulk_wait_group_read1();
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(out + (uint32_t)j * 64u + (uint32_t)lane * 2u),
+                                     "h"(__bfloat16_as_ushort(__float2bfloat16_rn(v[j] * scale))) : "memory");
+                    ptx::fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        ptx::tma_store_2d(&tmap_c, out, (int)(n0 + quarter * 32u), (int)(m0 + c0));
+                        ptx::bulk_commit_group();
+                    }
+                    block ^= 1u;
+                } else if (nn < p.n) {
+                    uint16_t* dst = p.c + (size_t)(m0 + c0) * p.ldc + nn;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (c0 + j < valid) dst[(size_t)j * p.ldc] = __bfloat16_as_ushort(__float2bfloat16_rn(v[j] * scale));
+                }
+            };
+            float* part = p.ws + (size_t)(2 * blockIdx.x + (x.t != first_tile ? 1 : 0)) * p.rows * kCh + ch;
+            auto emit = [&](uint32_t c0, const float (&v)[16]) {
+                if (whole) { store(c0, v); return; }
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (c0 + j < valid) __stcg(part + (size_t)(c0 + j) * kCh, v[j]);
+            };
+            if (MODE == kSums) {
+                float sum[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) sum[j] = 0.f;
+                const size_t g0 = (size_t)nn * groups_per_row;
+                auto group_scale = [&](uint32_t l) {
+                    if (nn >= p.n || l >= ns) return 0.f;
+                    const size_t i = g0 + ((x.kb0 * SPB + l) >> p.group_shift);
+                    return p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[i] << 16)
+                                                           : reinterpret_cast<const float*>(p.scale)[i];
+                };
+                float sc[kSet];
+#pragma unroll
+                for (uint32_t i = 0; i < kSet; ++i) sc[i] = group_scale(i * p.flush);
+                for (uint32_t l = 0; l < ns; l += kSet * p.flush) {
+                    float sc_nxt[kSet];
+#pragma unroll
+                    for (uint32_t i = 0; i < kSet; ++i) sc_nxt[i] = group_scale(l + (kSet + i) * p.flush);
+                    if (!warp_wait(acc_full(rc.i), rc.phase, abort_flag)) { give_up(37, x.t, l); ok = false; break; }
+                    ptx::tc_fence_after_sync();
+#pragma unroll
+                    for (uint32_t i = 0; i < kSet; i += 2) {
+                        if (l + i * p.flush >= ns) break;
+                        uint32_t r[2][16];   // (sums that this accumulator does not hold are read, too, and left alone)
+                        ptx::tmem_ld_32x16(lane_base + rc.i * p.acc_cols + i * 16, r[0]);
+                        ptx::tmem_ld_32x16(lane_base + rc.i * p.acc_cols + i * 16 + 16, r[1]);
+                        ptx::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) sum[j] = fmaf(sc[i], __uint_as_float(r[0][j]), sum[j]);
+                        if (l + (i + 1) * p.flush < ns)
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) sum[j] = fmaf(sc[i + 1], __uint_as_float(r[1][j]), sum[j]);
+                    }
+                    ptx::tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(acc_empty(rc.i));
+                    rc.step(1, p.accs);
+#pragma unroll
+                    for (uint32_t i = 0; i < kSet; ++i) sc[i] = sc_nxt[i];
+                }
+                if (!ok) break;
+                emit(0, sum);
+            } else {
+                if (!warp_wait(acc_full(rc.i), rc.phase, abort_flag)) { give_up(37, x.t, 0); break; }
+                ptx::tc_fence_after_sync();
+#pragma unroll 1
+                for (uint32_t c0 = 0; c0 < p.rows; c0 += 32) {
+                    uint32_t r[2][16];
+                    ptx::tmem_ld_32x16(lane_base + rc.i * p.acc_cols + c0, r[0]);
+                    if (c0 + 16 < p.rows) ptx::tmem_ld_32x16(lane_base + rc.i * p.acc_cols + c0 + 16, r[1]);
+                    ptx::tmem_ld_wait();
+                    if (c0 + 32 >= p.rows) {   // everything is in registers: the accumulator is free
+                        ptx::tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive(acc_empty(rc.i));
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (c0 + 16 * h >= p.rows) break;
+                        float v[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[h][j]);
+                        emit(c0 + 16 * h, v);
+                    }
+                }
+                rc.step(1, p.accs);
+            }
+            if (!whole) {
+                // the CTAs holding units of this tile meet at its counter
+                const uint32_t first = cta_of(x.t * p.blocks), last = cta_of(x.t * p.blocks + p.blocks - 1);
+                __threadfence();
+                __syncwarp();
+                if (lane == 0) {
+                    ptx::mbar_arrive(bar_stored);
+                    if (quarter == 0) {
+                        misc[2] = wait_or_abort(bar_stored, meeting, abort_flag) && atomicAdd(p.counters + x.t, 1u) == last - first ? 1u : 0u;
+                        ptx::mbar_arrive(bar_verdict);
+                    }
+                }
+                if (!warp_wait(bar_verdict, meeting, abort_flag)) { give_up(38, x.t, 0); break; }
+                meeting ^= 1u;   // misc[2] is written again only after all four warps have arrived at the next meeting
+                if (misc[2]) {
+                    __threadfence();
+                    if (p.finish_late) {   // all the warps together, when this CTA's work is done (at most two tiles are shared)
+                        if (quarter == 0 && lane == 0) misc[4 + to_finish] = x.t;
+                        ++to_finish;
+                    } else {
+                        finish_tile(x.t, threadIdx.x - 32 * kFirstEpi, 128);
+                    }
+                    if (quarter == 0 && lane == 0) p.counters[x.t] = 0u;
+                }
+            }
+        }
+        if (p.finish_late) {
+            if (quarter == 0 && lane == 0) misc[3] = ok ? to_finish : 0u;
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(bar_finish);
+        }
+        if (p.c_tma && lane == 0) ptx::bulk_wait_group0();   // this warp's tile stores are complete
+    }
+
+    if (p.finish_late && warp >= kFirstEpi && warp_wait(bar_finish, 0u, abort_flag)) {
+        __threadfence();
+        for (uint32_t i = 0; i < misc[3]; ++i) finish_tile(misc[4 + i], threadIdx.x - 32 * kFirstEpi, kThreads - 32 * kFirstEpi);
+    }
+
+    // ---- teardown: every thread gets here, also after an abort ----
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 2) {
+        ptx::tc_fence_after_sync();
+        ptx::tmem_dealloc(tmem_base, kTmemCols);
+    }
+}
+
+int tmap_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
+            uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swz) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return AFB_ERR_CUDA;
+    cuuint64_t dims[2] = {inner, outer};
+    cuuint64_t strides[1] = {row_stride_bytes};
+    cuuint32_t box[2] = {box_inner, box_outer};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? AFB_OK : AFB_ERR_CUDA;
+}
+
+template <int BITS, int MODE, int KS, int PAIR>
+int launch_cfg(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& tc, const StreamParams& p, uint32_t grid, bool pdl,
+               DeviceCtx* ctx, cudaStream_t s) {
+    auto kern = stream_kernel<BITS, MODE, KS, PAIR>;
+    static DeviceOnce attr_set;  // per template instance
+    if (!attr_set.done(ctx->device)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+        if (e != cudaSuccess) return cuda_fail(e);
+        attr_set.mark(ctx->device);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kThreads); cfg.stream = s;
+    cfg.dynamicSmemBytes = 1024 + kOffRaw + p.raw_stages * kRawBytes + p.slots * p.rows * 128 * (PAIR * KS / kSlab);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tw, tc, p);
+    count_launch();
+    return e == cudaSuccess ? AFB_OK : cuda_fail(e);
+}
+
+}  // namespace
+
+namespace {
+
+bool stream_supports(const afb_gemm_args& a) {
+    if (a.b_layout != AFB_LAYOUT_COL && a.b_layout != AFB_LAYOUT_COL_PACKED) return false;
+    if (a.k % kSlab || a.lda % 8) return false;
+    if (((uint64_t)a.ldb * a.b_bits / 8) % 16) return false;
+    if ((uintptr_t)a.ptr_a % 16 || (uintptr_t)a.ptr_b % 16) return false;
+    // forced forms, explicit variants, fp32 results (their order of addition is that of the exchange forms) and the two-term mode stay where they are
+    if (a.flags & (AFB_FLAG_C_F32 | AFB_FLAG_PREFILL_SMEM_B | AFB_FLAG_PREFILL_TMEM_A)) return false;
+    if ((a.flags & AFB_FLAG_GROUP_EXACT) && a.group_size) return false;
+    if (a.group_size) {
+        if (a.group_size % kSlab || (a.group_size & (a.group_size - 1)) || a.k % a.group_size) return false;
+        if (a.m > 16 && a.scale_dtype != AFB_SCALE_BF16) return false;
+    }
+    return true;
+}
+
+// Rows per tile for M rows.  Up to 192 (two accumulators next to four weight slots in tensor memory), or up to 128 where steps of
+// 128 k are possible and the tiles are few enough that the finer grain pays for the weights being unpacked once more per 128 rows
+// instead of 192 (28672 x 8192 int4 group-128: 222 against 236 us at M = 512, 449 against 496 at 1024, 944 against 915 at 2048).
+uint32_t tile_rows(const afb_gemm_args& a) {
+    const bool wide_steps = a.k % 128 == 0 && a.group_size % 128 == 0;
+    const uint32_t most = wide_steps && a.m > 192 && a.m <= 1024 ? 128 : 192;
+    const uint32_t tiles = (a.m + most - 1) / most;
+    return ((a.m + tiles - 1) / tiles + 15) / 16 * 16;
+}
+
+// Where this form is the faster one, from times of both forms on one B200 (us, the other form / this one).
+bool is_faster(const afb_gemm_args& a, uint32_t sms) {
+    const double weights = (double)a.n * a.k, mbytes = weights * a.b_bits / 8 / 1e6;
+    if (a.m <= 16) {
+        // The decode kernel has about 9 us less to set up and finish, and its arithmetic grows with M; this form's does not.
+        //   28672 x 8192 int8   M = 2: 44 / 44   4: 51 / 44    8: 68 / 44   16: 64 / 45
+        //   28672 x 8192 int4   M = 1: 40 / 53   4: 53 / 53    8: 64 / 53   16: 63 / 53    (group 128)
+        //   12288 x 4096 int8   M = 1: 14 / 22   8: 21 / 22   16: 27 / 22
+        //    4096 x 11008 int4  M = 1: 14 / 21   4: 22 / 21    8: 30 / 21   16: 31 / 22    (one activation row is staged in several passes)
+        //   12288 x 4096 int4   M = 8: 18 / 24  16: 23 / 23;   4096 x 4096: never
+        if (mbytes >= 100) return a.m >= (a.b_bits == 8 ? 4u : 5u);
+        if (a.k >= 8192 && mbytes >= 20) return a.m >= 8;
+        return mbytes >= 40 && a.m >= 9;
+    }
+    if (a.m <= 128) {
+        // Both other forms unpack at the pace of one step's hand-off chain (79 to 88 us on 28672 x 8192 whatever M is: 45 to 69 here;
+        // 8192 x 8192: 29 to 31 / 24 to 31 int8, 41 / 23 to 31 int4; 12288 x 4096: 29 to 38 / 22 to 30).  On small matrices what
+        // remains is the cost of sharing tiles between CTAs (4096 x 4096: 16 / 17 to 22 int8, 18 / 16 to 23 int4).
+        return weights >= 40e6 || (a.b_bits == 4 && a.m <= 40);
+    }
+    // Many rows: the tensor-memory form with 256-row tiles has the higher rate, this one fits its tiles to M and shares the last
+    // ones evenly.  Group-scaled int4 is bound by the unpack there and faster here throughout (28672 x 8192 group 128: 154 / 113 at
+    // M = 256, 245 / 222 at 512, 971 / 915 at 2048, 1904 / 1819 at 4096; 4096 x 4096: 30 / 31 at 512, 72 / 69 at 2048).
+    if (a.b_bits == 4 && a.group_size) return weights >= 40e6 || weights * a.m >= 30e9;
+    // Otherwise compared in rows per SM, with 1.2 for the difference in rate (int8: 28672 x 8192: 117 / 99 at M = 129, 182 / 164 at
+    // 333, 186 / 213 at 512; 11008 x 4096: 50 / 43 at 333, 51 / 50 at 512, 81 / 71 at 777, 138 / 160 at 2048).
+    if (weights < 40e6) return false;
+    const uint32_t n_tiles = (a.n + kCh - 1) / kCh, rows = tile_rows(a);
+    const uint32_t others = (a.m + 255) / 256 * n_tiles, waves = others / sms, rest = others % sms;
+    const uint32_t parts = rest == 0 || rest > sms / 2 ? 1 : sms / rest < 4 ? sms / rest : 4;
+    const double there = 256.0 * (waves + (rest ? 1.0 / parts : 0.0)), here = (double)((a.m + rows - 1) / rows) * n_tiles * rows / sms;
+    return 1.2 * here < there;
+}
+
+}  // namespace
+
+int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, bool* done) {
+    *done = false;
+    const char* env = getenv("AFB_STREAM");   // tuning aid: 1 wherever possible, 0 never
+    const int forced = env ? atoi(env) : -1;
+    if (forced == 0 || !stream_supports(a) || (forced < 0 && !is_faster(a, (uint32_t)ctx->sm_count))) return AFB_OK;
+    const uint32_t sms = (uint32_t)ctx->sm_count;
+    StreamParams p{};
+    p.c = reinterpret_cast<uint16_t*>(a.ptr_c);
+    p.scale = a.ptr_scale;
+    p.zero = reinterpret_cast<const uint8_t*>(a.ptr_zero);
+    p.m = a.m; p.n = a.n; p.k = a.k; p.ldc = a.ldc;
+    p.enc = a.b_encoding; p.scale_dtype = a.scale_dtype;
+    p.packed = a.b_layout == AFB_LAYOUT_COL_PACKED ? 1u : 0u;
+    const int mode = !a.group_size ? kChannel : a.m > 16 ? kFold : kSums;
+    p.rows = tile_rows(a);
+    p.m_tiles = (a.m + p.rows - 1) / p.rows;
+    p.n_tiles = (a.n + kCh - 1) / kCh;
+    p.group_m = pick_group_m(a, p.m_tiles, p.n_tiles, p.rows, ctx->sm_count);
+    // k per step: 128 halves the number of hand-offs per weight, which is what bounds few rows; more rows need the tensor memory
+    // for their accumulators, and steps of 64 keep the tensor cores busy for longer than a hand-off takes
+    const uint32_t ks = p.rows <= 128 && a.k % 128 == 0 && a.group_size % 128 == 0 ? 128 : 64;
+    const uint32_t spb = (a.b_bits == 8 ? 128 : 256) / ks;
+    p.parts = a.k / ks;
+    p.blocks = (p.parts + spb - 1) / spb;
+    while (a.group_size && ks << p.group_shift < a.group_size) ++p.group_shift;
+    p.flush = mode == kSums ? (1u << p.group_shift < spb ? 1u << p.group_shift : spb) : 0;
+    p.acc_cols = mode == kSums ? kSet * 16 : p.rows;
+    p.accs = mode == kSums ? 4 : p.rows <= 192 ? 2 : 1;
+    const uint32_t pair = ks == 128 && p.rows <= 64 ? 2 : 1;
+    p.slots = (kTmemCols - p.accs * p.acc_cols) / (pair * ks / 2);
+    if (p.slots > (uint32_t)kMaxSlots) p.slots = kMaxSlots;
+    const uint32_t act_bytes = p.rows * ks * 2 * pair;
+    while (p.slots * pair > (uint32_t)kGroups && (kRingBudget - p.slots * act_bytes) / kRawBytes < p.slots * pair) --p.slots;
+    p.raw_stages = (kRingBudget - p.slots * act_bytes) / kRawBytes;
+    if (p.raw_stages > (uint32_t)kMaxRaw) p.raw_stages = kMaxRaw;
+
+    // A converter warp sees only every fourth part, and a wait for phase n of a raw stage means something only once phase n - 1 has
+    // completed.  What tells it that is the MMA order: a free slot means that everything up to `slots` steps earlier has been
+    // consumed.  With the slot wait of the PREVIOUS part behind it, up to 3 + slots * pair earlier parts may still be under way,
+    // with that of its own part up to slots * pair - 1; a raw block has at least one part, so the ring must be longer than that.
+    p.slot_first = p.raw_stages >= kGroups + p.slots * pair ? 0u : 1u;
+    if (p.raw_stages < p.slots * pair || p.slots * pair < (uint32_t)kGroups) return AFB_OK;
+
+    const uint32_t tiles = p.m_tiles * p.n_tiles;
+    uint32_t grid = sms;
+    const uint32_t waves = tiles / sms, rest = tiles - waves * sms;
+    if (rest == 0) { p.shared_tiles = 0; p.whole_waves = waves; }
+    else if (waves == 0) { p.shared_tiles = tiles; p.whole_waves = 0; }
+    else if (rest * 4 >= sms) { p.shared_tiles = rest; p.whole_waves = waves; }
+    else { p.shared_tiles = sms + rest; p.whole_waves = waves - 1; }
+    if (p.shared_tiles && p.whole_waves == 0 && (uint64_t)p.shared_tiles * p.blocks < grid) grid = p.shared_tiles * p.blocks;
+    if (p.shared_tiles) {
+        if (p.shared_tiles > ctx->splitk_counter_count || (size_t)2 * grid * p.rows * kCh * sizeof(float) > ctx->splitk_ws_bytes) return AFB_OK;
+        int rc = AFB_OK;
+        const DeviceCtx::Workspace* w = workspace_for(ctx, s, &rc, true);
+        if (!w) return rc;   // the caller's other forms
+
+        p.ws = w->ws; p.counters = w->counters;
+    }
+    p.status = ctx->status;
+
+    *done = true;
+    CUtensorMap ta, tw;
+    int rc = tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.ptr_a, a.k, a.m, (uint64_t)a.lda * 2, kSlab, p.rows, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    rc = tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, a.ptr_b, (uint64_t)a.k * a.b_bits / 8, a.n, (uint64_t)a.ldb * a.b_bits / 8, 128, kCh,
+                 CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    CUtensorMap tc = ta;
+    p.c_tma = a.ldc % 8 == 0 && (uintptr_t)a.ptr_c % 16 == 0 && a.n % 8 == 0 &&
+              tmap_2d(&tc, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.ptr_c, a.n, a.m, (uint64_t)a.ldc * 2, 32, 16, CU_TENSOR_MAP_SWIZZLE_NONE) == AFB_OK;
+    p.c_vec = a.ldc % 4 == 0 && (uintptr_t)a.ptr_c % 8 == 0;
+    p.finish_late = p.whole_waves == 0 || (p.whole_waves == 1 && p.rows > 32);
+    const bool pdl = (a.flags & AFB_FLAG_PDL) != 0 && a.m <= 16;   // of the decode variant only
+#define AFB_STREAM_LAUNCH(B, M) (pair == 2 ? launch_cfg<B, M, 128, 2>(ta, tw, tc, p, grid, pdl, ctx, s) : ks == 128 ? launch_cfg<B, M, 128, 1>(ta, tw, tc, p, grid, pdl, ctx, s) : launch_cfg<B, M, 64, 1>(ta, tw, tc, p, grid, pdl, ctx, s))
+    if (a.b_bits == 8) return mode == kChannel ? AFB_STREAM_LAUNCH(8, kChannel) : mode == kFold ? AFB_STREAM_LAUNCH(8, kFold) : AFB_STREAM_LAUNCH(8, kSums);
+    return mode == kChannel ? AFB_STREAM_LAUNCH(4, kChannel) : mode == kFold ? AFB_STREAM_LAUNCH(4, kFold) : AFB_STREAM_LAUNCH(4, kSums);
+#undef AFB_STREAM_LAUNCH
+}
+
+}  // namespace afb

@@ -1,0 +1,64 @@
+"""The streaming form of the decode and prefill variants (csrc/stream.cu), forced onto small problems, against the CPU oracle.
+
+The sizes are those at which it can go wrong: activation rows around its tile heights (16, 64, 128, 192) and modes (up to 16 rows
+group scales multiply fp32 sums, above that the weights), K that leaves raw blocks and steps incomplete, channels that end inside a
+tile, fewer units of work than CTAs, tiles shared by many CTAs, whole waves next to shared tiles."""
+import numpy as np
+import pytest
+
+import afb_testlib as T
+import awesome_fusion_b200 as pkg
+from test_gpu_parity import check_close
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(afb, oracle, case, what, **kw):
+    got, _ = T.run_case(afb, case, **kw)
+    again, _ = T.run_case(afb, case, **kw)
+    assert np.array_equal(got, again), f"{what}: two runs differ"
+    folded = case.group and case.m > 16   # the weights are rounded to bf16 once more, as in the other prefill forms
+    check_close(oracle, oracle.gemm(case, threads=8, round_w=bool(folded)), got, what)
+    return got
+
+
+@pytest.fixture(autouse=True)
+def _forced(monkeypatch):
+    monkeypatch.setenv("AFB_STREAM", "1")
+
+
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 65, 128, 129, 192, 193, 385])
+@pytest.mark.parametrize("bits,group,n,k", [(8, 0, 264, 64), (8, 0, 1000, 960), (8, 0, 128, 4096), (4, 0, 392, 320), (4, 128, 520, 1152), (4, 256, 264, 2304),
+                                            (4, 64, 136, 704), (8, 128, 264, 640), (8, 64, 264, 448)])
+def test_rows_and_ragged_k(afb, oracle, m, bits, group, n, k):
+    case = T.make_case(m, n, k, bits=bits, group=group, enc=m & 1, seed=m + k, scale_range=(0.005, 0.05))
+    _check(afb, oracle, case, f"int{bits} g{group} {m}x{n}x{k}")
+
+
+@pytest.mark.parametrize("m,n,k,bits,group", [(16, 28672, 1024, 8, 0), (40, 20008, 640, 8, 0), (3, 24000, 1280, 4, 128), (128, 19200, 768, 4, 128),
+                                              (700, 6152, 512, 8, 0), (1400, 4104, 512, 4, 128)])
+def test_whole_waves_and_shared_tiles(afb, oracle, m, n, k, bits, group):
+    case = T.make_case(m, n, k, bits=bits, group=group, seed=5, scale_range=(0.005, 0.05))
+    _check(afb, oracle, case, f"int{bits} g{group} {m}x{n}x{k}")
+
+
+@pytest.mark.parametrize("m", [7, 16, 100])
+@pytest.mark.parametrize("bits,group", [(8, 0), (8, 128), (4, 0), (4, 128), (4, 64)])
+def test_zero_points_and_packed_layout(afb, oracle, m, bits, group):
+    case = T.make_case(m, 520, 1280, bits=bits, group=group, enc=1, seed=m + bits, zero_points=True, scale_range=(0.005, 0.05))
+    got = _check(afb, oracle, case, f"zero-points int{bits} g{group} m{m}")
+    assert np.array_equal(got, _check(afb, oracle, oracle.prepack(case), f"packed, zero-points int{bits} g{group} m{m}"))
+
+
+@pytest.mark.parametrize("m,ldc", [(9, 269), (16, 268), (1, 265)])
+@pytest.mark.parametrize("bits,group", [(8, 0), (4, 128)])
+def test_result_rows_that_no_tile_store_takes(afb, oracle, m, ldc, bits, group):
+    """Decode calls may have any ldc and any number of channels: register stores, and nothing written outside C."""
+    case = T.make_case(m, 261, 2048, bits=bits, group=group, seed=m, scale_range=(0.005, 0.05))
+    _check(afb, oracle, case, f"ldc {ldc} int{bits}", ldc=ldc)
+
+
+def test_bf16_group_scales_in_fp32_and_pdl(afb, oracle):
+    for group, dtype, flags in [(128, 0, 0), (0, 1, 0), (128, 1, pkg.FLAG_PDL), (0, 0, pkg.FLAG_PDL)]:
+        case = T.make_case(12, 776, 3072, bits=4, group=group, scale_dtype=dtype, seed=3, scale_range=(0.005, 0.05))
+        _check(afb, oracle, case, f"scale dtype {dtype} flags {flags}", flags=flags)
