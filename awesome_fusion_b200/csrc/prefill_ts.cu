@@ -47,7 +47,7 @@ struct TsParams {
     uint32_t m_rot;        // row tiles are taken in rotated order, starting at this one (spreads the peers a rank pushes to)
     uint32_t group_m;      // tile order: groups of group_m row tiles; inside a group the channel tiles advance, row tile fastest
     uint32_t c_f32;
-    uint32_t c_tma;        // bf16 C goes out as tile stores through shared memory (tmap_c is valid): plain GEMM, no fusion, no exchange
+    uint32_t c_tma;        // bf16 C goes out as tile stores through shared memory (tmap_c is valid): every bf16 result but those of the exchange forms
     uint32_t packed;       // B is in the pre-packed order of afb_prepack: the cheap unpack yields consecutive k
     uint32_t exact;        // group scales only: the weight q * s goes to the tensor cores as TWO bf16 terms, hi = bf16_rn(q * s) and
                            // lo = q * s - hi (exact: the product has at most 16 significant bits), in two TMEM slots and two MMAs
@@ -432,6 +432,26 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
                 if (sa == kSlotsA) { sa = 0; pa ^= 1u; }
             }
             if (!ok) break;
+            // Fused epilogue: the residual of the first block is fetched while the tile's last MMAs run.  (Fetched one element at a time
+            // between the stores, it made the epilogue take 370 us of 1000 x 2*11008 x 4096: each load waited for the one before.)
+            constexpr int kColsPerWarp = BMA / kKParts;   // the warps of a lane quarter split the activation rows
+            const bool gated = (p.fused & 2u) != 0;
+            const uint32_t nout = gated ? (nn >> 1) : nn;
+            uint32_t res_next[16];   // two rows each
+            auto load_residual = [&](int c0) {
+                if (!p.residual || c0 >= kColsPerWarp) return;
+                const uint32_t row0 = m0 + kq * kColsPerWarp + c0 + (gated && (lane & 1) ? 16u : 0u);
+                const uint16_t* src = p.residual + (size_t)row0 * p.ld_res + nout;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (gated && j >= 8) break;
+                    const uint32_t lo = nn < p.n && row0 + 2 * j < p.m ? src[(size_t)(2 * j) * p.ld_res] : 0u;
+                    const uint32_t hi = nn < p.n && row0 + 2 * j + 1 < p.m ? src[(size_t)(2 * j + 1) * p.ld_res] : 0u;
+                    res_next[j] = lo | hi << 16;
+                }
+            };
+            if (p.fused) load_residual(0);
+            const float bias = (p.bias && nn < p.n) ? p.bias[nn] : 0.f;
             // ---- epilogue of this tile: the accumulator is complete once the last MMA has been committed ----
             if (!wait_or_abort(bar_acc_full, it & 1u, abort_flag)) {
                 if (!*abort_flag) { report_timeout(p.status, 25, (int)t, -1); *abort_flag = 1; }
@@ -447,7 +467,6 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
                 if (!*abort_flag) { report_timeout(p.status, 26, (int)t, -1); *abort_flag = 1; }
                 break;
             }
-            constexpr int kColsPerWarp = BMA / kKParts;   // the warps of a lane quarter split the activation rows
 #pragma unroll 1
             for (int c0 = 0; c0 < kColsPerWarp; c0 += 32) {
                 uint32_t r[32];
@@ -459,25 +478,44 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
 #pragma unroll
                     for (int j = 0; j < 32; ++j) __stcg(wsp + (size_t)j * BNW, __uint_as_float(r[j]));
                 } else if (p.fused) {
-                    // every lane takes part (the gated form exchanges values between the two lanes of a pair): range checks only guard the accesses
-                    const uint32_t mrow = m0 + col;
-                    const bool gated = (p.fused & 2u) != 0;
-                    const float bias = (p.bias && nn < p.n) ? p.bias[nn] : 0.f;
-                    const uint32_t nout = gated ? (nn >> 1) : nn;
-                    const bool writer = nn < p.n && (!gated || (lane & 1) == 0);
+                    // Gated: the lanes of a pair hold gate (even) and up (odd) of one output channel for 32 rows.  They exchange half of
+                    // their rows, so that the even lane finishes rows 0-15 of the block and the odd lane rows 16-31.  Otherwise every
+                    // lane finishes its channel's 32 rows.
+                    const uint32_t mrow = m0 + col, out = smem_base + L::kOffOut + (uint32_t)(warp - 2) * L::kStageOutBytes;
+                    uint32_t res[16];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        float v = fmaf(__uint_as_float(r[j]), scale, bias);
-                        if (gated) {   // even lane: gate, odd lane: up
-                            const float other = __shfl_xor_sync(0xffffffffu, v, 1);
-                            if (p.act == AFB_ACT_SILU) v = v / (1.f + __expf(-v));
-                            v *= other;
-                        } else if (p.act == AFB_ACT_SILU) {
-                            v = v / (1.f + __expf(-v));
+                    for (int j = 0; j < 16; ++j) res[j] = res_next[j];
+                    load_residual(c0 + 32);   // of the next block, while this one is finished
+                    if (p.c_tma) {
+                        if (lane == 0) ptx::bulk_wait_group_read0();   // the previous block of this warp has been read out
+                        __syncwarp();
+                    }
+                    auto finish = [&](float gate, float up, uint32_t j, uint32_t row) {   // j: which of the lane's rows
+                        float v = p.act == AFB_ACT_SILU ? gate / (1.f + __expf(-gate)) : gate;
+                        if (gated) v *= up;
+                        if (p.residual) v += __uint_as_float((j & 1) ? res[j / 2] & 0xffff0000u : res[j / 2] << 16);
+                        const uint16_t o = __bfloat16_as_ushort(__float2bfloat16_rn(v));
+                        if (p.c_tma) asm volatile("st.shared.u16 [%0], %1;" ::"r"(out + (gated ? row * 32u + ((uint32_t)lane >> 1) * 2u : row * 64u + (uint32_t)lane * 2u)), "h"(o) : "memory");
+                        else if (nn < p.n && mrow + row < p.m) p.c[(size_t)(mrow + row) * p.ldc + nout] = o;
+                    };
+                    if (gated) {
+                        const bool odd = lane & 1;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const float lo = fmaf(__uint_as_float(r[j]), scale, bias), hi = fmaf(__uint_as_float(r[j + 16]), scale, bias);
+                            const float other = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
+                            finish(odd ? other : lo, odd ? hi : other, (uint32_t)j, odd ? 16u + j : (uint32_t)j);
                         }
-                        if (writer && mrow + j < p.m) {
-                            if (p.residual) v += __uint_as_float((uint32_t)p.residual[(size_t)(mrow + j) * p.ld_res + nout] << 16);
-                            p.c[(size_t)(mrow + j) * p.ldc + nout] = __bfloat16_as_ushort(__float2bfloat16_rn(v));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) finish(fmaf(__uint_as_float(r[j]), scale, bias), 0.f, (uint32_t)j, (uint32_t)j);
+                    }
+                    if (p.c_tma) {
+                        ptx::fence_proxy_async_smem();
+                        __syncwarp();
+                        if (lane == 0) {
+                            ptx::tma_store_2d(&tmap_c, out, (int)(gated ? (n0 + q * 32u) >> 1 : n0 + q * 32u), (int)mrow);
+                            ptx::bulk_commit_group();
                         }
                     }
                 } else if (p.c_tma) {
@@ -779,14 +817,15 @@ int launch_ts_cfg(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, uint32
                     BITS == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
     if (rc) return rc;
     TsParams p;
-    // bf16 C of a plain GEMM leaves through tile stores (32 channels x 32 rows per store); every other form stores from registers
+    // bf16 C leaves through tile stores (32 channels x 32 rows per store, 16 x 32 of a gated result); the exchange forms store from registers
+    const bool gated = fused && fused->gated;
     CUtensorMap tc = ta;
     p.c_tma = 0;
     {
         const char* e = getenv("AFB_PREFILL_TILE_STORE");   // tuning aid: 0 switches it off
         const bool wanted = !(e && atoi(e) == 0);
-        if (wanted && !(a.flags & AFB_FLAG_C_F32) && !tile_done && !push && !fused && a.ldc % 8 == 0 && (uintptr_t)a.ptr_c % 16 == 0 &&
-            ts_tmap_2d(&tc, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.ptr_c, a.n, a.m, (uint64_t)a.ldc * 2, 32, 32, CU_TENSOR_MAP_SWIZZLE_NONE) == AFB_OK)
+        if (wanted && !(a.flags & AFB_FLAG_C_F32) && !tile_done && !push && a.ldc % 8 == 0 && (uintptr_t)a.ptr_c % 16 == 0 &&
+            ts_tmap_2d(&tc, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.ptr_c, gated ? a.n / 2 : a.n, a.m, (uint64_t)a.ldc * 2, gated ? 16 : 32, 32, CU_TENSOR_MAP_SWIZZLE_NONE) == AFB_OK)
             p.c_tma = 1;
     }
     p.c = reinterpret_cast<uint16_t*>(a.ptr_c);

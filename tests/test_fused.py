@@ -101,3 +101,29 @@ def test_fused_launch_refuses_what_it_cannot_do(afb):
     assert afb.gemm_fused_launch_status(afb.make_fused_args(a)) == -2                      # bf16 output only
     a = afb.make_args(0x1000, 0x1000, 0x1000, 0x1000, 64, 128, 256, layout=pkg.LAYOUT_ROW, ldb=128)
     assert afb.gemm_fused_launch_status(afb.make_fused_args(a)) == -2
+
+
+@pytest.mark.parametrize("m,n", [(257, 136), (300, 264), (64, 72)])
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("tile_store", ["1", "0"])
+def test_in_place_residual_and_padded_rows(afb, oracle, monkeypatch, m, n, gated, tile_store):
+    """The residual may be C itself; rows of C and of the residual may be padded, and the padding stays as it was.  Both ways out
+    (tile stores and register stores) at the edges of tiles."""
+    monkeypatch.setenv("AFB_PREFILL_TILE_STORE", tile_store)
+    rows = 2 * n if gated else n
+    case = T.make_case(m, rows, 512, seed=m + n, scale_range=(0.002, 0.01))
+    v = oracle.gemm(case, threads=8)
+    ldc = n + 24
+    before = T.np_bf16_rne(np.random.default_rng(9).standard_normal((m, ldc), dtype=np.float32))
+    want = (silu(v[:, 0::2]) * v[:, 1::2] if gated else silu(v)) + T.np_bf16_to_f32(before[:, :n])
+    d_a, d_b, d_s, d_c = (afb.to_device(x) for x in (case.a, case.b, case.scale, before))
+    try:
+        args = afb.make_args(d_c, d_a, d_b, d_s, m, rows, 512, ldc=ldc)
+        afb.gemm_fused_launch(afb.make_fused_args(args, gated=gated, activation=pkg.ACT_SILU, residual=d_c, ld_residual=ldc))
+        afb.device_sync()
+        got = afb.to_host(d_c, (m, ldc), np.uint16)
+    finally:
+        for p in (d_a, d_b, d_s, d_c):
+            afb.free(p)
+    check_close(oracle, want, np.ascontiguousarray(got[:, :n]), f"in-place residual gated={gated} {m}x{n}")
+    assert np.array_equal(got[:, n:], before[:, n:])
