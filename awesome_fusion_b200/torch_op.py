@@ -49,15 +49,21 @@ def bf16_aintb_gemm(a: torch.Tensor, b: torch.Tensor, scale: torch.Tensor, bits:
     m, n, k = _check(a, b, scale, bits, group_size)
     if not (a.is_contiguous() and b.is_contiguous() and scale.is_contiguous()):
         raise ValueError("a, b and scale must be contiguous")
-    lib = load()
     dev = a.device.index if a.device.index is not None else torch.cuda.current_device()
-    with torch.cuda.device(dev):
-        lib.init(dev)
-        out = torch.empty((m, n), device=a.device, dtype=torch.bfloat16)
-        args = lib.make_args(out, a, b, scale, m, n, k, bits=bits, group=group_size,
-                             encoding=ENC_OFFSET if offset_binary else ENC_TWOS,
-                             scale_dtype=SCALE_BF16 if scale.dtype == torch.bfloat16 else SCALE_F32, flags=flags)
-        lib.gemm_launch(args, torch.cuda.current_stream().cuda_stream)
+    if dev != torch.cuda.current_device():   # the guard costs a microsecond or two: only where there is a device to come back to
+        with torch.cuda.device(dev):
+            return _launch(dev, a, b, scale, m, n, k, bits, group_size, offset_binary, flags)
+    return _launch(dev, a, b, scale, m, n, k, bits, group_size, offset_binary, flags)
+
+
+def _launch(dev, a, b, scale, m, n, k, bits, group_size, offset_binary, flags):
+    lib = load()
+    lib.init(dev)
+    out = torch.empty((m, n), device=a.device, dtype=torch.bfloat16)
+    args = lib.make_args(out, a, b, scale, m, n, k, bits=bits, group=group_size,
+                         encoding=ENC_OFFSET if offset_binary else ENC_TWOS,
+                         scale_dtype=SCALE_BF16 if scale.dtype == torch.bfloat16 else SCALE_F32, flags=flags)
+    lib.gemm_launch(args, torch.cuda.current_stream(dev).cuda_stream)
     return out
 
 
