@@ -65,7 +65,7 @@ struct TsParams {
     const float* bias;
     const uint16_t* residual;
     uint32_t ld_res;
-    uint32_t fused;        // 0: off; bit 0: on; bit 1: gated
+    uint32_t fused;        // 0: off; bit 0: on (the FUSED instances); bit 1: gated
     uint32_t act;          // AFB_ACT_*
     uint32_t push_rows, push_rank;
     // optional (pipelined reduce-scatter): the tiles are taken in units of (owner's row tiles) x (n_tiles / push_sub channel tiles);
@@ -135,7 +135,8 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
     return true;
 }
 
-template <int BITS, bool GROUPED, int BMA>
+// FUSED: instances of afb_gemm_fused_launch (the fused epilogue's registers would cost the plain instances spills)
+template <int BITS, bool GROUPED, int BMA, bool FUSED>
 __global__ void __launch_bounds__(kThreadsFwd, 1)
 prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_w,
                   const __grid_constant__ CUtensorMap tmap_c, const TsParams p) {
@@ -435,7 +436,7 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
             // Fused epilogue: the residual of the first block is fetched while the tile's last MMAs run.  (Fetched one element at a time
             // between the stores, it made the epilogue take 370 us of 1000 x 2*11008 x 4096: each load waited for the one before.)
             constexpr int kColsPerWarp = BMA / kKParts;   // the warps of a lane quarter split the activation rows
-            const bool gated = (p.fused & 2u) != 0;
+            const bool gated = FUSED && (p.fused & 2u) != 0;
             const uint32_t nout = gated ? (nn >> 1) : nn;
             uint32_t res_next[16];   // two rows each
             auto load_residual = [&](int c0) {
@@ -450,8 +451,8 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
                     res_next[j] = lo | hi << 16;
                 }
             };
-            if (p.fused) load_residual(0);
-            const float bias = (p.bias && nn < p.n) ? p.bias[nn] : 0.f;
+            if (FUSED) load_residual(0);
+            const float bias = (FUSED && p.bias && nn < p.n) ? p.bias[nn] : 0.f;
             // ---- epilogue of this tile: the accumulator is complete once the last MMA has been committed ----
             if (!wait_or_abort(bar_acc_full, it & 1u, abort_flag)) {
                 if (!*abort_flag) { report_timeout(p.status, 25, (int)t, -1); *abort_flag = 1; }
@@ -477,7 +478,7 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
                     float* wsp = p.tail_ws + ((size_t)(w.tail_r * p.tail_parts + w.part) * BMA + col) * BNW + ch;
 #pragma unroll
                     for (int j = 0; j < 32; ++j) __stcg(wsp + (size_t)j * BNW, __uint_as_float(r[j]));
-                } else if (p.fused) {
+                } else if (FUSED) {
                     // Gated: the lanes of a pair hold gate (even) and up (odd) of one output channel for 32 rows.  They exchange half of
                     // their rows, so that the even lane finishes rows 0-15 of the block and the odd lane rows 16-31.  Otherwise every
                     // lane finishes its channel's 32 rows.
@@ -890,12 +891,12 @@ int launch_ts_cfg(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, uint32
     for (uint32_t q = 0; q < AFB_MAX_RANKS; ++q) p.push[q] = (push && q < push_world) ? reinterpret_cast<float*>(push[q]) : nullptr;
     p.status = ctx->status;
     p.ts = push ? phase_ts_if_enabled(ctx) : nullptr;
-    auto kern = prefill_ts_kernel<BITS, GROUPED, BMA>;
-    static DeviceOnce attr_set;  // per template instance
-    if (!attr_set.done(ctx->device)) {
+    auto kern = fused ? prefill_ts_kernel<BITS, GROUPED, BMA, true> : prefill_ts_kernel<BITS, GROUPED, BMA, false>;
+    static DeviceOnce attr_set[2];  // per template instance
+    if (!attr_set[fused ? 1 : 0].done(ctx->device)) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
         if (e != cudaSuccess) return cuda_fail(e);
-        attr_set.mark(ctx->device);
+        attr_set[fused ? 1 : 0].mark(ctx->device);
     }
     const uint32_t tiles = p.m_tiles * p.n_tiles;
     uint32_t grid = tiles < (uint32_t)ctx->sm_count ? tiles : (uint32_t)ctx->sm_count;
