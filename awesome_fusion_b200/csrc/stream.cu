@@ -24,7 +24,7 @@
 //
 // What bounds it: for few rows int8 the weight stream (28672 x 8192, 16 rows: 44.7 us = 5.3 TB/s of weights, 63.8 with decode.cu; the
 // stream, the hand-offs and the shared tiles alone, without unpack and MMAs, take 44.7 too), int4 the issue slots of the unpack and of
-// the hand-offs (53 against 63 us; 40 without unpack and MMAs); for 65 to 128 rows the activations through L2 (28672 x 8192 int4
+// the hand-offs (50 against 63 us; 40 without unpack and MMAs); for 65 to 128 rows the activations through L2 (28672 x 8192 int4
 // group-128, 128 rows: 66 us, 82 with prefill.cu); for many rows the pace of the issuing warp next to the unpack.
 #include <cstdlib>
 #include "afb_internal.h"
@@ -43,8 +43,8 @@ constexpr int kFirstEpi = 4, kFirstConv = 8;
 constexpr int kThreads = 32 * (kFirstConv + 4 * kGroups);
 constexpr int kMaxRaw = 12, kMaxSlots = 8, kMaxAcc = 8;
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kSet = 2;            // kSums: group sums handed to the epilogue at a time
-constexpr int kBars = 2 * (kMaxRaw + kMaxSlots + kMaxAcc) + 3;
+constexpr uint32_t kSet = 4;            // kSums: group sums handed to the epilogue at a time (5 x 28672 x 8192 int4: 51.5 us with 2, 50.4 with 4)
+constexpr int kBars = 2 * (kMaxRaw + kMaxSlots + kMaxAcc) + kMaxSlots + 3;
 constexpr int kOffMisc = kBars * 8, kOffOut = 1024;
 constexpr int kOutBytes = 16 * 32 * 2;                    // one block of the result: 16 rows x 32 channels
 constexpr int kOffRaw = kOffOut + 4 * 2 * kOutBytes;      // two blocks per epilogue warp
@@ -149,6 +149,11 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
     auto raw_empty = [&](uint32_t s) { return bar(kMaxRaw + s); };
     auto step_full = [&](uint32_t s) { return bar(2 * kMaxRaw + s); };                // converted weights in TMEM, activations in shared memory
     auto step_empty = [&](uint32_t s) { return bar(2 * kMaxRaw + kMaxSlots + s); };   // the MMAs of the step are done with both
+    // The arrival of a step's activations.  Where a step is two parts (few rows) a converter warp waits for it before it reports its part,
+    // so that the issuing warp, whose own instructions set the pace there, has one thing to wait for that is usually complete (28672 x
+    // 8192, 1 row: 43.3 -> 41.9 us int8); with more rows it counts into step_full (39 against 38 us on 333 x 11008 x 4096 otherwise).
+    constexpr bool kActApart = PAIR == 2;
+    auto act_full = [&](uint32_t s) { return kActApart ? bar(2 * (kMaxRaw + kMaxSlots + kMaxAcc) + s) : step_full(s); };
     auto acc_full = [&](uint32_t s) { return bar(2 * (kMaxRaw + kMaxSlots) + s); };
     auto acc_empty = [&](uint32_t s) { return bar(2 * (kMaxRaw + kMaxSlots) + kMaxAcc + s); };
     // a shared tile: every epilogue warp has published its part; the count has been taken.  The end: the epilogue is through
@@ -171,7 +176,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
     } else {
         if (warp == 1 && lane == 0) {
-            for (uint32_t s = 0; s < p.slots; ++s) { ptx::mbar_init(step_full(s), 4 * PAIR + 1); ptx::mbar_init(step_empty(s), 1); }
+            for (uint32_t s = 0; s < p.slots; ++s) { ptx::mbar_init(step_full(s), kActApart ? 4 * PAIR : 4 * PAIR + 1); ptx::mbar_init(step_empty(s), 1); if (kActApart) ptx::mbar_init(act_full(s), 1); }
             for (uint32_t s = 0; s < p.accs; ++s) { ptx::mbar_init(acc_full(s), 1); ptx::mbar_init(acc_empty(s), 4); }
             ptx::mbar_init(bar_stored, 4);
             ptx::mbar_init(bar_verdict, 1);
@@ -288,18 +293,18 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
             for (uint32_t l = 0; l < ns; l += PAIR) {
                 if (!warp_wait(step_empty(r.i), r.phase ^ 1u, abort_flag)) { give_up(32, x.t, l); ok = false; break; }
                 if (ptx::elect_one()) {
-                    ptx::mbar_arrive_expect_tx(step_full(r.i), l + PAIR <= ns ? act_bytes : part_bytes);
+                    ptx::mbar_arrive_expect_tx(act_full(r.i), l + PAIR <= ns ? act_bytes : part_bytes);
 #pragma unroll
                     for (int h = 0; h < PAIR * KS / kSlab; ++h)
                         if (PAIR == 1 || h < KS / kSlab || l + 1 < ns)
-                            ptx::tma_load_2d(smem_base + off_act + r.i * act_bytes + h * slab_bytes, &tmap_act, (int)((k0 + l) * KS + h * kSlab), (int)m0, step_full(r.i));
+                            ptx::tma_load_2d(smem_base + off_act + r.i * act_bytes + h * slab_bytes, &tmap_act, (int)((k0 + l) * KS + h * kSlab), (int)m0, act_full(r.i));
                 }
                 issued |= 1u << r.i; parity = (parity & ~(1u << r.i)) | (r.phase << r.i);
                 r.step(1, p.slots);
             }
         }
         for (uint32_t s = 0; s < p.slots; ++s)
-            if (issued & (1u << s)) ptx::mbar_wait(step_full(s), (parity >> s) & 1u);   // after an abort the converters' part may be missing: then the limit of the wait, far above the time of a copy
+            if (issued & (1u << s)) ptx::mbar_wait(act_full(s), (parity >> s) & 1u);   // after an abort the converters' part may be missing: then the limit of the wait, far above the time of a copy
     } else if (warp == 2) {
         // ======================= MMA issuer =======================
         const uint32_t idesc = ptx::umma_idesc_bf16_f32(kCh, p.rows);
@@ -421,6 +426,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                     ptx::tmem_st_32x32(slot_base + ((quarter * 32u) << 16) + rs.i * kSlotCols + (l % PAIR) * kPartCols + h * 32, o);
                 }
                 if (!ok) break;
+                if (kActApart && quarter == 0 && !warp_wait(act_full(rs.i), rs.phase, abort_flag)) { give_up(39, x.t, l); ok = false; break; }
                 ptx::tmem_st_wait();
                 ptx::tc_fence_before_sync();
                 __syncwarp();   // every lane's weights are in tensor memory
@@ -671,7 +677,7 @@ bool is_faster(const afb_gemm_args& a, uint32_t sms) {
     if (a.m <= 16) {
         // The decode kernel has about 9 us less to set up and finish, and its arithmetic grows with M; this form's does not.
         //   28672 x 8192 int8   M = 2: 44 / 44   4: 51 / 44    8: 68 / 44   16: 64 / 45
-        //   28672 x 8192 int4   M = 1: 40 / 53   4: 53 / 53    8: 64 / 53   16: 63 / 53    (group 128)
+        //   28672 x 8192 int4   M = 1: 40 / 50   4: 53 / 50    8: 64 / 50   16: 63 / 50    (group 128)
         //   12288 x 4096 int8   M = 1: 14 / 22   8: 21 / 22   16: 27 / 22
         //    4096 x 11008 int4  M = 1: 14 / 21   4: 22 / 21    8: 30 / 21   16: 31 / 22    (one activation row is staged in several passes)
         //   12288 x 4096 int4   M = 8: 18 / 24  16: 23 / 23;   4096 x 4096: never
@@ -728,7 +734,7 @@ int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, boo
     while (a.group_size && ks << p.group_shift < a.group_size) ++p.group_shift;
     p.flush = mode == kSums ? (1u << p.group_shift < spb ? 1u << p.group_shift : spb) : 0;
     p.acc_cols = mode == kSums ? kSet * 16 : p.rows;
-    p.accs = mode == kSums ? 4 : p.rows <= 192 ? 2 : 1;
+    p.accs = p.rows <= 192 ? 2 : 1;
     const uint32_t pair = ks == 128 && p.rows <= 64 ? 2 : 1;
     p.slots = (kTmemCols - p.accs * p.acc_cols) / (pair * ks / 2);
     if (p.slots > (uint32_t)kMaxSlots) p.slots = kMaxSlots;
