@@ -402,7 +402,8 @@ static void pick_shape(const afb_gemm_args& a, int sm_count, int ctas_per_sm, si
     // round trip; measured on 4096 x 4096: 10.2 vs 12.4 us at m = 9, 11.9 vs 12.6 at m = 12, equal at m = 16)
     if (weight_mb < 48.0 && a.m > 8 && ctas(1) >= sms * 3 / 2 && (size_t)a.m * (ch * kWarps * 2 + 16) <= act_cap) wr = 1;
     while (wr < 8 && (size_t)a.m * (ch * (kWarps / wr) * 2 + 16) > act_cap) wr *= 2;   // one round of the WK warps must fit the staging area
-    // the balanced form (below) pays off for more than 8 activation rows on large matrices (measured: 8 to 25 % there, a loss
+    // the balanced form (below; the streaming form of stream.cu takes these shapes wherever it may, so this is the one of
+    // afb_gemm_launch_static) pays off for more than 8 activation rows on large matrices (measured: 8 to 25 % there, a loss
     // of up to 10 % for m <= 8, whose grid form needs no K-slices); it runs best with the widest CTA
     bool want_balanced = weight_mb >= 48.0 && a.m > 8;
     if (const char* e = getenv("AFB_DECODE_BALANCED")) want_balanced = atoi(e) != 0;   // tuning aid
