@@ -15,8 +15,8 @@ struct DeviceCtx {
     int      sm_count = 0;
     int32_t* status = nullptr;        // device int32[4]: {code, where, a, b}
     // Split-K workspaces (fp32 partial sums + arrival counters, used by decode K-slices, the balanced decode form and the
-    // prefill tail split): one per stream that has launched such a GEMM, so that launches on different streams never share
-    // one.  Slot 0 is allocated by afb_init, the others on a stream's first launch (outside any stream capture).
+    // prefill tail split and the streaming form): one per stream that has launched such a GEMM, so that launches on different streams
+    // never share one.  The first eight are allocated by afb_init, the others on a stream's first launch (outside any stream capture).
     static constexpr int kMaxWorkspaces = 64;
     struct Workspace {
         bool          assigned = false;

@@ -130,9 +130,10 @@ int afb_device_sync(void);
  * GEMMs that split K between CTAs (decode K-slices, short last wave of prefill tiles) meet in an
  * fp32 workspace that belongs to the STREAM they are launched on: launches on one stream are
  * serialised by the stream, launches on different streams use different workspaces (32 MiB each).
- * afb_init allocates four of them; a fifth and later stream allocates its own on its first such
- * launch, which then must not happen inside a stream capture; at most 16 streams per device, after
- * that AFB_ERR_TOO_LARGE.  A captured graph keeps using the workspace of the stream it was captured on. */
+ * afb_init allocates eight of them; a ninth and later stream allocates its own on its first such
+ * launch, which then must not happen inside a stream capture; at most 64 streams per device, after
+ * that AFB_ERR_TOO_LARGE.  Launches that have a form without a workspace take that one instead when
+ * only 16 slots are left, or, inside a capture, when only four allocated ones are.  A captured graph keeps using the workspace of the stream it was captured on. */
 int afb_gemm_launch(const afb_gemm_args* args, void* stream);
 /* Which variant AFB_VARIANT_AUTO resolves to for these args (no launch). */
 int afb_gemm_resolve_variant(const afb_gemm_args* args, uint32_t* variant);
