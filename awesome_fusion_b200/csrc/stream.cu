@@ -43,7 +43,11 @@ constexpr int kFirstEpi = 4, kFirstConv = 8;
 constexpr int kThreads = 32 * (kFirstConv + 4 * kGroups);
 constexpr int kMaxRaw = 12, kMaxSlots = 8, kMaxAcc = 8;
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kSet = 4;            // kSums: group sums handed to the epilogue at a time (5 x 28672 x 8192 int4: 51.5 us with 2, 50.4 with 4)
+constexpr uint32_t kSet = 4;            // kSums, kParts: sums handed to the epilogue at a time (5 x 28672 x 8192 int4: 51.5 us with 2, 50.4 with 4)
+// kParts: k that one accumulator adds up before the sum goes on in fp32 registers.  The tensor cores cut off what an addition shifts out,
+// so a sum over all of K drifts: of 16 x 28672 x 8192 int8 results 15 in 10000 were not the correctly rounded ones (8 rows: 14), with
+// decode.cu, whose warps and CTAs each add a stretch of K, 10 (5), with sums over 1024 k 3 (3).
+constexpr uint32_t kPartSum = 1024;
 constexpr int kBars = 2 * (kMaxRaw + kMaxSlots + kMaxAcc) + kMaxSlots + 3;
 constexpr int kOffMisc = kBars * 8, kOffOut = 1024;
 constexpr int kOutBytes = 16 * 32 * 2;                    // one block of the result: 16 rows x 32 channels
@@ -53,7 +57,10 @@ static_assert(kOffMisc + 32 <= kOffOut && kOffRaw % 1024 == 0, "shared memory la
 
 enum Mode { kChannel = 0,   // per-channel scale on the finished sum
             kFold = 1,      // group scale folded into the bf16 weight (more than 16 activation rows)
-            kSums = 2 };    // group scale on the fp32 sum of each group (up to 16 rows)
+            kSums = 2,      // group scale on the fp32 sum of each group (up to 16 rows)
+            kParts = 3 };   // as kChannel, for up to 16 rows: the tensor cores' sums over kPartSum of k are added in fp32
+__host__ __device__ constexpr bool channel_scaled(int mode) { return mode == kChannel || mode == kParts; }
+__host__ __device__ constexpr bool summed(int mode) { return mode == kSums || mode == kParts; }
 
 struct StreamParams {
     uint16_t* c;
@@ -62,8 +69,8 @@ struct StreamParams {
     uint32_t m, n, k, ldc;
     uint32_t enc, scale_dtype, packed;
     uint32_t group_shift;     // log2(group / k of a part)
-    uint32_t flush;           // kSums: parts per group sum
-    uint32_t acc_cols;        // TMEM columns handed to the epilogue at a time (kSums: kSet group sums)
+    uint32_t flush;           // kSums, kParts: parts per sum
+    uint32_t acc_cols;        // TMEM columns handed to the epilogue at a time (kSums, kParts: kSet sums)
     uint32_t rows, m_tiles, n_tiles, group_m;
     uint32_t blocks, parts;   // raw blocks and parts along K
     uint32_t shared_tiles, whole_waves;   // tiles [0, shared_tiles) are dealt in units, the rest are whole tiles
@@ -314,7 +321,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         bool ok = true, ready = false;
         while (ok && walk.next(p, x)) {
             const uint32_t ns = parts_of(x);
-            uint32_t in_sum = 0, sum = 0;   // parts in the current sum; sums in the current accumulator (kSums)
+            uint32_t in_sum = 0, sum = 0;   // parts in the current sum; sums in the current accumulator (kSums, kParts)
             for (uint32_t l = 0; l < ns; l += PAIR) {
                 if (in_sum == 0 && sum == 0 && !warp_wait(acc_empty(rc.i), rc.phase ^ 1u, abort_flag)) { give_up(33, x.t, l); ok = false; break; }
                 if (!__all_sync(0xffffffffu, ready) && !warp_wait(step_full(rs.i), rs.phase, abort_flag)) { give_up(34, x.t, l); ok = false; break; }
@@ -333,8 +340,8 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                             ptx::umma_bf16_ts(td + sum * 16, ta + h * kPartCols + 8 * j, db + (uint32_t)(h * (KS / kSlab) + j / 4) * slab_d + 2u * (j % 4), idesc, (in_sum | (uint32_t)j) ? 1u : 0u);
                     }
                     ++in_sum;
-                    if (MODE == kSums && in_sum == p.flush) { in_sum = 0; ++sum; }
-                    last = l + h + 1 == ns || (MODE == kSums && sum == kSet);
+                    if (summed(MODE) && in_sum == p.flush) { in_sum = 0; ++sum; }
+                    last = l + h + 1 == ns || (summed(MODE) && sum == kSet);
                 }
                 if (ptx::elect_one()) {
                     ptx::umma_commit(done);
@@ -351,7 +358,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         const uint32_t sel0 = p.packed ? kSel8Strided02 : kSel8Natural01, sel1 = p.packed ? kSel8Strided13 : kSel8Natural23;
         const Nibbles nib = nibbles(p.packed != 0);
         const bool has_zero = p.zero != nullptr;
-        const uint32_t groups_per_row = MODE == kChannel ? 0 : (p.parts >> p.group_shift);
+        const uint32_t groups_per_row = channel_scaled(MODE) ? 0 : (p.parts >> p.group_shift);
         auto zero_of = [&](uint32_t zb) { return !has_zero ? 0 : (BITS == 8 ? decode_zero8(zb, p.enc) : decode_zero4(zb, p.enc)); };
         GroupUnpack up;
         up.mul0 = BITS == 8 ? kMulByte : nib.mul[0]; up.mul1 = nib.mul[1]; up.add = unpack_add(BITS, 0); up.scale = 0;
@@ -364,12 +371,12 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
             const size_t g0 = (size_t)nn * groups_per_row;
             uint32_t sc = 0, zb = 0, sc_nxt = 0, zb_nxt = 0;
             auto load_group = [&](uint32_t l, uint32_t& s, uint32_t& z) {
-                if (MODE == kChannel || nn >= p.n || l >= ns) return;
+                if (channel_scaled(MODE) || nn >= p.n || l >= ns) return;
                 const size_t i = g0 + ((k0 + l) >> p.group_shift);
                 if (MODE == kFold) s = reinterpret_cast<const uint16_t*>(p.scale)[i];
                 if (has_zero) z = p.zero[i];
             };
-            if (MODE == kChannel && has_zero) up.add = unpack_add(BITS, zero_of(nn < p.n ? p.zero[nn] : 0u));
+            if (channel_scaled(MODE) && has_zero) up.add = unpack_add(BITS, zero_of(nn < p.n ? p.zero[nn] : 0u));
             uint32_t l = (g - steps_before * PAIR) & (kGroups - 1);
             Ring rr, rs;
             rr.set(blocks_before + l / SPB, p.raw_stages);
@@ -385,7 +392,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                     continue;
                 }
                 const uint32_t sub = l % SPB, left = ns - (l - sub);   // `left`: parts of this block and all after it
-                if (MODE != kChannel) { sc = sc_nxt; zb = zb_nxt; load_group(l + kGroups, sc_nxt, zb_nxt); }
+                if (!channel_scaled(MODE)) { sc = sc_nxt; zb = zb_nxt; load_group(l + kGroups, sc_nxt, zb_nxt); }
                 if (p.slot_first && !warp_wait(step_empty(rs.i), rs.phase ^ 1u, abort_flag)) { give_up(36, x.t, l); ok = false; break; }
                 if (!warp_wait(raw_full(rr.i), rr.phase, abort_flag)) { give_up(35, x.t, l); ok = false; break; }
                 const uint8_t* raw = smem_gen + kOffRaw + rr.i * kRawBytes + ch * 128;
@@ -445,7 +452,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         const uint32_t quarter = (uint32_t)warp & 3u, ch = quarter * 32 + lane;
         const uint32_t lane_base = tmem_base + ((quarter * 32u) << 16);
         const uint32_t first_tile = walk.u / p.blocks;
-        const uint32_t groups_per_row = MODE == kChannel ? 0 : (p.parts >> p.group_shift);
+        const uint32_t groups_per_row = channel_scaled(MODE) ? 0 : (p.parts >> p.group_shift);
         Ring rc{0, 0};
         uint32_t meeting = 0, to_finish = 0;
         uint32_t block = 0;   // staging block of the next tile store
@@ -492,13 +499,14 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                 for (int j = 0; j < 16; ++j)
                     if (c0 + j < valid) __stcg(part + (size_t)(c0 + j) * kCh, v[j]);
             };
-            if (MODE == kSums) {
+            if (summed(MODE)) {
                 float sum[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) sum[j] = 0.f;
                 const size_t g0 = (size_t)nn * groups_per_row;
                 auto group_scale = [&](uint32_t l) {
                     if (nn >= p.n || l >= ns) return 0.f;
+                    if (MODE == kParts) return 1.f;
                     const size_t i = g0 + ((x.kb0 * SPB + l) >> p.group_shift);
                     return p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[i] << 16)
                                                            : reinterpret_cast<const float*>(p.scale)[i];
@@ -720,7 +728,7 @@ int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, boo
     p.m = a.m; p.n = a.n; p.k = a.k; p.ldc = a.ldc;
     p.enc = a.b_encoding; p.scale_dtype = a.scale_dtype;
     p.packed = a.b_layout == AFB_LAYOUT_COL_PACKED ? 1u : 0u;
-    const int mode = !a.group_size ? kChannel : a.m > 16 ? kFold : kSums;
+    const int mode = a.m > 16 ? (a.group_size ? kFold : kChannel) : (a.group_size ? kSums : kParts);
     p.rows = tile_rows(a);
     p.m_tiles = (a.m + p.rows - 1) / p.rows;
     p.n_tiles = (a.n + kCh - 1) / kCh;
@@ -732,8 +740,8 @@ int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, boo
     p.parts = a.k / ks;
     p.blocks = (p.parts + spb - 1) / spb;
     while (a.group_size && ks << p.group_shift < a.group_size) ++p.group_shift;
-    p.flush = mode == kSums ? (1u << p.group_shift < spb ? 1u << p.group_shift : spb) : 0;
-    p.acc_cols = mode == kSums ? kSet * 16 : p.rows;
+    p.flush = mode == kParts ? kPartSum / ks : mode == kSums ? (1u << p.group_shift < spb ? 1u << p.group_shift : spb) : 0;
+    p.acc_cols = summed(mode) ? kSet * 16 : p.rows;
     p.accs = p.rows <= 192 ? 2 : 1;
     const uint32_t pair = ks == 128 && p.rows <= 64 ? 2 : 1;
     p.slots = (kTmemCols - p.accs * p.acc_cols) / (pair * ks / 2);
@@ -782,8 +790,12 @@ int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, boo
     p.finish_late = p.whole_waves == 0 || (p.whole_waves == 1 && p.rows > 32);
     const bool pdl = (a.flags & AFB_FLAG_PDL) != 0 && a.m <= 16;   // of the decode variant only
 #define AFB_STREAM_LAUNCH(B, M) (pair == 2 ? launch_cfg<B, M, 128, 2>(ta, tw, tc, p, grid, pdl, ctx, s) : ks == 128 ? launch_cfg<B, M, 128, 1>(ta, tw, tc, p, grid, pdl, ctx, s) : launch_cfg<B, M, 64, 1>(ta, tw, tc, p, grid, pdl, ctx, s))
-    if (a.b_bits == 8) return mode == kChannel ? AFB_STREAM_LAUNCH(8, kChannel) : mode == kFold ? AFB_STREAM_LAUNCH(8, kFold) : AFB_STREAM_LAUNCH(8, kSums);
-    return mode == kChannel ? AFB_STREAM_LAUNCH(4, kChannel) : mode == kFold ? AFB_STREAM_LAUNCH(4, kFold) : AFB_STREAM_LAUNCH(4, kSums);
+    switch (mode) {
+        case kChannel: return a.b_bits == 8 ? AFB_STREAM_LAUNCH(8, kChannel) : AFB_STREAM_LAUNCH(4, kChannel);
+        case kFold:    return a.b_bits == 8 ? AFB_STREAM_LAUNCH(8, kFold) : AFB_STREAM_LAUNCH(4, kFold);
+        case kSums:    return a.b_bits == 8 ? AFB_STREAM_LAUNCH(8, kSums) : AFB_STREAM_LAUNCH(4, kSums);
+        default:       return a.b_bits == 8 ? AFB_STREAM_LAUNCH(8, kParts) : AFB_STREAM_LAUNCH(4, kParts);
+    }
 #undef AFB_STREAM_LAUNCH
 }
 
