@@ -30,6 +30,7 @@
 #include "afb_internal.h"
 #include "dequant.cuh"
 #include "ptx_sm100.cuh"
+#include "stream_deal.h"
 
 namespace afb {
 
@@ -72,8 +73,8 @@ struct StreamParams {
     uint32_t flush;           // kSums, kParts: parts per sum
     uint32_t acc_cols;        // TMEM columns handed to the epilogue at a time (kSums, kParts: kSet sums)
     uint32_t rows, m_tiles, n_tiles, group_m;
-    uint32_t blocks, parts;   // raw blocks and parts along K
-    uint32_t shared_tiles, whole_waves;   // tiles [0, shared_tiles) are dealt in units, the rest are whole tiles
+    uint32_t parts;           // parts along K
+    StreamDeal deal;          // who does what, in units of one raw block
     uint32_t raw_stages, slots, accs;
     uint32_t slot_first;      // converters wait for their slot before they wait for their raw block
     uint32_t c_tma, c_vec;    // tile stores; 8-byte stores of finished shared tiles
@@ -109,29 +110,6 @@ struct Ring {
     __device__ __forceinline__ void set(uint32_t count, uint32_t len) { const uint32_t w = count / len; i = count - w * len; phase = w & 1u; }
 };
 
-// The pieces of work of one CTA, in order; every role walks the same list.
-struct Piece { uint32_t t, kb0, kb1; };
-struct Walk {
-    uint32_t u, u_end, it;
-    __device__ __forceinline__ void start(const StreamParams& p) {
-        const uint32_t total = p.shared_tiles * p.blocks;
-        u = (uint32_t)((uint64_t)blockIdx.x * total / gridDim.x);
-        u_end = (uint32_t)((uint64_t)(blockIdx.x + 1) * total / gridDim.x);
-        it = 0;
-    }
-    __device__ __forceinline__ bool next(const StreamParams& p, Piece& x) {
-        if (u < u_end) {
-            x.t = u / p.blocks; x.kb0 = u - x.t * p.blocks;
-            x.kb1 = min(p.blocks, x.kb0 + (u_end - u));
-            u += x.kb1 - x.kb0;
-            return true;
-        }
-        if (it >= p.whole_waves) return false;
-        x.t = p.shared_tiles + blockIdx.x + it * gridDim.x; x.kb0 = 0; x.kb1 = p.blocks;
-        ++it;
-        return true;
-    }
-};
 // Groups of group_m row tiles; inside a group the channel tiles advance, row tile fastest.
 __device__ __forceinline__ void tile_origin(const StreamParams& p, uint32_t t, uint32_t& m0, uint32_t& n0) {
     const uint32_t per_group = p.group_m * p.n_tiles;
@@ -208,19 +186,16 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         if (!*abort_flag) { report_timeout(p.status, where, (int)a, (int)b); *abort_flag = 1; }
     };
     Walk walk;
-    walk.start(p);
+    walk.start(p.deal, blockIdx.x);   // every role walks the same list of pieces
     Piece x;
     auto parts_of = [&](const Piece& q) { return min(q.kb1 * SPB, p.parts) - q.kb0 * SPB; };
 
     // Adds the partial sums of shared tile t in CTA order, scales, rounds and stores it; `tid` of `threads` threads, four channels of
     // one row at a time, up to eight 16-byte loads in flight per thread.
-    const uint32_t total_units = p.shared_tiles * p.blocks;
-    // the CTA holding unit u: the largest c with c * total / grid <= u
-    auto cta_of = [&](uint32_t u) { return (uint32_t)((((uint64_t)u + 1) * gridDim.x + total_units - 1) / total_units) - 1u; };
     auto finish_tile = [&](uint32_t t, uint32_t tid, uint32_t threads) {
         uint32_t m0, n0;
         tile_origin(p, t, m0, n0);
-        const uint32_t first = cta_of(t * p.blocks), last = cta_of(t * p.blocks + p.blocks - 1);
+        const uint32_t first = p.deal.first_cta(t), last = p.deal.last_cta(t);
         const uint32_t valid = min(p.rows, p.m - m0), vecs = valid * (kCh / 4);
         const uint32_t nn = n0 + (tid & 31u) * 4;   // threads is a multiple of 32: the same four channels in every turn
         float sc[4];
@@ -229,8 +204,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
             sc[e] = MODE == kSums ? kUnpackInverse : MODE == kFold ? kGroupInverse : nn + e >= p.n ? 0.f :
                 kUnpackInverse * (p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn + e] << 16)
                                                                   : reinterpret_cast<const float*>(p.scale)[nn + e]);
-        // Only the first contributor can hold the tile as anything but its first shared tile (slot 1).
-        const uint32_t first_slot = 2 * first + ((uint32_t)((uint64_t)first * total_units / gridDim.x) / p.blocks != t ? 1u : 0u);
+        const uint32_t first_slot = p.deal.slot(first, t);   // the others' runs begin in this tile: slot 2c
         const size_t stride = (size_t)p.rows * kCh;
         for (uint32_t v = tid; v < vecs; v += 2 * threads) {
             float4 sum[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
@@ -272,7 +246,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         Ring r{0, 0};
         uint32_t issued = 0, parity = 0;
         bool ok = true;
-        while (ok && walk.next(p, x)) {
+        while (ok && walk.next(p.deal, blockIdx.x, x)) {
             uint32_t m0, n0;
             tile_origin(p, x.t, m0, n0);
             for (uint32_t kb = x.kb0; kb < x.kb1; ++kb) {
@@ -293,7 +267,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         Ring r{0, 0};
         uint32_t issued = 0, parity = 0;
         bool ok = true;
-        while (ok && walk.next(p, x)) {
+        while (ok && walk.next(p.deal, blockIdx.x, x)) {
             uint32_t m0, n0;
             tile_origin(p, x.t, m0, n0);
             const uint32_t k0 = x.kb0 * SPB, ns = parts_of(x);
@@ -319,7 +293,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         const uint32_t slab_d = slab_bytes >> 4, act_d = act_bytes >> 4;   // in units of the descriptor's address field
         Ring rs{0, 0}, rc{0, 0};
         bool ok = true, ready = false;
-        while (ok && walk.next(p, x)) {
+        while (ok && walk.next(p.deal, blockIdx.x, x)) {
             const uint32_t ns = parts_of(x);
             uint32_t in_sum = 0, sum = 0;   // parts in the current sum; sums in the current accumulator (kSums, kParts)
             for (uint32_t l = 0; l < ns; l += PAIR) {
@@ -364,7 +338,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         up.mul0 = BITS == 8 ? kMulByte : nib.mul[0]; up.mul1 = nib.mul[1]; up.add = unpack_add(BITS, 0); up.scale = 0;
         uint32_t steps_before = 0, blocks_before = 0;   // of the pieces walked so far (a step is PAIR parts, the last of a piece may lack one)
         bool ok = true;
-        while (ok && walk.next(p, x)) {
+        while (ok && walk.next(p.deal, blockIdx.x, x)) {
             uint32_t m0, n0;
             tile_origin(p, x.t, m0, n0);
             const uint32_t nn = n0 + ch, ns = parts_of(x), k0 = x.kb0 * SPB;
@@ -451,19 +425,18 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         // ======================= epilogue =======================
         const uint32_t quarter = (uint32_t)warp & 3u, ch = quarter * 32 + lane;
         const uint32_t lane_base = tmem_base + ((quarter * 32u) << 16);
-        const uint32_t first_tile = walk.u / p.blocks;
         const uint32_t groups_per_row = channel_scaled(MODE) ? 0 : (p.parts >> p.group_shift);
         Ring rc{0, 0};
         uint32_t meeting = 0, to_finish = 0;
         uint32_t block = 0;   // staging block of the next tile store
         bool ok = true;
         asm volatile("griddepcontrol.wait;" ::: "memory");   // workspace, counters and C belong to the predecessor until it has ended
-        while (ok && walk.next(p, x)) {
+        while (ok && walk.next(p.deal, blockIdx.x, x)) {
             uint32_t m0, n0;
             tile_origin(p, x.t, m0, n0);
             const uint32_t nn = n0 + ch, ns = parts_of(x);
             const uint32_t valid = min(p.rows, p.m - m0);
-            const bool whole = x.kb0 == 0 && x.kb1 == p.blocks;
+            const bool whole = x.kb0 == 0 && x.kb1 == p.deal.blocks;
             const float scale = MODE == kSums ? kUnpackInverse : MODE == kFold ? kGroupInverse :
                 nn >= p.n ? 0.f : kUnpackInverse * (p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn] << 16)
                                                                                     : reinterpret_cast<const float*>(p.scale)[nn]);
@@ -492,7 +465,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                         if (c0 + j < valid) dst[(size_t)j * p.ldc] = __bfloat16_as_ushort(__float2bfloat16_rn(v[j] * scale));
                 }
             };
-            float* part = p.ws + (size_t)(2 * blockIdx.x + (x.t != first_tile ? 1 : 0)) * p.rows * kCh + ch;
+            float* part = p.ws + (size_t)(whole ? 0 : p.deal.slot(blockIdx.x, x.t)) * p.rows * kCh + ch;
             auto emit = [&](uint32_t c0, const float (&v)[16]) {
                 if (whole) { store(c0, v); return; }
 #pragma unroll
@@ -569,7 +542,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
             }
             if (!whole) {
                 // the CTAs holding units of this tile meet at its counter
-                const uint32_t first = cta_of(x.t * p.blocks), last = cta_of(x.t * p.blocks + p.blocks - 1);
+                const uint32_t first = p.deal.first_cta(x.t), last = p.deal.last_cta(x.t);
                 __threadfence();
                 __syncwarp();
                 if (lane == 0) {
@@ -738,7 +711,6 @@ int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, boo
     const uint32_t ks = p.rows <= 128 && a.k % 128 == 0 && a.group_size % 128 == 0 ? 128 : 64;
     const uint32_t spb = (a.b_bits == 8 ? 128 : 256) / ks;
     p.parts = a.k / ks;
-    p.blocks = (p.parts + spb - 1) / spb;
     while (a.group_size && ks << p.group_shift < a.group_size) ++p.group_shift;
     p.flush = mode == kParts ? kPartSum / ks : mode == kSums ? (1u << p.group_shift < spb ? 1u << p.group_shift : spb) : 0;
     p.acc_cols = summed(mode) ? kSet * 16 : p.rows;
@@ -758,16 +730,10 @@ int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, boo
     p.slot_first = p.raw_stages >= kGroups + p.slots * pair ? 0u : 1u;
     if (p.raw_stages < p.slots * pair || p.slots * pair < (uint32_t)kGroups) return AFB_OK;
 
-    const uint32_t tiles = p.m_tiles * p.n_tiles;
-    uint32_t grid = sms;
-    const uint32_t waves = tiles / sms, rest = tiles - waves * sms;
-    if (rest == 0) { p.shared_tiles = 0; p.whole_waves = waves; }
-    else if (waves == 0) { p.shared_tiles = tiles; p.whole_waves = 0; }
-    else if (rest * 4 >= sms) { p.shared_tiles = rest; p.whole_waves = waves; }
-    else { p.shared_tiles = sms + rest; p.whole_waves = waves - 1; }
-    if (p.shared_tiles && p.whole_waves == 0 && (uint64_t)p.shared_tiles * p.blocks < grid) grid = p.shared_tiles * p.blocks;
-    if (p.shared_tiles) {
-        if (p.shared_tiles > ctx->splitk_counter_count || (size_t)2 * grid * p.rows * kCh * sizeof(float) > ctx->splitk_ws_bytes) return AFB_OK;
+    p.deal = deal_tiles(p.m_tiles * p.n_tiles, (p.parts + spb - 1) / spb, sms);
+    const uint32_t grid = p.deal.grid;
+    if (p.deal.shared_tiles) {
+        if (p.deal.shared_tiles > ctx->splitk_counter_count || (size_t)2 * grid * p.rows * kCh * sizeof(float) > ctx->splitk_ws_bytes) return AFB_OK;
         int rc = AFB_OK;
         const DeviceCtx::Workspace* w = workspace_for(ctx, s, &rc, true);
         if (!w) return rc;   // the caller's other forms
@@ -787,7 +753,7 @@ int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, boo
     p.c_tma = a.ldc % 8 == 0 && (uintptr_t)a.ptr_c % 16 == 0 && a.n % 8 == 0 &&
               tmap_2d(&tc, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.ptr_c, a.n, a.m, (uint64_t)a.ldc * 2, 32, 16, CU_TENSOR_MAP_SWIZZLE_NONE) == AFB_OK;
     p.c_vec = a.ldc % 4 == 0 && (uintptr_t)a.ptr_c % 8 == 0;
-    p.finish_late = p.whole_waves == 0 || (p.whole_waves == 1 && p.rows > 32);
+    p.finish_late = p.deal.whole_waves == 0 || (p.deal.whole_waves == 1 && p.rows > 32);
     const bool pdl = (a.flags & AFB_FLAG_PDL) != 0 && a.m <= 16;   // of the decode variant only
 #define AFB_STREAM_LAUNCH(B, M) (pair == 2 ? launch_cfg<B, M, 128, 2>(ta, tw, tc, p, grid, pdl, ctx, s) : ks == 128 ? launch_cfg<B, M, 128, 1>(ta, tw, tc, p, grid, pdl, ctx, s) : launch_cfg<B, M, 64, 1>(ta, tw, tc, p, grid, pdl, ctx, s))
     switch (mode) {

@@ -1,0 +1,48 @@
+// Walks the dealing of csrc/stream_deal.h as the kernel's CTAs do (test infrastructure, built by tests/test_stream_deal.py).
+#include <vector>
+#include "stream_deal.h"
+
+// 0, or which rule is broken: 1 a unit not dealt exactly once, 2 a contributor missing between the first and the last CTA of a tile (it
+// would be waited for), 3 two partial sums in one place, 4 more than two shared tiles to finish in one CTA, 5 a CTA with nothing to do,
+// 6 a run that is longer than another by more than one unit
+extern "C" int check_deal(uint32_t tiles, uint32_t blocks, uint32_t sms) {
+    const afb::StreamDeal d = afb::deal_tiles(tiles, blocks, sms);
+    std::vector<uint8_t> seen((size_t)tiles * blocks, 0);
+    std::vector<uint32_t> arrivals(d.shared_tiles, 0);
+    std::vector<uint8_t> slots((size_t)2 * d.grid, 0);
+    uint32_t shortest = ~0u, longest = 0;
+    for (uint32_t c = 0; c < d.grid; ++c) {
+        afb::Walk w;
+        w.start(d, c);
+        if (c < d.dealers && d.shared_tiles) {
+            const uint32_t run = w.u_end - w.u;
+            shortest = run < shortest ? run : shortest;
+            longest = run > longest ? run : longest;
+        }
+        afb::Piece x;
+        uint32_t pieces = 0, parts = 0;
+        while (w.next(d, c, x)) {
+            ++pieces;
+            if (x.t >= tiles || x.kb0 >= x.kb1 || x.kb1 > blocks) return 1;
+            for (uint32_t kb = x.kb0; kb < x.kb1; ++kb)
+                if (seen[(size_t)x.t * blocks + kb]++) return 1;
+            if (x.kb0 == 0 && x.kb1 == blocks) continue;
+            if (x.t >= d.shared_tiles || c < d.first_cta(x.t) || c > d.last_cta(x.t)) return 2;
+            ++arrivals[x.t];
+            if (++parts > 2) return 4;
+            if (slots[d.slot(c, x.t)]++) return 3;
+        }
+        if (!pieces) return 5;
+    }
+    for (uint8_t s : seen) if (!s) return 1;
+    for (uint32_t t = 0; t < d.shared_tiles; ++t)
+        if (arrivals[t] && arrivals[t] != d.last_cta(t) - d.first_cta(t) + 1) return 2;
+    if (d.shared_tiles && longest - shortest > 1) return 6;
+    return 0;
+}
+extern "C" uint32_t check_range(uint32_t tiles_end, uint32_t blocks_end, uint32_t sms, uint32_t* where) {
+    for (uint32_t t = 1; t < tiles_end; ++t)
+        for (uint32_t b = 1; b < blocks_end; ++b)
+            if (const int rc = check_deal(t, b, sms)) { where[0] = t; where[1] = b; return (uint32_t)rc; }
+    return 0;
+}

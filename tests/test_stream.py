@@ -85,3 +85,19 @@ def test_sums_of_few_rows_do_not_drift(afb, m):
     got, _ = T.run_case(afb, case)
     off = (T.np_bf16_to_f32(got) - exact).mean() / half_sum
     assert abs(off) < 1e-6, off
+
+
+@pytest.mark.parametrize("m,n,k", [(32, 24576, 512), (24, 25600, 512), (20, 24576, 768), (2048, 19456, 768)])
+def test_few_units_next_to_whole_waves(afb, oracle, monkeypatch, m, n, k):
+    """Fewer units of shared tiles than CTAs, next to whole waves: every tile is finished, and the arrival counters are back at zero for
+    the next launch on the stream (the same, and a decode launch with K-slices).  By the automatic choice and forced."""
+    case = T.make_case(m, n, k, bits=4, group=128, seed=m, scale_range=(0.005, 0.05))
+    rows = list(range(0, m, 97)) if m > 64 else list(range(m))   # one or two of every row tile
+    ref = oracle.gemm(case, threads=8, round_w=True, rows=rows)
+    for form in (None, "1", "1"):
+        monkeypatch.setenv("AFB_STREAM", form) if form else monkeypatch.delenv("AFB_STREAM")
+        got, _ = T.run_case(afb, case)
+        check_close(oracle, ref, np.ascontiguousarray(got[rows]), f"{m}x{n}x{k} AFB_STREAM={form}")
+    monkeypatch.delenv("AFB_STREAM")
+    sliced = T.make_case(16, 1024, 8192, seed=1)
+    check_close(oracle, oracle.gemm(sliced, threads=8), T.run_case(afb, sliced)[0], "decode K-slices after it")

@@ -1,0 +1,35 @@
+"""The dealing of the streaming form's work (csrc/stream_deal.h), walked on the CPU as the kernel's CTAs walk it: every unit is dealt
+once, a tile's contributors are as many as the count it waits for, and no two partial sums share a place."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("deal") / "libdeal.so")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I" + os.path.join(ROOT, "awesome_fusion_b200", "csrc"),
+                           "-o", out, os.path.join(ROOT, "tests", "stream_deal_shim.cc")])
+    lib = ctypes.CDLL(out)
+    lib.check_deal.argtypes = [ctypes.c_uint32] * 3
+    lib.check_range.argtypes = [ctypes.c_uint32] * 3 + [ctypes.POINTER(ctypes.c_uint32)]
+    return lib
+
+
+@pytest.mark.parametrize("sms,tiles,blocks", [(148, 620, 14), (132, 420, 9), (7, 60, 12), (1, 5, 5)])
+def test_every_number_of_tiles_and_blocks(shim, sms, tiles, blocks):
+    """148 SMs: up to four waves of tiles with up to 13 units each (beyond one wave's rest the pattern repeats)."""
+    where = (ctypes.c_uint32 * 2)()
+    rc = shim.check_range(tiles, blocks, sms, where)
+    assert rc == 0, f"rule {rc} broken at {where[0]} tiles of {where[1]} blocks on {sms} SMs"
+
+
+@pytest.mark.parametrize("tiles,blocks", [(192, 2), (200, 2), (192, 3), (3300, 3), (1672, 3), (224, 64), (86, 32), (32, 512), (4928, 32)])
+def test_sizes_of_calls(shim, tiles, blocks):
+    """24576 x 512 and 25600 x 512 int4 at 17 to 32 rows, 24576 x 768, 2048 rows of 38400 x 768 and of 19456 x 768 (fewer units than
+    CTAs next to whole waves: such tiles were lost), and sizes with more units than CTAs."""
+    assert shim.check_deal(tiles, blocks, 148) == 0
