@@ -41,6 +41,44 @@ unsigned long long* phase_ts_if_enabled(DeviceCtx* ctx) {
     return on ? ctx->phase_ts : nullptr;
 }
 
+namespace {
+// While it lives, the thread's calls are none of another thread's captures' business: cudaMalloc would break a capture in global mode.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Memory for partial sums and arrival counters at zero, ready for the next launch on `s`.  The counters are cleared on `s` itself:
+// nothing orders the legacy stream before a launch on a non-blocking stream.  Inside a capture (which only one in relaxed mode survives:
+// in the other modes cudaMalloc refuses) that clearing would become part of the graph; there it is waited for instead.
+cudaError_t allocate_workspace(float** ws, size_t bytes, uint32_t** counters, size_t count, cudaStream_t s) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &capture);
+    if (e != cudaSuccess) return e;
+    const size_t counter_bytes = count * sizeof(uint32_t);
+    auto allocate = [&] {
+        cudaError_t r = cudaMalloc(ws, bytes);
+        return r == cudaSuccess ? cudaMalloc(counters, counter_bytes) : r;
+    };
+    if (capture == cudaStreamCaptureStatusNone) {
+        RelaxedCapture relaxed;
+        e = allocate();
+        if (e == cudaSuccess) e = cudaMemsetAsync(*counters, 0, counter_bytes, s);
+    } else {
+        e = allocate();
+        if (e == cudaSuccess) e = cudaMemset(*counters, 0, counter_bytes);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    }
+    if (e != cudaSuccess) {
+        if (*ws) cudaFree(*ws);
+        if (*counters) cudaFree(*counters);
+        *ws = nullptr; *counters = nullptr;
+    }
+    return e;
+}
+}  // namespace
+
 const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* rc, bool optional) {
     std::lock_guard<std::mutex> lock(g_mutex);
     DeviceCtx::Workspace* with_memory = nullptr;
@@ -69,16 +107,8 @@ const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* r
     }
     if (!free_slot) { *rc = AFB_ERR_TOO_LARGE; return nullptr; }   // more streams than workspaces
     if (!free_slot->ws) {
-        cudaError_t e = cudaMalloc(&free_slot->ws, ctx->splitk_ws_bytes);
-        if (e == cudaSuccess) e = cudaMalloc(&free_slot->counters, ctx->splitk_counter_count * sizeof(uint32_t));
-        if (e == cudaSuccess) e = cudaMemset(free_slot->counters, 0, ctx->splitk_counter_count * sizeof(uint32_t));
-        if (e != cudaSuccess) {
-            if (free_slot->ws) cudaFree(free_slot->ws);
-            if (free_slot->counters) cudaFree(free_slot->counters);
-            free_slot->ws = nullptr; free_slot->counters = nullptr;
-            *rc = cuda_fail(e);
-            return nullptr;
-        }
+        const cudaError_t e = allocate_workspace(&free_slot->ws, ctx->splitk_ws_bytes, &free_slot->counters, ctx->splitk_counter_count, s);
+        if (e != cudaSuccess) { *rc = cuda_fail(e); return nullptr; }
     }
     free_slot->assigned = true;
     free_slot->stream = s;
