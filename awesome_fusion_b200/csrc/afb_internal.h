@@ -15,7 +15,7 @@ struct DeviceCtx {
     int      sm_count = 0;
     int32_t* status = nullptr;        // device int32[4]: {code, where, a, b}
     // Split-K workspaces (fp32 partial sums + arrival counters, used by decode K-slices, the balanced decode form and the
-    // prefill tail split and the streaming form): one per stream that has launched such a GEMM, so that launches on different streams
+    // prefill tail split): one per stream that has launched such a GEMM, so that launches on different streams
     // never share one.  The first eight are allocated by afb_init, the others on a stream's first launch (outside any stream capture).
     static constexpr int kMaxWorkspaces = 64;
     struct Workspace {
@@ -27,6 +27,24 @@ struct DeviceCtx {
     Workspace workspaces[kMaxWorkspaces];
     size_t    splitk_ws_bytes = 0;        // size of every workspace
     size_t    splitk_counter_count = 0;   // counters of every workspace
+    // The streaming form's workspaces.  Nearly all its launches need one, also of sizes whose other form needs none; so they are apart
+    // from those above, and a captured graph has one of its own: graphs captured on the same stream, and that stream itself, may run at
+    // the same time.  A graph's workspace goes back to the pool when the graph and its executables are gone (`hold`).
+    struct GraphHold;
+    static constexpr int kMaxStreamWorkspaces = 256;
+    struct StreamWorkspace {
+        float*             ws = nullptr;
+        uint32_t*          counters = nullptr;
+        size_t             bytes = 0;
+        bool               assigned = false;
+        cudaStream_t       stream = nullptr;
+        unsigned long long capture = 0;      // id of the capture it was taken in, 0: launches on the stream itself
+        GraphHold*         hold = nullptr;
+    };
+    StreamWorkspace stream_workspaces[kMaxStreamWorkspaces];
+    size_t       stream_workspace_total = 0;    // bytes of them all
+    size_t       stream_counter_count = 0;      // counters of every one
+    cudaStream_t clear_stream = nullptr;        // clears the counters of a workspace that is taken inside a capture
     // optional phase timestamps (globaltimer ns of THIS GPU) written by the row-parallel GEMM and the exchange kernel when the
     // environment variable AFB_PHASE_TIMESTAMPS is set: [0] GEMM start, [1] GEMM end (latest CTA), [2] exchange start,
     // [3] all ranks' GEMMs seen complete, [4] sum + broadcast done (latest CTA), [5] all ranks' blocks seen in place
@@ -54,10 +72,12 @@ unsigned long long* phase_ts_if_enabled(DeviceCtx* ctx);   // ctx->phase_ts when
 
 DeviceCtx* current_ctx();           // nullptr when afb_init was not called on the current device
 // The split-K workspace of `s` on this device (allocates it on the stream's first use); nullptr + *rc on failure.
-// `optional`: the caller has a form that does without; nullptr with *rc = AFB_OK then means that it is to take that one.
-const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* rc, bool optional = false);
+const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* rc);
+// A workspace of at least `bytes` for a streaming launch on `s`; false: there is none to be had, the caller takes another form.
+bool stream_workspace(DeviceCtx* ctx, cudaStream_t s, size_t bytes, float** ws, uint32_t** counters);
 int  cuda_fail(cudaError_t e);      // records e, returns AFB_ERR_CUDA
 void count_launch(unsigned n = 1);
+void count_stream_launch();          // of the streaming form (counted by count_launch as well)
 
 // Driver entry point for tensor-map encoding, fetched once through the runtime.
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

@@ -3,6 +3,7 @@
 // driver (bfAintBGemm.cc:60-66,99-101,148-186; simple_device_mem.hpp:20,25).
 #include <atomic>
 #include <mutex>
+#include <new>
 #include <cstring>
 #include <cstdlib>
 #include "afb_internal.h"
@@ -14,12 +15,13 @@ constexpr int kMaxDevices = 32;
 DeviceCtx g_ctx[kMaxDevices];
 std::mutex g_mutex;
 std::atomic<int> g_last_cuda_error{0};
-std::atomic<unsigned long long> g_launches{0};
+std::atomic<unsigned long long> g_launches{0}, g_stream_launches{0};
 constexpr size_t kSplitKWorkspaceBytes = 32u << 20;
 constexpr size_t kSplitKCounters = 4096;
 constexpr int kPreallocatedWorkspaces = 8;
-constexpr int kReservedWorkspaces = 16;              // slots that only launches which cannot do without one may take ...
-constexpr int kReservedPreallocated = 4;             // ... and among them preallocated ones, for first launches inside a capture
+constexpr size_t kMinStreamWorkspace = 4u << 20;       // of a captured graph: a power of two from here on
+constexpr size_t kMaxStreamWorkspaceTotal = 2048u << 20;   // beyond this, and beyond kMaxStreamWorkspaces, launches take another form
+constexpr uint32_t kMaxStreamRows = 192;              // tile height of the streaming form
 constexpr uint32_t kPrefillTsMinM = 128;   // measured: above 128 activation rows the tensor-memory form is 1.3x faster, at 128 it is slower
 }  // namespace
 
@@ -29,6 +31,7 @@ int cuda_fail(cudaError_t e) {
     return AFB_ERR_CUDA;
 }
 void count_launch(unsigned n) { g_launches.fetch_add(n); }
+void count_stream_launch() { g_stream_launches.fetch_add(1); }
 
 DeviceCtx* current_ctx() {
     int dev = -1;
@@ -77,33 +80,97 @@ cudaError_t allocate_workspace(float** ws, size_t bytes, uint32_t** counters, si
     }
     return e;
 }
+
+// Memory of a streaming workspace: the partial sums, behind them the counters.
+cudaError_t allocate_stream_workspace(DeviceCtx* ctx, DeviceCtx::StreamWorkspace* w, size_t bytes) {
+    const cudaError_t e = cudaMalloc(&w->ws, bytes + ctx->stream_counter_count * sizeof(uint32_t));
+    if (e != cudaSuccess) { w->ws = nullptr; return e; }
+    w->counters = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(w->ws) + bytes);
+    w->bytes = bytes;
+    ctx->stream_workspace_total += bytes;
+    return e;
+}
 }  // namespace
 
-const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* rc, bool optional) {
+// Shared by a workspace and the graph that it was taken for; the last of the two deletes it.
+struct DeviceCtx::GraphHold {
+    std::atomic<bool> gone{false};   // the graph and all executables made of it have been destroyed
+    std::atomic<int>  owners{2};
+    void release() { if (owners.fetch_sub(1, std::memory_order_acq_rel) == 1) delete this; }
+};
+static void CUDART_CB graph_gone(void* hold) {   // may run on any thread, with any lock of the caller's held: no CUDA call, no mutex
+    auto* h = static_cast<DeviceCtx::GraphHold*>(hold);
+    h->gone.store(true, std::memory_order_release);
+    h->release();
+}
+
+bool stream_workspace(DeviceCtx* ctx, cudaStream_t s, size_t bytes, float** ws, uint32_t** counters) {
+    if (s == cudaStreamPerThread) return false;   // one handle for a stream per thread: it names no stream to keep a workspace for
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(s, &status, &id, &graph) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+    if (status == cudaStreamCaptureStatusInvalidated) return false;
+    const bool capturing = status == cudaStreamCaptureStatusActive;
+    if (!capturing) id = 0;
     std::lock_guard<std::mutex> lock(g_mutex);
-    DeviceCtx::Workspace* with_memory = nullptr;
-    DeviceCtx::Workspace* without = nullptr;
-    int free_slots = 0, free_with_memory = 0;
+    // a stream's own workspace serves all its launches to come, a graph's the one at hand and those no larger
+    size_t want = (size_t)2 * ctx->sm_count * kMaxStreamRows * 128 * sizeof(float);
+    if (capturing) for (want = kMinStreamWorkspace; want < bytes;) want *= 2;
+    DeviceCtx::StreamWorkspace* spare = nullptr;   // smallest one with memory that is large enough
+    DeviceCtx::StreamWorkspace* empty = nullptr;
+    for (auto& w : ctx->stream_workspaces) {
+        if (w.assigned && w.hold && w.hold->gone.load(std::memory_order_acquire)) {
+            w.hold->release();
+            w.hold = nullptr; w.assigned = false;
+        }
+        if (w.assigned) {
+            if (w.stream == s && w.capture == id && w.bytes >= bytes) { *ws = w.ws; *counters = w.counters; return true; }
+        } else if (w.ws) {
+            if (w.bytes >= (capturing ? bytes : want) && (!spare || w.bytes < spare->bytes)) spare = &w;
+        } else if (!empty) {
+            empty = &w;
+        }
+    }
+    DeviceCtx::StreamWorkspace* w = spare ? spare : empty;
+    if (!w) return false;
+    RelaxedCapture relaxed;
+    cudaError_t e = cudaSuccess;
+    if (!w->ws) {
+        if (ctx->stream_workspace_total + want > kMaxStreamWorkspaceTotal) return false;
+        e = allocate_stream_workspace(ctx, w, want);
+    }
+    // The counters of a graph are cleared here and now, not by a node of the graph; those of a stream in the stream's order.
+    cudaStream_t clear = capturing ? ctx->clear_stream : s;
+    if (e == cudaSuccess) e = cudaMemsetAsync(w->counters, 0, ctx->stream_counter_count * sizeof(uint32_t), clear);
+    if (e == cudaSuccess && capturing) e = cudaStreamSynchronize(clear);
+    if (e != cudaSuccess) { (void)cuda_fail(e); return false; }
+    if (capturing) {
+        auto* hold = new (std::nothrow) DeviceCtx::GraphHold;
+        if (!hold) return false;
+        cudaUserObject_t object = nullptr;
+        e = cudaUserObjectCreate(&object, hold, graph_gone, 1, cudaUserObjectNoDestructorSync);
+        if (e != cudaSuccess) { delete hold; (void)cuda_fail(e); return false; }
+        w->hold = hold;
+        e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+        if (e != cudaSuccess) {   // the object goes, and with it the graph's half of `hold`; the slot's at the next look at it
+            (void)cudaUserObjectRelease(object, 1);
+            w->assigned = true; w->stream = s; w->capture = id;
+            (void)cuda_fail(e);
+            return false;
+        }
+    }
+    w->assigned = true; w->stream = s; w->capture = id;
+    *ws = w->ws; *counters = w->counters;
+    return true;
+}
+
+const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* rc) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    DeviceCtx::Workspace* free_slot = nullptr;
     for (auto& w : ctx->workspaces) {
         if (w.assigned && w.stream == s) return &w;
-        if (w.assigned) continue;
-        ++free_slots;
-        if (w.ws) { ++free_with_memory; if (!with_memory) with_memory = &w; }
-        else if (!without) without = &w;
-    }
-    DeviceCtx::Workspace* free_slot = with_memory ? with_memory : without;   // one that already has memory first
-    if (optional) {
-        // a launch that has another form to fall back on: it leaves the others what they had before it existed, and does not
-        // allocate inside a capture
-        *rc = AFB_OK;
-        if (free_slots <= kReservedWorkspaces) return nullptr;
-        if (free_with_memory <= kReservedPreallocated) {
-            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
-            if (capture != cudaStreamCaptureStatusNone) return nullptr;
-            free_slot = without;
-            if (!free_slot) return nullptr;
-        }
+        if (!w.assigned && (!free_slot || (w.ws && !free_slot->ws))) free_slot = &w;   // an unassigned slot that already has memory first
     }
     if (!free_slot) { *rc = AFB_ERR_TOO_LARGE; return nullptr; }   // more streams than workspaces
     if (!free_slot->ws) {
@@ -203,6 +270,9 @@ int afb_init(int device) {
         AFB_CUDA(cudaMalloc(&c.workspaces[i].counters, kSplitKCounters * sizeof(uint32_t)));
         AFB_CUDA(cudaMemset(c.workspaces[i].counters, 0, kSplitKCounters * sizeof(uint32_t)));
     }
+    c.stream_counter_count = 2 * (size_t)c.sm_count;   // a launch shares fewer than two tiles per SM
+    AFB_CUDA(allocate_stream_workspace(&c, &c.stream_workspaces[0], (size_t)2 * c.sm_count * kMaxStreamRows * 128 * sizeof(float)));   // the first stream's
+    AFB_CUDA(cudaStreamCreateWithFlags(&c.clear_stream, cudaStreamNonBlocking));
     AFB_CUDA(cudaMalloc(&c.phase_ts, 8 * sizeof(unsigned long long)));
     AFB_CUDA(cudaMemset(c.phase_ts, 0, 8 * sizeof(unsigned long long)));
     AFB_CUDA(cudaMalloc(&c.ar_words, 4 * sizeof(uint32_t)));
@@ -221,6 +291,8 @@ int afb_finalize(void) {
     cudaDeviceSynchronize();
     cudaFree(c.status); cudaFree(c.ar_words); cudaFree(c.phase_ts);
     for (auto& w : c.workspaces) { if (w.ws) cudaFree(w.ws); if (w.counters) cudaFree(w.counters); }
+    for (auto& w : c.stream_workspaces) { if (w.ws) cudaFree(w.ws); if (w.hold) w.hold->release(); }
+    if (c.clear_stream) cudaStreamDestroy(c.clear_stream);
     for (int j = 0; j < 2; ++j) {
         for (int i = 0; i < 4; ++i) if (c.stage[j][i]) cudaFree(c.stage[j][i]);
         if (c.stage_free[j]) cudaEventDestroy(c.stage_free[j]);
@@ -494,6 +566,8 @@ int afb_read_status(int32_t out[4]) {
         std::lock_guard<std::mutex> lock(g_mutex);
         for (auto& w : ctx->workspaces)
             if (w.counters) AFB_CUDA(cudaMemset(w.counters, 0, ctx->splitk_counter_count * sizeof(uint32_t)));
+        for (auto& w : ctx->stream_workspaces)
+            if (w.ws) AFB_CUDA(cudaMemset(w.counters, 0, ctx->stream_counter_count * sizeof(uint32_t)));
         AFB_CUDA(cudaMemset(ctx->ar_words, 0, 4 * sizeof(uint32_t)));
     }
     return AFB_OK;
@@ -549,6 +623,7 @@ const char* afb_status_string(int status) {
 int afb_last_cuda_error(void) { return g_last_cuda_error.load(); }
 const char* afb_last_cuda_error_string(void) { return cudaGetErrorString((cudaError_t)g_last_cuda_error.load()); }
 unsigned long long afb_launch_count(void) { return g_launches.load(); }
+unsigned long long afb_stream_launch_count(void) { return g_stream_launches.load(); }
 const char* afb_version(void) { return "afb 0.1 (sm_100a)"; }
 
 }  // extern "C"

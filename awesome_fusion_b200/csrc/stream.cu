@@ -620,6 +620,7 @@ int launch_cfg(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& 
     cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tw, tc, p);
     count_launch();
+    count_stream_launch();
     return e == cudaSuccess ? AFB_OK : cuda_fail(e);
 }
 
@@ -733,12 +734,8 @@ int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, boo
     p.deal = deal_tiles(p.m_tiles * p.n_tiles, (p.parts + spb - 1) / spb, sms);
     const uint32_t grid = p.deal.grid;
     if (p.deal.shared_tiles) {
-        if (p.deal.shared_tiles > ctx->splitk_counter_count || (size_t)2 * grid * p.rows * kCh * sizeof(float) > ctx->splitk_ws_bytes) return AFB_OK;
-        int rc = AFB_OK;
-        const DeviceCtx::Workspace* w = workspace_for(ctx, s, &rc, true);
-        if (!w) return rc;   // the caller's other forms
-
-        p.ws = w->ws; p.counters = w->counters;
+        if (p.deal.shared_tiles > ctx->stream_counter_count) return AFB_OK;
+        if (!stream_workspace(ctx, s, (size_t)2 * grid * p.rows * kCh * sizeof(float), &p.ws, &p.counters)) return AFB_OK;   // the caller's other forms
     }
     p.status = ctx->status;
 

@@ -132,8 +132,15 @@ int afb_device_sync(void);
  * serialised by the stream, launches on different streams use different workspaces (32 MiB each).
  * afb_init allocates eight of them; a ninth and later stream allocates its own on its first such
  * launch, which then must not happen inside a stream capture; at most 64 streams per device, after
- * that AFB_ERR_TOO_LARGE.  Launches that have a form without a workspace take that one instead when
- * only 16 slots are left, or, inside a capture, when only four allocated ones are.  A captured graph keeps using the workspace of the stream it was captured on. */
+ * that AFB_ERR_TOO_LARGE.  A captured graph keeps using the workspace of the stream it was captured on,
+ * so it must not run next to launches on that stream or to other graphs captured on it.
+ * The streaming form of both variants (M >= 4 on large matrices, 17 and more rows, group-scaled int4; see
+ * stream.cu) has workspaces of its own: one per stream (30 MB; afb_init allocates the first) and one per captured
+ * graph (4 to 32 MB, by need), which goes back to the library when the graph and its executables are destroyed: such graphs
+ * may run next to each other and to their capture stream.  (Two executables of ONE graph share its workspace; an executable
+ * updated from another graph uses that graph's, which must then outlive it.)  They are allocated when first needed, also
+ * inside a capture.  At most 256 and 2 GB of them per device; launches beyond that, and launches on cudaStreamPerThread, take a
+ * form without, whose results may differ in the order of the fp32 additions. */
 int afb_gemm_launch(const afb_gemm_args* args, void* stream);
 /* Which variant AFB_VARIANT_AUTO resolves to for these args (no launch). */
 int afb_gemm_resolve_variant(const afb_gemm_args* args, uint32_t* variant);
@@ -336,6 +343,8 @@ int afb_probe_launch(uint32_t kind, const void* src, size_t bytes, uint32_t ctas
 int afb_phase_timestamps(unsigned long long out[8]);
 /* Number of kernels this library launched since afb_init (all variants). */
 unsigned long long afb_launch_count(void);
+/* ... and how many of them were of the streaming form of the decode and prefill variants */
+unsigned long long afb_stream_launch_count(void);
 const char* afb_version(void);
 
 #ifdef __cplusplus

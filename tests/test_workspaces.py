@@ -1,5 +1,6 @@
 """Workspaces of GEMMs that split K between CTAs: who shares one, first launches on new streams, captures, graphs."""
 import ctypes
+import gc
 import threading
 
 import numpy as np
@@ -96,3 +97,92 @@ def test_first_launch_on_a_new_stream_leaves_a_capture_elsewhere_alone(afb):
     graph.replay()
     torch.cuda.synchronize()
     assert x.tolist() == [2.0] * 8
+
+
+def _captured(g):
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(8):
+            g.launch()
+    return graph
+
+
+def test_graphs_of_one_capture_stream_may_run_at_the_same_time(afb):
+    """Two graphs captured one after the other (torch captures on one stream) and eager launches on that very stream, all at once: the
+    streaming form's partial sums and counters are each one's own."""
+    gemms = [Gemm(afb, *STREAMING, seed=3), Gemm(afb, *STREAMING, seed=4), Gemm(afb, *STREAMING, seed=5)]
+    graphs = [_captured(g) for g in gemms[:2]]
+    sides = [torch.cuda.Stream(), torch.cuda.Stream()]
+    capture_stream = torch.cuda.graph.default_capture_stream
+    before = afb.stream_launch_count()
+    for turn in range(10):
+        for graph, side in zip(graphs, sides):
+            with torch.cuda.stream(side):
+                graph.replay()
+        for _ in range(8):
+            gemms[2].launch(capture_stream.cuda_stream)
+        for i, g in enumerate(gemms):
+            g.check(f"turn {turn}, GEMM {i}")
+    assert afb.stream_launch_count() - before == 80   # (a graph's launches are counted when it is captured)
+
+
+def test_streams_at_the_same_time(afb):
+    gemms = [Gemm(afb, *STREAMING, seed=6 + i) for i in range(4)]
+    streams = _new_streams(afb, 4)
+    for turn in range(5):
+        for _ in range(6):
+            for g, s in zip(gemms, streams):
+                g.launch(s)
+        for i, g in enumerate(gemms):
+            g.check(f"turn {turn}, stream {i}")
+
+
+def test_a_graphs_workspace_is_given_back(afb):
+    """Captured, replayed and destroyed forty times: the streaming form stays in use and device memory does not grow by more than what
+    two of the 8 MB workspaces of these launches take, rounded to the allocator's pages."""
+    g = Gemm(afb, *STREAMING, seed=10)
+    for turn in range(40):
+        before = afb.stream_launch_count()
+        graph = _captured(g)
+        assert afb.stream_launch_count() - before == 8
+        graph.replay()
+        g.check(f"turn {turn}")
+        del graph
+        gc.collect()
+        torch.cuda.synchronize()
+        if turn == 1:
+            free = torch.cuda.mem_get_info()[0]
+    assert free - torch.cuda.mem_get_info()[0] <= 32 << 20
+
+
+def test_first_streaming_launch_next_to_a_capture_and_on_the_per_thread_stream(afb):
+    """A first launch on a new stream allocates while another thread captures; the per-thread default stream, one handle for many streams,
+    keeps no workspace and takes the form without."""
+    g = Gemm(afb, *STREAMING, seed=11)
+    streams, graph, failed = _new_streams(afb, 6), torch.cuda.CUDAGraph(), []
+
+    def first_launches():
+        try:
+            for s in streams:
+                g.launch(s)
+        except Exception as e:   # noqa: BLE001
+            failed.append(e)
+
+    x = torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    before = afb.stream_launch_count()
+    with torch.cuda.graph(graph):
+        x += 1
+        t = threading.Thread(target=first_launches)
+        t.start()
+        t.join()
+        x += 1
+    assert not failed and afb.stream_launch_count() - before == 6
+    g.check("launched next to a capture")
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [2.0] * 8
+    g.launch(2)   # cudaStreamPerThread
+    torch.cuda.synchronize()
+    assert afb.stream_launch_count() - before == 6
+    assert ((g.c.float() - g.want.float()).norm() / g.want.float().norm()).item() < 1e-3   # another order of addition: a few roundings
