@@ -97,9 +97,10 @@ uint32_t sub_allreduce_sms();
 int launch_prefill_ts(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, const afb_fused_args* fused = nullptr);   // converted weights in tensor memory
 // Row tiles per group of a persistent kernel's tile order (tiles of bma rows x 128 channels).
 uint32_t pick_group_m(const afb_gemm_args& a, uint32_t m_tiles, uint32_t n_tiles, uint32_t bma, int sms);
-// The streaming form of the decode and prefill variants (stream.cu): launched where it takes the arguments and is the faster one
-// (*done = true, its status returned); otherwise nothing happens and the caller goes on to the other forms.
-int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, bool* done);
+// The streaming form of the decode and prefill variants (stream.cu), for a call that resolved to `variant`: launched where it takes the
+// arguments, is the faster one and no tuning variable asks for another (*done = true, its status returned); otherwise nothing happens
+// and the caller goes on to the other forms.
+int stream_if_faster(const afb_gemm_args& a, uint32_t variant, DeviceCtx* ctx, cudaStream_t s, bool* done);
 int launch_prefill_ts_tiles(const afb_gemm_args& a, DeviceCtx* ctx, uint32_t* tile_done, cudaStream_t s);
 // The sum and broadcast of the pipelined reduce-scatter done inside the pushing GEMM, by two extra warps of every CTA (so that no
 // second kernel has to share SMs with the GEMM): where the finished rows go, the words of the closing signal round, the count

@@ -380,12 +380,12 @@ int afb_gemm_launch(const afb_gemm_args* args, void* stream) {
     switch (v) {
         case AFB_VARIANT_DECODE: {
             bool done = false;
-            rc = stream_if_faster(*args, ctx, s, &done);
+            rc = stream_if_faster(*args, v, ctx, s, &done);
             return done ? rc : launch_decode(*args, ctx, s);
         }
         case AFB_VARIANT_PREFILL: {
             bool done = false;
-            rc = stream_if_faster(*args, ctx, s, &done);
+            rc = stream_if_faster(*args, v, ctx, s, &done);
             if (done) return rc;
             // two implementations of the prefill variant; a flag or AFB_PREFILL_IMPL=ss|ts overrides the default
             static const int env_ts = [] { const char* e = getenv("AFB_PREFILL_IMPL"); return e ? (e[0] == 't' ? 1 : 0) : -1; }();

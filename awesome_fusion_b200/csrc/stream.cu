@@ -633,7 +633,8 @@ bool stream_supports(const afb_gemm_args& a) {
     if (a.k % kSlab || a.lda % 8) return false;
     if (((uint64_t)a.ldb * a.b_bits / 8) % 16) return false;
     if ((uintptr_t)a.ptr_a % 16 || (uintptr_t)a.ptr_b % 16) return false;
-    // forced forms, explicit variants, fp32 results (their order of addition is that of the exchange forms) and the two-term mode stay where they are
+    // forced forms, fp32 results (their order of addition is that of the exchange forms) and the two-term mode stay where they are
+    // (an explicit decode or prefill variant does not: this is a form of both)
     if (a.flags & (AFB_FLAG_C_F32 | AFB_FLAG_PREFILL_SMEM_B | AFB_FLAG_PREFILL_TMEM_A)) return false;
     if ((a.flags & AFB_FLAG_GROUP_EXACT) && a.group_size) return false;
     if (a.group_size) {
@@ -689,11 +690,19 @@ bool is_faster(const afb_gemm_args& a, uint32_t sms) {
 
 }  // namespace
 
-int stream_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, bool* done) {
+// A tuning variable that asks for one of the variant's other forms, or for a shape of theirs.
+static bool other_form_asked(uint32_t variant) {
+    if (variant == AFB_VARIANT_PREFILL) return getenv("AFB_PREFILL_IMPL") != nullptr;
+    for (const char* name : {"AFB_DECODE_BALANCED", "AFB_DECODE_WR", "AFB_DECODE_SLICES", "AFB_DECODE_DEEP_RING", "AFB_DECODE_SINGLE_PASS"})
+        if (getenv(name)) return true;
+    return false;
+}
+
+int stream_if_faster(const afb_gemm_args& a, uint32_t variant, DeviceCtx* ctx, cudaStream_t s, bool* done) {
     *done = false;
     const char* env = getenv("AFB_STREAM");   // tuning aid: 1 wherever possible, 0 never
     const int forced = env ? atoi(env) : -1;
-    if (forced == 0 || !stream_supports(a) || (forced < 0 && !is_faster(a, (uint32_t)ctx->sm_count))) return AFB_OK;
+    if (forced == 0 || !stream_supports(a) || (forced < 0 && (!is_faster(a, (uint32_t)ctx->sm_count) || other_form_asked(variant)))) return AFB_OK;
     const uint32_t sms = (uint32_t)ctx->sm_count;
     StreamParams p{};
     p.c = reinterpret_cast<uint16_t*>(a.ptr_c);

@@ -101,3 +101,30 @@ def test_few_units_next_to_whole_waves(afb, oracle, monkeypatch, m, n, k):
     monkeypatch.delenv("AFB_STREAM")
     sliced = T.make_case(16, 1024, 8192, seed=1)
     check_close(oracle, oracle.gemm(sliced, threads=8), T.run_case(afb, sliced)[0], "decode K-slices after it")
+
+
+def _streamed(afb, m, n, k, **kw):
+    before = afb.stream_launch_count()
+    T.run_case(afb, T.make_case(m, n, k, seed=1), **kw)
+    return afb.stream_launch_count() - before
+
+
+def test_switches_of_the_other_forms_still_reach_them(afb, monkeypatch):
+    """Variables and flags that ask for another form get it, on sizes that the streaming form would take; AFB_STREAM outranks the variables."""
+    monkeypatch.delenv("AFB_STREAM")
+    few, many = (16, 28672, 8192), (40, 8192, 8192)
+    assert _streamed(afb, *few) == 1 and _streamed(afb, *many) == 1
+    for name, value in (("AFB_DECODE_BALANCED", "1"), ("AFB_DECODE_WR", "4"), ("AFB_DECODE_SLICES", "2")):
+        monkeypatch.setenv(name, value)
+        assert _streamed(afb, *few) == 0 and _streamed(afb, *many) == 1, name
+        monkeypatch.delenv(name)
+    monkeypatch.setenv("AFB_PREFILL_IMPL", "ts")
+    assert _streamed(afb, *few) == 1 and _streamed(afb, *many) == 0
+    monkeypatch.setenv("AFB_STREAM", "1")
+    assert _streamed(afb, *many) == 1
+    monkeypatch.setenv("AFB_STREAM", "0")
+    assert _streamed(afb, *few) == 0
+    monkeypatch.delenv("AFB_STREAM")
+    monkeypatch.delenv("AFB_PREFILL_IMPL")
+    for flag in (pkg.FLAG_PREFILL_SMEM_B, pkg.FLAG_PREFILL_TMEM_A):
+        assert _streamed(afb, *many, flags=flag) == 0
