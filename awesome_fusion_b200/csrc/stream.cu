@@ -741,6 +741,7 @@ int stream_if_faster(const afb_gemm_args& a, uint32_t variant, DeviceCtx* ctx, c
     if (p.raw_stages < p.slots * pair || p.slots * pair < (uint32_t)kGroups) return AFB_OK;
 
     p.deal = deal_tiles(p.m_tiles * p.n_tiles, (p.parts + spb - 1) / spb, sms);
+    if (!p.deal.fits()) return AFB_OK;
     const uint32_t grid = p.deal.grid;
     if (p.deal.shared_tiles) {
         if (p.deal.shared_tiles > ctx->stream_counter_count) return AFB_OK;

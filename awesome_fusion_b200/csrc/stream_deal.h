@@ -5,6 +5,7 @@
 // consecutive runs of them, the same number but for one.  The other tiles are dealt whole, one per CTA and wave.
 // No dealer's run is empty (dealers <= units): all CTAs from the first to the last one with a unit of a tile hold some of it, which is
 // what the count of a tile's arrivals and the adding up of its partial sums rely on.
+// 32-bit arithmetic (units * (dealers + 1) < 2^32, which fits() says): the division in begin() comes before a CTA's first load.
 #pragma once
 #include <stdint.h>
 #ifdef __CUDACC__
@@ -22,11 +23,12 @@ struct StreamDeal {
     uint32_t grid;           // CTAs
     uint32_t dealers;        // CTAs [0, dealers) hold units of shared tiles
 
+    bool fits() const { return ((uint64_t)shared_tiles * blocks * (dealers + 1)) >> 32 == 0; }
     AFB_DEAL uint32_t units() const { return shared_tiles * blocks; }
     // first unit of CTA c (= end of CTA c - 1)
-    AFB_DEAL uint32_t begin(uint32_t c) const { return c >= dealers ? units() : (uint32_t)((uint64_t)c * units() / dealers); }
+    AFB_DEAL uint32_t begin(uint32_t c) const { return c >= dealers ? units() : c * units() / dealers; }
     // the CTA holding unit u: the largest c with begin(c) <= u
-    AFB_DEAL uint32_t cta_of(uint32_t u) const { return (uint32_t)((((uint64_t)u + 1) * dealers + units() - 1) / units()) - 1u; }
+    AFB_DEAL uint32_t cta_of(uint32_t u) const { return ((u + 1) * dealers + units() - 1) / units() - 1u; }
     AFB_DEAL uint32_t first_cta(uint32_t t) const { return cta_of(t * blocks); }
     AFB_DEAL uint32_t last_cta(uint32_t t) const { return cta_of(t * blocks + blocks - 1); }
     // Where CTA c leaves its partial sums of shared tile t: slot 2c for the tile its run begins in, 2c + 1 for the one it ends in

@@ -4,9 +4,10 @@
 
 // 0, or which rule is broken: 1 a unit not dealt exactly once, 2 a contributor missing between the first and the last CTA of a tile (it
 // would be waited for), 3 two partial sums in one place, 4 more than two shared tiles to finish in one CTA, 5 a CTA with nothing to do,
-// 6 a run that is longer than another by more than one unit
+// 6 a run that is longer than another by more than one unit, 7 refused as too large
 extern "C" int check_deal(uint32_t tiles, uint32_t blocks, uint32_t sms) {
     const afb::StreamDeal d = afb::deal_tiles(tiles, blocks, sms);
+    if (!d.fits()) return 7;
     std::vector<uint8_t> seen((size_t)tiles * blocks, 0);
     std::vector<uint32_t> arrivals(d.shared_tiles, 0);
     std::vector<uint8_t> slots((size_t)2 * d.grid, 0);
@@ -46,3 +47,4 @@ extern "C" uint32_t check_range(uint32_t tiles_end, uint32_t blocks_end, uint32_
             if (const int rc = check_deal(t, b, sms)) { where[0] = t; where[1] = b; return (uint32_t)rc; }
     return 0;
 }
+extern "C" int fits(uint32_t tiles, uint32_t blocks, uint32_t sms) { return afb::deal_tiles(tiles, blocks, sms).fits(); }

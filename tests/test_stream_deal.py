@@ -16,6 +16,7 @@ def shim(tmp_path_factory):
                            "-o", out, os.path.join(ROOT, "tests", "stream_deal_shim.cc")])
     lib = ctypes.CDLL(out)
     lib.check_deal.argtypes = [ctypes.c_uint32] * 3
+    lib.fits.argtypes = [ctypes.c_uint32] * 3
     lib.check_range.argtypes = [ctypes.c_uint32] * 3 + [ctypes.POINTER(ctypes.c_uint32)]
     return lib
 
@@ -33,3 +34,11 @@ def test_sizes_of_calls(shim, tiles, blocks):
     """24576 x 512 and 25600 x 512 int4 at 17 to 32 rows, 24576 x 768, 2048 rows of 38400 x 768 and of 19456 x 768 (fewer units than
     CTAs next to whole waves: such tiles were lost), and sizes with more units than CTAs."""
     assert shim.check_deal(tiles, blocks, 148) == 0
+
+
+def test_the_limit_of_the_32_bit_arithmetic(shim):
+    """148 SMs, 200 tiles (52 shared): the largest number of blocks that is taken is dealt correctly, one more is refused (the launcher
+    takes another form)."""
+    most = (2 ** 32 - 1) // (52 * 149)
+    assert shim.fits(200, most, 148) and not shim.fits(200, most + 1, 148)
+    assert shim.check_deal(60, 40000, 148) == 0 and shim.check_deal(200, 300000, 148) == 0
