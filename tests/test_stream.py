@@ -128,3 +128,25 @@ def test_switches_of_the_other_forms_still_reach_them(afb, monkeypatch):
     monkeypatch.delenv("AFB_PREFILL_IMPL")
     for flag in (pkg.FLAG_PREFILL_SMEM_B, pkg.FLAG_PREFILL_TMEM_A):
         assert _streamed(afb, *many, flags=flag) == 0
+
+
+def test_group_sums_are_added_in_two_levels(afb):
+    """128 group sums of one sign up to half of K, taken back by the other half: what is left is the error of the fp32 additions.  An addition
+    at a magnitude of at most S (the half sum) is off by 2^-24 S / sqrt(3) in the root mean square; magnitudes that rise from 0 to S and fall
+    again make that 2^-24 S / 3 times the square root of their number: 1.3 for 16 sums of 8 groups (1.4 with the additions inside
+    them), 3.8 for one chain of 128 (2.8 measured).  All tiles are whole ones (148 SMs)."""
+    m, n, k, group = 4, 18944, 16384, 128
+    half, rng = k // 2, np.random.default_rng(3)
+    case = T.make_case(m, 128, k, bits=4, group=group, seed=3, scale_range=(0.005, 0.05))
+    a = np.abs(T.np_bf16_to_f32(case.a))
+    a[:, half:] = -a[:, :half]
+    u = rng.integers(0, 8, size=(n, half), dtype=np.uint8)
+    b = u[:, 0::2] | (u[:, 1::2] << np.uint8(4))
+    scale = T.np_bf16_rne(rng.uniform(0.005, 0.05, size=(n, half // group)).astype(np.float32))
+    case.n, case.a, case.b, case.scale = n, T.np_bf16_rne(a), np.concatenate([b, b], 1), np.concatenate([scale, scale], 1)
+    sums = np.stack([a[:, :half].reshape(m, -1, group)[:, i].astype(np.float64) @ u[:, i * group:(i + 1) * group].T.astype(np.float64)
+                     for i in range(half // group)])   # [group of k][m][n]
+    half_sum = (sums * T.np_bf16_to_f32(scale).T[:, None, :]).sum(0)
+    got, _ = T.run_case(afb, case)
+    off = np.sqrt(((T.np_bf16_to_f32(got) / half_sum) ** 2).mean()) * 2 ** 24
+    assert off < 2, off
