@@ -56,6 +56,16 @@ def _new_streams(lib, count):
     return out
 
 
+@pytest.fixture(scope="module", autouse=True)
+def _leave_no_streams_behind(afb):
+    """These tests use up the workspaces that afb_init allocates; what runs after them finds the library as they did."""
+    yield
+    gc.collect()
+    torch.cuda.synchronize()
+    afb.finalize()
+    afb.init(0)
+
+
 def test_first_launches_on_new_streams_while_the_legacy_stream_is_busy(afb):
     """A stream without a workspace gets one on its first launch.  Its arrival counters are at zero when that launch counts on them,
     whatever waits on the legacy stream (nothing orders a non-blocking stream after it)."""
