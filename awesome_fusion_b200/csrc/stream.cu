@@ -664,34 +664,57 @@ uint32_t tile_rows(const afb_gemm_args& a) {
     return ((a.m + tiles - 1) / tiles + 15) / 16 * 16;
 }
 
-// Where this form is the faster one, from times of both forms on one B200 (us, the other form / this one).
+// Where this form is the faster one, from times of both forms on one B200 (us, the other form / this one): 23 matrices from 1024 x 1024
+// to 28672 x 8192, 35 row counts from 4 to 4096, int8, int4, int4 in groups of 128 and 64, int8 in groups of 128.  At none of those that it takes is this form more than 4 %
+// the slower one.
 bool is_faster(const afb_gemm_args& a, uint32_t sms) {
     const double weights = (double)a.n * a.k, mbytes = weights * a.b_bits / 8 / 1e6;
+    const uint32_t n_tiles = (a.n + kCh - 1) / kCh;
     if (a.m <= 16) {
         // The decode kernel has about 9 us less to set up and finish, and its arithmetic grows with M; this form's does not.
         //   28672 x 8192 int8   M = 2: 44 / 44   4: 51 / 44    8: 68 / 44   16: 64 / 45
-        //   28672 x 8192 int4   M = 1: 40 / 50   4: 53 / 50    8: 64 / 50   16: 63 / 50    (group 128)
-        //   12288 x 4096 int8   M = 1: 14 / 22   8: 21 / 22   16: 27 / 22
-        //    4096 x 11008 int4  M = 1: 14 / 21   4: 22 / 21    8: 30 / 21   16: 31 / 22    (one activation row is staged in several passes)
-        //   12288 x 4096 int4   M = 8: 18 / 24  16: 23 / 23;   4096 x 4096: never
+        //   28672 x 8192 int4   M = 4: 53 / 50   5: 57 / 50    8: 64 / 50   16: 63 / 50    (group 128; without groups 4: 45 / 50   5: 50 / 50)
+        //   12288 x 4096 int8   M = 8: 21 / 22  16: 27 / 22;   4096 x 4096: never
         if (mbytes >= 100) return a.m >= (a.b_bits == 8 ? 4u : 5u);
-        if (a.k >= 8192 && mbytes >= 20) return a.m >= 8;
+        // Long rows: the decode kernel stages the activations in several passes.  Without groups its int4 arithmetic is so much
+        // cheaper that this must cost it more, more than 192 KiB of activations:
+        //   4096 x 11008 int4   M = 8: 30 / 21 (group 128)   8: 20 / 22   9: 34 / 22 (no groups);   8192 x 8192 int4   M = 9: 20 / 22   12: 25 / 22
+        if (a.k >= 8192 && mbytes >= 20) return a.m >= 8 && (a.b_bits == 8 || a.group_size || a.m * a.k >= 98304);
         return mbytes >= 40 && a.m >= 9;
     }
     if (a.m <= 128) {
-        // Both other forms unpack at the pace of one step's hand-off chain (79 to 88 us on 28672 x 8192 whatever M is: 45 to 69 here;
-        // 8192 x 8192: 29 to 31 / 24 to 31 int8, 41 / 23 to 31 int4; 12288 x 4096: 29 to 38 / 22 to 30).  On small matrices what
-        // remains is the cost of sharing tiles between CTAs (4096 x 4096: 16 / 17 to 22 int8, 18 / 16 to 23 int4).
-        return weights >= 40e6 || (a.b_bits == 4 && a.m <= 40);
+        // Both other forms unpack at the pace of one step's hand-off chain (79 to 88 us on 28672 x 8192 whatever M is: 45 to 69 here);
+        // what remains here is the cost of sharing tiles between CTAs, which grows with M.
+        if (weights >= 40e6) {
+            // group-scaled:  8192 x 8192 int4: 41 / 23 to 31;  int4 in short rows of more than a wave of tiles, 28672 x 2048: 26 / 22 at M = 17,
+            // 26 / 23 at 40, 27 / 31 at 128 (groups of 64: 0.98 at 32, 1.11 at 40)
+            if (a.group_size) return a.b_bits == 8 || n_tiles <= sms || a.k >= 4096 || a.m <= (a.group_size % 128 ? 32u : 64u);
+            // int8:  8192 x 8192: 29 to 31 / 24 to 31;  12288 x 4096: 25 / 23 at M = 64, 25 / 27 at 128;  4096 x 11008: 24 / 24 and 25 / 29
+            return a.m <= 64 || weights >= 55e6;
+        }
+        if (a.b_bits == 8 || a.m > 40) return false;   // 4096 x 4096 int8: 16 / 17 to 22
+        // Small int4 matrices, up to 40 rows.  Tiles that fill half a wave to a whole one keep the other forms busy, too:
+        // 12288 x 1024: 13 / 16 group-scaled, 10 / 16 without; 16384 x 2048: 18 / 15 and 16 / 14 to 18
+        if (n_tiles > sms / 2 && n_tiles <= sms) return a.k >= 2048 && (a.group_size || a.m <= 24);
+        if (n_tiles > sms && a.group_size && a.k < 1536) return a.m <= 32;   // 28672 x 1024: 16 / 16 at 32, 16 / 17 at 40 (groups of 64: 1.13)
+        if (a.group_size) return true;                 // 1024 x 1024 ... 8192 x 2560: this form 0.8 to 0.95 of the other; 1024 x 11008 0.3
+        // 4096 x 4096: 15 / 15 at M = 20, 15 / 17 at 40;  3072 x 3072: 13 / 13 and 13 / 14;  5120 x 5120 and 1024 x 11008: 0.85 and 0.7 throughout
+        return a.m <= 24 || n_tiles > sms || a.k >= 8192 || weights >= 25e6 || weights <= 5e6;
     }
     // Many rows: the tensor-memory form with 256-row tiles has the higher rate, this one fits its tiles to M and shares the last
-    // ones evenly.  Group-scaled int4 is bound by the unpack there and faster here throughout (28672 x 8192 group 128: 154 / 113 at
-    // M = 256, 245 / 222 at 512, 971 / 915 at 2048, 1904 / 1819 at 4096; 4096 x 4096: 30 / 31 at 512, 72 / 69 at 2048).
-    if (a.b_bits == 4 && a.group_size) return weights >= 40e6 || weights * a.m >= 30e9;
-    // Otherwise compared in rows per SM, with 1.2 for the difference in rate (int8: 28672 x 8192: 117 / 99 at M = 129, 182 / 164 at
-    // 333, 186 / 213 at 512; 11008 x 4096: 50 / 43 at 333, 51 / 50 at 512, 81 / 71 at 777, 138 / 160 at 2048).
+    // ones evenly.  Group-scaled int4 is bound by the unpack there and faster here (28672 x 8192 group 128: 138 / 114 at
+    // M = 256, 261 / 223 at 512, 971 / 915 at 2048, 1904 / 1819 at 4096; 4096 x 4096: 29 / 30 at 512, 72 / 68 at 2048), but for
+    // next to no channels and very many rows (1024 x 11008: 91 / 77 at 3000, 94 / 110 at 4096; groups of 64 0.86).
+    if (a.b_bits == 4 && a.group_size) return weights >= 40e6 || (weights * a.m >= 30e9 && (n_tiles >= 16 || a.m <= 3072 || a.group_size % 128));
+    // Otherwise compared in rows per SM, with 1.2 for the difference in rate.  Without group scales the other form has little to unpack
+    // besides, and the comparison holds only where its 256-row tiles are mostly padding: one tile and a little more (28672 x 8192 int8:
+    // 102 / 86 at M = 129, 106 / 109 at 200; 8192 x 8192: 37 / 35 and 38 / 41; 12288 x 4096: 28 / 31 at 129), or two, with enough channels
+    // (11008 x 4096: 47 / 40 at 333; 8192 x 8192: 50 / 52; at 640 and 777 rows 12288 x 4096: 56 / 63 and 78 / 80, 28672 x 8192: 353 / 392).
+    // Between 193 and 256 rows it would also add up longer stretches of K in one accumulator than the other form, which cuts them
+    // (8192 x 8192, 200 rows: 13057 of 9830400 results wrongly rounded, 9665 there).
     if (weights < 40e6) return false;
-    const uint32_t n_tiles = (a.n + kCh - 1) / kCh, rows = tile_rows(a);
+    if (!a.group_size && !(a.m <= 192 ? weights >= 60e6 : a.m > 256 && a.m <= 384 && n_tiles >= 80)) return false;
+    const uint32_t rows = tile_rows(a);
     const uint32_t others = (a.m + 255) / 256 * n_tiles, waves = others / sms, rest = others % sms;
     const uint32_t parts = rest == 0 || rest > sms / 2 ? 1 : sms / rest < 4 ? sms / rest : 4;
     const double there = 256.0 * (waves + (rest ? 1.0 / parts : 0.0)), here = (double)((a.m + rows - 1) / rows) * n_tiles * rows / sms;

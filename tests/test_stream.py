@@ -150,3 +150,26 @@ def test_group_sums_are_added_in_two_levels(afb):
     got, _ = T.run_case(afb, case)
     off = np.sqrt(((T.np_bf16_to_f32(got) / half_sum) ** 2).mean()) * 2 ** 24
     assert off < 2, off
+
+
+@pytest.mark.parametrize("m,n,k,bits,group,streamed", [
+    (3, 28672, 8192, 8, 0, 0), (4, 28672, 8192, 8, 0, 1), (4, 28672, 8192, 4, 128, 0), (5, 28672, 8192, 4, 128, 1), (16, 4096, 4096, 8, 0, 0),
+    (9, 12288, 4096, 8, 0, 1), (8, 8192, 8192, 4, 0, 0), (12, 8192, 8192, 4, 0, 1), (8, 4096, 11008, 4, 128, 1), (17, 12288, 1024, 4, 128, 0),
+    (40, 16384, 2048, 4, 128, 1), (24, 4096, 4096, 4, 0, 1), (40, 4096, 4096, 4, 0, 0), (40, 4096, 4096, 8, 0, 0), (64, 12288, 4096, 8, 0, 1),
+    (80, 12288, 4096, 8, 0, 0), (128, 8192, 8192, 8, 0, 1), (129, 8192, 8192, 8, 0, 1), (200, 8192, 8192, 8, 0, 0), (129, 12288, 4096, 8, 0, 0),
+    (333, 11000, 4096, 8, 0, 1), (333, 8192, 8192, 8, 0, 0), (777, 12288, 4096, 8, 0, 0), (777, 12288, 4096, 4, 128, 1), (4096, 1024, 11008, 4, 128, 0), (40, 28672, 2048, 4, 64, 0),
+    (40, 28672, 2048, 4, 128, 1), (777, 12288, 4096, 8, 128, 1), (40, 28672, 1024, 4, 128, 0)])
+def test_choice_of_the_form(afb, monkeypatch, m, n, k, bits, group, streamed):
+    """On both sides of the lines of the automatic choice (148 SMs)."""
+    monkeypatch.delenv("AFB_STREAM")
+    before = afb.stream_launch_count()
+    a, b, s, c = (afb.malloc(size) for size in (m * k * 2, n * k * bits // 8, n * (k // group if group else 1) * 4, m * n * 2))
+    try:
+        for p, size in ((a, m * k * 2), (b, n * k * bits // 8), (s, n * (k // group if group else 1) * 4)):
+            afb.memset(p, 0, size)
+        afb.gemm_launch(afb.make_args(c, a, b, s, m, n, k, bits=bits, group=group, scale_dtype=pkg.SCALE_BF16 if group else pkg.SCALE_F32))
+        afb.device_sync()
+    finally:
+        for p in (a, b, s, c):
+            afb.free(p)
+    assert afb.stream_launch_count() - before == streamed
