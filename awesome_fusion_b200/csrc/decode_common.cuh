@@ -87,7 +87,7 @@ __device__ __forceinline__ void decode_finish(const DecodeParams& p, const float
         float sum = 0.f;
         for (uint32_t w = 0; w < wk_count; ++w) sum += s_red[((w0 + w) * 16 + (r & 15)) * 17 + mm];
         if (single) {
-            sum *= GROUPED ? kUnpackInverse : kUnpackInverse * load_scale(p.scale, nn, p.scale_dtype);
+            sum = GROUPED ? sum * kUnpackInverse : unscaled(sum, load_scale(p.scale, nn, p.scale_dtype));
             p.c[(size_t)mm * p.ldc + nn] = __bfloat16_as_ushort(__float2bfloat16_rn(sum));
         } else {
             __stcg(p.ws + ((size_t)my_slot * p.m + mm) * p.n + nn, sum);
@@ -116,7 +116,7 @@ __device__ __forceinline__ void decode_finish(const DecodeParams& p, const float
 #pragma unroll
                     for (int i2 = 0; i2 < 8; ++i2) sum += v[i2];
                 }
-                sum *= GROUPED ? kUnpackInverse : kUnpackInverse * load_scale(p.scale, nn, p.scale_dtype);
+                sum = GROUPED ? sum * kUnpackInverse : unscaled(sum, load_scale(p.scale, nn, p.scale_dtype));
                 p.c[(size_t)mm * p.ldc + nn] = __bfloat16_as_ushort(__float2bfloat16_rn(sum));
             }
             if (tid == 0) p.counters[cb] = 0u;  // ready for the next launch

@@ -7,8 +7,10 @@
 //     fma(u * 2^-133, 2^127, -(128 + zero) * 2^-6)  =  (u - 128 - zero) * 2^-6,
 // makes two exact weights of it (both operands and the result have at most 8 significant bits).  An int4 weight in the upper
 // half of a byte is 16 u * 2^-133 and takes 2^123.  Zero-points and the storage encoding live in the constants.
-// Every routine returns the weights times kUnpackFactor = 2^-6; the kernels multiply the finished fp32 sums by 64 (powers of
-// two: no bit of a result depends on it).  Cost per 4 int8 weights: 1 xor + 2 permutes + 2 fma (splice, sign and add: 8 in natural
+// Every routine returns the weights times kUnpackFactor = 2^-6; the kernels multiply the finished fp32 sums by 64, and only then by a
+// channel's scale (64 * scale overflows from 2^122 on).  Powers of two: no bit of a result depends on it while the products of weight
+// and activation stay in the normal range of fp32 with the factor, that is above 2^-120 (with folded group scales 2^-116).  Group scales
+// below 2^-100 are not folded; their weights q * scale * 2^-10 lose bits once q * scale is below 2^-116.  Cost per 4 int8 weights: 1 xor + 2 permutes + 2 fma (splice, sign and add: 8 in natural
 // order, 7 strided); per 8 int4 weights 10 in natural order, 9 strided (13, 11).  The unpack is what the decode kernels and the
 // converter warps of the prefill kernels issue most; see the figures there.
 #pragma once
@@ -43,6 +45,7 @@ __device__ __forceinline__ uint32_t bf16x2_fma(uint32_t a, uint32_t b, uint32_t 
 
 // What the unpack adds and multiplies.  kUnpackFactor * 64 = 1.
 constexpr float kUnpackInverse = 64.f;
+__device__ __forceinline__ float unscaled(float sum, float scale) { return (sum * kUnpackInverse) * scale; }
 constexpr uint32_t kMulByte = 0x7F007F00u;       // 2^127 in both halves: weights in the low bits of their byte
 constexpr uint32_t kMulHighNibble = 0x7D007D00u; // 2^123: weights in bits [4,8) of their byte
 constexpr uint32_t kMulNibblePair = 0x7D007F00u; // low half from bits [0,4), high half from bits [4,8)

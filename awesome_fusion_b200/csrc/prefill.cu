@@ -224,7 +224,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                                 float sc[8];
                                 load_scale8(p.scale, p.scale_dtype, col, sc);  // same address in all lanes: one broadcast
 #pragma unroll
-                                for (int e = 0; e < 8; ++e) v[e] *= kUnpackInverse * sc[e];
+                                for (int e = 0; e < 8; ++e) v[e] = unscaled(v[e], sc[e]);
                             } else {
 #pragma unroll
                                 for (int e = 0; e < 8; ++e) v[e] *= kUnpackInverse;

@@ -461,9 +461,11 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
             ptx::tc_fence_after_sync();
             count_pending();   // the previous tile of this CTA (pipelined reduce-scatter only)
             float scale = GROUPED ? kGroupInverse : 0.f;
+            bool huge = false;   // 64 * scale could overflow: the factor is taken out of the accumulator instead
             if (!GROUPED && nn < p.n)
-                scale = kUnpackInverse * (p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn] << 16)
-                                                       : reinterpret_cast<const float*>(p.scale)[nn]);
+                scale = p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn] << 16)
+                                                        : reinterpret_cast<const float*>(p.scale)[nn];
+            if (!GROUPED) { huge = fabsf(scale) >= 0x1p121f; scale *= huge ? 1.f : kUnpackInverse; }
             if (p.push_on == 2 && !wait_or_abort(bar_tile_fwd, (it & 1u) ^ 1u, abort_flag)) {   // the previous tile has left
                 if (!*abort_flag) { report_timeout(p.status, 26, (int)t, -1); *abort_flag = 1; }
                 break;
@@ -474,6 +476,10 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
                 const uint32_t col = kq * kColsPerWarp + c0;
                 ptx::tmem_ld_32x32(tmem_base + ((q * 32u) << 16) + col, r);
                 ptx::tmem_ld_wait();
+                if (!GROUPED && huge && !w.tail) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * kUnpackInverse);
+                }
                 if (w.tail) {   // a stretch of K of a tail tile: the raw fp32 sums go to the workspace, [part][row][channel]
                     float* wsp = p.tail_ws + ((size_t)(w.tail_r * p.tail_parts + w.part) * BMA + col) * BNW + ch;
 #pragma unroll
@@ -584,13 +590,13 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
                     __threadfence();
                     const uint32_t tid = threadIdx.x - 64;                  // 0 .. 255 over the converter warps
                     const uint32_t c4 = tid & 31u, nv = n0 + c4 * 4;        // this thread's four channels (the same in every row)
-                    float sc4[4] = {kGroupInverse, kGroupInverse, kGroupInverse, kGroupInverse};
+                    float sc4[4] = {0.f, 0.f, 0.f, 0.f};
                     if (!GROUPED) {
 #pragma unroll
                         for (int e = 0; e < 4; ++e)
                             if (nv + e < p.n)
-                                sc4[e] = kUnpackInverse * (p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nv + e] << 16)
-                                                                         : reinterpret_cast<const float*>(p.scale)[nv + e]);
+                                sc4[e] = p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nv + e] << 16)
+                                                                         : reinterpret_cast<const float*>(p.scale)[nv + e];
                     }
                     const float* wst = p.tail_ws + (size_t)w.tail_r * p.tail_parts * BMA * BNW;
                     constexpr uint32_t kVecs = BMA * (BNW / 4), kMaxParts = 4, kU = 4;
@@ -610,7 +616,8 @@ prefill_ts_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_con
                                 if (j < p.tail_parts) { a4.x += v[j][u2].x; a4.y += v[j][u2].y; a4.z += v[j][u2].z; a4.w += v[j][u2].w; }
                             const uint32_t row = (base + u2 * 256) >> 5, mrow = m0 + row;
                             if (mrow < p.m && nv < p.n) {
-                                a4.x *= sc4[0]; a4.y *= sc4[1]; a4.z *= sc4[2]; a4.w *= sc4[3];
+                                if (GROUPED) { a4.x *= kGroupInverse; a4.y *= kGroupInverse; a4.z *= kGroupInverse; a4.w *= kGroupInverse; }
+                                else { a4.x = unscaled(a4.x, sc4[0]); a4.y = unscaled(a4.y, sc4[1]); a4.z = unscaled(a4.z, sc4[2]); a4.w = unscaled(a4.w, sc4[3]); }
                                 if (p.c_f32) {
                                     *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.c) + (size_t)mrow * p.ldc + nv) = a4;
                                 } else {

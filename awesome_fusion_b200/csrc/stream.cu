@@ -190,6 +190,15 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
     Piece x;
     auto parts_of = [&](const Piece& q) { return min(q.kb1 * SPB, p.parts) - q.kb0 * SPB; };
 
+    auto channel_scale = [&](uint32_t nn) {
+        if (!channel_scaled(MODE) || nn >= p.n) return 0.f;
+        return p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn] << 16)
+                                               : reinterpret_cast<const float*>(p.scale)[nn];
+    };
+    auto finished = [&](float sum, float scale) {
+        return channel_scaled(MODE) ? unscaled(sum, scale) : sum * (MODE == kSums ? kUnpackInverse : kGroupInverse);
+    };
+
     // Adds the partial sums of shared tile t in CTA order, scales, rounds and stores it; `tid` of `threads` threads, four channels of
     // one row at a time, up to eight 16-byte loads in flight per thread.
     auto finish_tile = [&](uint32_t t, uint32_t tid, uint32_t threads) {
@@ -201,9 +210,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         float sc[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-            sc[e] = MODE == kSums ? kUnpackInverse : MODE == kFold ? kGroupInverse : nn + e >= p.n ? 0.f :
-                kUnpackInverse * (p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn + e] << 16)
-                                                                  : reinterpret_cast<const float*>(p.scale)[nn + e]);
+            sc[e] = channel_scale(nn + e);
         const uint32_t first_slot = p.deal.slot(first, t);   // the others' runs begin in this tile: slot 2c
         const size_t stride = (size_t)p.rows * kCh;
         for (uint32_t v = tid; v < vecs; v += 2 * threads) {
@@ -226,7 +233,8 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (v + h * threads >= vecs) break;
-                const __nv_bfloat162 lo = __floats2bfloat162_rn(sum[h].x * sc[0], sum[h].y * sc[1]), hi = __floats2bfloat162_rn(sum[h].z * sc[2], sum[h].w * sc[3]);
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(finished(sum[h].x, sc[0]), finished(sum[h].y, sc[1])),
+                                     hi = __floats2bfloat162_rn(finished(sum[h].z, sc[2]), finished(sum[h].w, sc[3]));
                 uint16_t* dst = p.c + (size_t)(m0 + (v + h * threads) / (kCh / 4)) * p.ldc + nn;
                 if (p.c_vec && nn + 4 <= p.n) {
                     *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
@@ -437,9 +445,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
             const uint32_t nn = n0 + ch, ns = parts_of(x);
             const uint32_t valid = min(p.rows, p.m - m0);
             const bool whole = x.kb0 == 0 && x.kb1 == p.deal.blocks;
-            const float scale = MODE == kSums ? kUnpackInverse : MODE == kFold ? kGroupInverse :
-                nn >= p.n ? 0.f : kUnpackInverse * (p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[nn] << 16)
-                                                                                    : reinterpret_cast<const float*>(p.scale)[nn]);
+            const float scale = channel_scale(nn);
             // 16 rows of this lane's channel, finished
             auto store = [&](uint32_t c0, const float (&v)[16]) {
                 if (p.c_tma) {
@@ -450,7 +456,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
                         asm volatile("st.shared.u16 [%0], %1;" ::"r"(out + (uint32_t)j * 64u + (uint32_t)lane * 2u),
-                                     "h"(__bfloat16_as_ushort(__float2bfloat16_rn(v[j] * scale))) : "memory");
+                                     "h"(__bfloat16_as_ushort(__float2bfloat16_rn(finished(v[j], scale)))) : "memory");
                     ptx::fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -462,7 +468,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                     uint16_t* dst = p.c + (size_t)(m0 + c0) * p.ldc + nn;
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        if (c0 + j < valid) dst[(size_t)j * p.ldc] = __bfloat16_as_ushort(__float2bfloat16_rn(v[j] * scale));
+                        if (c0 + j < valid) dst[(size_t)j * p.ldc] = __bfloat16_as_ushort(__float2bfloat16_rn(finished(v[j], scale)));
                 }
             };
             float* part = p.ws + (size_t)(whole ? 0 : p.deal.slot(blockIdx.x, x.t)) * p.rows * kCh + ch;

@@ -514,3 +514,27 @@ def test_decode_back_to_back_with_dependent_launch(afb, oracle, m, n, k, bits, g
         assert np.array_equal(a, b)
         check_close(oracle, oracle.gemm(c, threads=4), a, f"decode with dependent launch {m}x{n}x{k}")
     assert afb.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("form", ["decode", "stream-few", "stream-many", "smem", "tmem", "tail", "fused"])
+def test_channel_scales_at_the_upper_end(afb, oracle, monkeypatch, form):
+    """Channel scales around 2^123 with activations that keep the results finite: the unpack's factor is taken out of the sum before the
+    scale is applied (64 * 2^123 would overflow)."""
+    monkeypatch.setenv("AFB_STREAM", "1" if form.startswith("stream") else "0")
+    m = {"decode": 8, "stream-few": 8, "tail": 192}.get(form, 64)
+    case = T.make_case(m, 264, 2048 if form == "tail" else 512, seed=11, scale_range=(0.5, 1.0))
+    plain = oracle.gemm(case, threads=4)
+    case.a = T.np_bf16_rne(T.np_bf16_to_f32(case.a) * np.float32(2.0 ** -24))
+    case.scale = case.scale * np.float32(2.0 ** 124)
+    if form == "fused":
+        d_a, d_b, d_s, d_c = (afb.to_device(x) for x in (case.a, case.b, case.scale, np.zeros((m, case.n), np.uint16)))
+        afb.gemm_fused_launch(afb.make_fused_args(afb.make_args(d_c, d_a, d_b, d_s, m, case.n, case.k)))
+        afb.device_sync()
+        got = afb.to_host(d_c, (m, case.n), np.uint16)
+        for p in (d_a, d_b, d_s, d_c):
+            afb.free(p)
+    else:
+        got, _ = T.run_case(afb, case, flags={"smem": pkg.FLAG_PREFILL_SMEM_B, "tmem": pkg.FLAG_PREFILL_TMEM_A, "tail": pkg.FLAG_PREFILL_TMEM_A}.get(form, 0))
+    got32 = T.np_bf16_to_f32(got)
+    assert np.isfinite(got32).all()
+    check_close(oracle, plain, T.np_bf16_rne(got32 * np.float32(2.0 ** -100)), form)   # exact: powers of two in and out
