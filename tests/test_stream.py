@@ -14,8 +14,10 @@ pytestmark = pytest.mark.gpu
 
 
 def _check(afb, oracle, case, what, **kw):
+    before = afb.stream_launch_count()
     got, _ = T.run_case(afb, case, **kw)
     again, _ = T.run_case(afb, case, **kw)
+    assert afb.stream_launch_count() - before == 2, f"{what}: another form took the call"
     assert np.array_equal(got, again), f"{what}: two runs differ"
     folded = case.group and case.m > 16   # the weights are rounded to bf16 once more, as in the other prefill forms
     check_close(oracle, oracle.gemm(case, threads=8, round_w=bool(folded)), got, what)
@@ -173,3 +175,45 @@ def test_choice_of_the_form(afb, monkeypatch, m, n, k, bits, group, streamed):
         for p in (a, b, s, c):
             afb.free(p)
     assert afb.stream_launch_count() - before == streamed
+
+
+def test_dependent_launches_in_a_chain(afb):
+    """GEMMs of a decode loop back to back with AFB_FLAG_PDL, each reading what the one before it wrote, all in the streaming form: eagerly
+    and captured, the bits of launches that wait for one another."""
+    torch = pytest.importorskip("torch")
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(5)
+    h, m, layers = 8192, 16, 4
+    weights = [torch.randint(-127, 128, (h, h), device="cuda", generator=gen, dtype=torch.int8) for _ in range(layers)]
+    scale = torch.full((h,), 1.0 / (73.6 * h ** 0.5), device="cuda")   # keeps the activations near N(0, 1)
+    x = [torch.randn((m, h), device="cuda", generator=gen).bfloat16()] + [torch.empty((m, h), device="cuda", dtype=torch.bfloat16) for _ in range(layers)]
+
+    def chain(flags, wait):
+        for i, w in enumerate(weights):
+            afb.gemm_launch(afb.make_args(x[i + 1], x[i], w, scale, m, h, h, flags=flags), torch.cuda.current_stream().cuda_stream)
+            if wait:
+                torch.cuda.synchronize()
+
+    def clear():
+        for t in x[1:]:
+            t.fill_(float("nan"))
+        torch.cuda.synchronize()
+
+    before = afb.stream_launch_count()
+    chain(0, True)
+    assert afb.stream_launch_count() - before == layers
+    want = [t.clone() for t in x]
+    assert all(0.5 < t.float().std().item() < 2 for t in want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain(pkg.FLAG_PDL, False)
+    for turn in range(6):
+        clear()
+        if turn % 2:
+            graph.replay()
+        else:
+            for _ in range(3):
+                chain(pkg.FLAG_PDL, False)
+        torch.cuda.synchronize()
+        for i, (got, ref) in enumerate(zip(x, want)):
+            assert torch.equal(got, ref), f"turn {turn}, layer {i}"
