@@ -81,11 +81,13 @@ cudaError_t allocate_workspace(float** ws, size_t bytes, uint32_t** counters, si
     return e;
 }
 
-// Memory of a streaming workspace: the partial sums, behind them the counters.
+// Memory of a streaming workspace: the counters, behind them the partial sums.  They share a page: the count is the last thing that
+// a launch waits for, and a page of its own would be looked up only then.
 cudaError_t allocate_stream_workspace(DeviceCtx* ctx, DeviceCtx::StreamWorkspace* w, size_t bytes) {
-    const cudaError_t e = cudaMalloc(&w->ws, bytes + ctx->stream_counter_count * sizeof(uint32_t));
-    if (e != cudaSuccess) { w->ws = nullptr; return e; }
-    w->counters = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(w->ws) + bytes);
+    const size_t counter_bytes = (ctx->stream_counter_count * sizeof(uint32_t) + 1023) / 1024 * 1024;
+    const cudaError_t e = cudaMalloc(&w->counters, counter_bytes + bytes);
+    if (e != cudaSuccess) { w->counters = nullptr; return e; }
+    w->ws = reinterpret_cast<float*>(reinterpret_cast<char*>(w->counters) + counter_bytes);
     w->bytes = bytes;
     ctx->stream_workspace_total += bytes;
     return e;
@@ -291,7 +293,7 @@ int afb_finalize(void) {
     cudaDeviceSynchronize();
     cudaFree(c.status); cudaFree(c.ar_words); cudaFree(c.phase_ts);
     for (auto& w : c.workspaces) { if (w.ws) cudaFree(w.ws); if (w.counters) cudaFree(w.counters); }
-    for (auto& w : c.stream_workspaces) { if (w.ws) cudaFree(w.ws); if (w.hold) w.hold->release(); }
+    for (auto& w : c.stream_workspaces) { if (w.counters) cudaFree(w.counters); if (w.hold) w.hold->release(); }
     if (c.clear_stream) cudaStreamDestroy(c.clear_stream);
     for (int j = 0; j < 2; ++j) {
         for (int i = 0; i < 4; ++i) if (c.stage[j][i]) cudaFree(c.stage[j][i]);
