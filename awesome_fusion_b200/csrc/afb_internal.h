@@ -29,7 +29,8 @@ struct DeviceCtx {
     size_t    splitk_counter_count = 0;   // counters of every workspace
     // The streaming form's workspaces.  Nearly all its launches need one, also of sizes whose other form needs none; so they are apart
     // from those above, and a captured graph has one of its own: graphs captured on the same stream, and that stream itself, may run at
-    // the same time.  A graph's workspace goes back to the pool when the graph and its executables are gone (`hold`).
+    // the same time.  The first few graphs keep theirs; a further graph's goes back to the pool when the graph and its executables are
+    // gone (`hold`).
     struct GraphHold;
     static constexpr int kMaxStreamWorkspaces = 256;
     struct StreamWorkspace {
@@ -43,6 +44,7 @@ struct DeviceCtx {
     };
     StreamWorkspace stream_workspaces[kMaxStreamWorkspaces];
     size_t       stream_workspace_total = 0;    // bytes of them all
+    int          kept_graph_workspaces = 0;     // taken by graphs for good
     size_t       stream_counter_count = 0;      // counters of every one
     cudaStream_t clear_stream = nullptr;        // clears the counters of a workspace that is taken inside a capture
     // optional phase timestamps (globaltimer ns of THIS GPU) written by the row-parallel GEMM and the exchange kernel when the

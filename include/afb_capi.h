@@ -136,8 +136,9 @@ int afb_device_sync(void);
  * so it must not run next to launches on that stream or to other graphs captured on it.
  * The streaming form of both variants (M >= 4 on large matrices, 17 and more rows, group-scaled int4; see
  * stream.cu) has workspaces of its own: one per stream (30 MB; afb_init allocates the first) and one per captured
- * graph (4 to 32 MB, by need), which goes back to the library when the graph and its executables are destroyed: such graphs
- * may run next to each other and to their capture stream.  (Two executables of ONE graph share its workspace; an executable
+ * graph (4 to 32 MB, by need): such graphs may run next to each other and to their capture stream.  The first 32 captured graphs
+ * keep theirs until afb_finalize; a further graph's goes back to the library when the graph and its executables are destroyed,
+ * which costs its replays 2.5 us each.  (Two executables of ONE graph share its workspace; an executable
  * updated from another graph uses that graph's, which must then outlive it.)  They are allocated when first needed, also
  * inside a capture.  At most 256 and 2 GB of them per device; launches beyond that, and launches on cudaStreamPerThread, take a
  * form without, whose results may differ in the order of the fp32 additions. */
