@@ -5,14 +5,15 @@
 // D[n, m] = sum_k W[n,k] * A[m,k]: a tile has 128 output channels (the TMEM lanes) and `rows` activation rows (a multiple of 16,
 // fitted to M).  One CTA per SM:
 //
-//   warp 0      (1 lane)  TMA: raw weight blocks, 128 channels x 128 bytes (128 k of int8, 256 k of int4), 128-byte swizzle
-//   warp 1      (1 lane)  TMA: activation slabs [rows x 64] bf16, 128-byte swizzle
-//   warp 2      (1 lane)  tcgen05.mma 128 x rows x 16, weights from TMEM, activations from shared memory
+//   warp 0                TMA: raw weight blocks, 128 channels x 128 bytes (128 k of int8, 256 k of int4), 128-byte swizzle
+//   warp 1                TMA: activation slabs [rows x 64] bf16, 128-byte swizzle
+//   warp 2                tcgen05.mma 128 x rows x 16, weights from TMEM, activations from shared memory
+//                         (warps 0 to 2 run as whole warps and elect a lane for the asynchronous instructions)
 //   warps 4-7             epilogue, one lane quarter each: accumulator -> scale -> bf16 -> C, or fp32 partial sums -> workspace
-//   warps 8-23            converters: four groups of four warps (one per lane quarter); group g takes every fourth 64-wide step,
-//                         so that four steps are being unpacked at any time.  A warp's chain wait -> load -> unpack -> tcgen05.st
-//                         -> arrive takes about 800 cycles; what bounds a form in which all converters share ONE step is that
-//                         chain, whatever M is.
+//   warps 8-23            converters: four groups of four warps (one per lane quarter); group g takes every fourth part of k,
+//                         64 or 128 wide, so that four parts are being unpacked at any time.  A warp's chain wait -> load ->
+//                         unpack -> tcgen05.st -> arrive takes about 800 cycles; what bounds a form in which all converters
+//                         share ONE step is that chain, whatever M is.
 //
 // k goes by in parts (one converter group's work: 64 or 128 k) and steps (one hand-off to and from the issuing warp: one part, or
 // two where few rows make the hand-off the larger cost).  Weights and activations have rings of their own.
@@ -20,11 +21,12 @@
 // waves (contiguous, so at most two of its tiles are shared with neighbours), then whole tiles, one wave after the other.
 // A shared tile is finished by the last CTA to arrive, which adds the fp32 partial sums in CTA order (= ascending K): the bits do
 // not depend on who that is, and no CTA waits for another.  Up to 16 rows the group scales multiply the fp32 sum of each group, in the
-// epilogue warps, while the next groups are being computed; above that they are folded into the bf16 weights.
+// epilogue warps, while the next groups are being computed (per-channel sums are handed over every 1024 k); above that they are folded
+// into the bf16 weights.
 //
 // What bounds it: for few rows int8 the weight stream (28672 x 8192, 16 rows: 44.7 us = 5.3 TB/s of weights, 63.8 with decode.cu; the
 // stream, the hand-offs and the shared tiles alone, without unpack and MMAs, take 44.7 too), int4 the issue slots of the unpack and of
-// the hand-offs (50 against 63 us; 40 without unpack and MMAs); for 65 to 128 rows the activations through L2 (28672 x 8192 int4
+// the hand-offs (50 against 63 us with decode.cu; 40 without unpack and MMAs); for 65 to 128 rows the activations through L2 (28672 x 8192 int4
 // group-128, 128 rows: 66 us, 82 with prefill.cu); for many rows the pace of the issuing warp next to the unpack.
 #include <cstdlib>
 #include "afb_internal.h"
@@ -44,7 +46,7 @@ constexpr int kFirstEpi = 4, kFirstConv = 8;
 constexpr int kThreads = 32 * (kFirstConv + 4 * kGroups);
 constexpr int kMaxRaw = 12, kMaxSlots = 8, kMaxAcc = 8;
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kSet = 4;            // kSums, kParts: sums handed to the epilogue at a time (5 x 28672 x 8192 int4: 51.5 us with 2, 50.4 with 4)
+constexpr uint32_t kSet = 4;            // kSums, kParts: sums handed to the epilogue at a time (5 x 28672 x 8192 int4: 51.5 us with 2, 49.7 with 4)
 // kParts: k that one accumulator adds up before the sum goes on in fp32 registers.  The tensor cores cut off what an addition shifts out,
 // so a sum over all of K drifts: of 16 x 28672 x 8192 int8 results 15 in 10000 were not the correctly rounded ones (8 rows: 14), with
 // decode.cu, whose warps and CTAs each add a stretch of K, 10 (5), with sums over 1024 k 3 (3).

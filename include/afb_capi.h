@@ -44,8 +44,8 @@ extern "C" {
 #define AFB_SCALE_BF16 1u
 
 #define AFB_VARIANT_AUTO    0u /* decode for M <= 16, prefill above, naive where neither applies */
-#define AFB_VARIANT_DECODE  1u /* memory-bound small-M kernel                                   */
-#define AFB_VARIANT_PREFILL 2u /* TMA + tcgen05/TMEM kernel                                    */
+#define AFB_VARIANT_DECODE  1u /* memory-bound small-M kernels (decode.cu or, where faster, stream.cu) */
+#define AFB_VARIANT_PREFILL 2u /* TMA + tcgen05/TMEM kernels (prefill.cu, prefill_ts.cu or stream.cu)  */
 #define AFB_VARIANT_NAIVE   3u /* one thread per output element, fp32, order of host_ref.hpp:15-24 */
 
 #define AFB_FLAG_C_F32 1u /* C is fp32 [M,N] instead of bf16: prefill variant (partial sums of a K-split) and naive variant */
@@ -172,9 +172,9 @@ int afb_gemm_launch_static(const afb_gemm_args* args, void* stream);
  * (AFB_LAYOUT_ROW [K,N] int8, or AFB_LAYOUT_COL [N,K] int8 / int4) and writes the same integers as
  * AFB_LAYOUT_COL_PACKED into out_b: [N,K], pitch out_ldb elements, inside every 32-bit word the order
  *   int8: bytes [k0,k2,k1,k3]      int4: nibbles [k0,k2,k4,k6,k1,k3,k5,k7]
- * which is the order the kernels' unpack reads as pairs, so they skip the re-pairing of the activations (decode)
- * or of the weights (prefill).  A GEMM on the result sets b_layout = AFB_LAYOUT_COL_PACKED, ptr_b = out_b,
- * ldb = out_ldb; its result is bit-identical to the GEMM on the plain [N,K] weights.  [N,K] input may be packed
+ * which is the order the decode kernel's unpack reads as pairs, so that it skips the re-pairing of the activations
+ * (the other kernels' unpack takes either order at the same cost).  A GEMM on the result sets
+ * b_layout = AFB_LAYOUT_COL_PACKED, ptr_b = out_b, ldb = out_ldb; its result is bit-identical to the GEMM on the plain [N,K] weights.  [N,K] input may be packed
  * in place (out_b == ptr_b, out_ldb == ldb).  Asynchronous on `stream`. */
 int afb_prepack(const afb_gemm_args* args, void* out_b, uint32_t out_ldb, void* stream);
 /* ---- fused neighbours of the GEMM ------------------------------------------------ */
