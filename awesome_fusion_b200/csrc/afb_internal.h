@@ -79,7 +79,8 @@ const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* r
 bool stream_workspace(DeviceCtx* ctx, cudaStream_t s, size_t bytes, float** ws, uint32_t** counters);
 int  cuda_fail(cudaError_t e);      // records e, returns AFB_ERR_CUDA
 void count_launch(unsigned n = 1);
-void count_stream_launch();          // of the streaming form (counted by count_launch as well)
+void count_stream_launch();          // of the streaming form, or of the pair form in its place (counted by count_launch as well)
+void count_pair_launch();            // of the pair form (likewise)
 
 // Driver entry point for tensor-map encoding, fetched once through the runtime.
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -97,12 +98,15 @@ int launch_prefill(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s);     
 // (environment variable AFB_SUB_AR_SMS, default 16: on 2 GPUs 1.03 ms for the down-projection with 16, 1.13 with 8)
 uint32_t sub_allreduce_sms();
 int launch_prefill_ts(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, const afb_fused_args* fused = nullptr);   // converted weights in tensor memory
-// Row tiles per group of a persistent kernel's tile order (tiles of bma rows x 128 channels).
-uint32_t pick_group_m(const afb_gemm_args& a, uint32_t m_tiles, uint32_t n_tiles, uint32_t bma, int sms);
+// Row tiles per group of a persistent kernel's tile order (tiles of bma rows x `channels` channels, one per SM or pair of SMs).
+uint32_t pick_group_m(const afb_gemm_args& a, uint32_t m_tiles, uint32_t n_tiles, uint32_t bma, int sms, uint32_t channels = 128);
 // The streaming form of the decode and prefill variants (stream.cu), for a call that resolved to `variant`: launched where it takes the
 // arguments, is the faster one and no tuning variable asks for another (*done = true, its status returned); otherwise nothing happens
 // and the caller goes on to the other forms.
 int stream_if_faster(const afb_gemm_args& a, uint32_t variant, DeviceCtx* ctx, cudaStream_t s, bool* done);
+bool stream_is_faster(const afb_gemm_args& a, uint32_t sms);   // ... than the forms with one step for all converters; the pair form left aside
+// The pair form of the prefill variant (pair.cu), for a call that resolved to it or (`fused`) for a fused launch; otherwise as above.
+int pair_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, const afb_fused_args* fused, bool* done);
 int launch_prefill_ts_tiles(const afb_gemm_args& a, DeviceCtx* ctx, uint32_t* tile_done, cudaStream_t s);
 // The sum and broadcast of the pipelined reduce-scatter done inside the pushing GEMM, by two extra warps of every CTA (so that no
 // second kernel has to share SMs with the GEMM): where the finished rows go, the words of the closing signal round, the count

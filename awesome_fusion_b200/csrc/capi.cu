@@ -15,7 +15,7 @@ constexpr int kMaxDevices = 32;
 DeviceCtx g_ctx[kMaxDevices];
 std::mutex g_mutex;
 std::atomic<int> g_last_cuda_error{0};
-std::atomic<unsigned long long> g_launches{0}, g_stream_launches{0};
+std::atomic<unsigned long long> g_launches{0}, g_stream_launches{0}, g_pair_launches{0};
 constexpr size_t kSplitKWorkspaceBytes = 32u << 20;
 constexpr size_t kSplitKCounters = 4096;
 constexpr int kPreallocatedWorkspaces = 8;
@@ -35,6 +35,7 @@ int cuda_fail(cudaError_t e) {
 }
 void count_launch(unsigned n) { g_launches.fetch_add(n); }
 void count_stream_launch() { g_stream_launches.fetch_add(1); }
+void count_pair_launch() { g_pair_launches.fetch_add(1); }
 
 DeviceCtx* current_ctx() {
     int dev = -1;
@@ -122,6 +123,7 @@ bool stream_workspace(DeviceCtx* ctx, cudaStream_t s, size_t bytes, float** ws, 
     // a stream's own workspace serves all its launches to come, a graph's the one at hand and those no larger
     size_t want = (size_t)2 * ctx->sm_count * kMaxStreamRows * 128 * sizeof(float);
     if (capturing) for (want = kMinStreamWorkspace; want < bytes;) want *= 2;
+    else if (want < bytes) want = bytes;
     DeviceCtx::StreamWorkspace* spare = nullptr;   // smallest one with memory that is large enough
     DeviceCtx::StreamWorkspace* empty = nullptr;
     for (auto& w : ctx->stream_workspaces) {
@@ -277,7 +279,7 @@ int afb_init(int device) {
         AFB_CUDA(cudaMalloc(&c.workspaces[i].counters, kSplitKCounters * sizeof(uint32_t)));
         AFB_CUDA(cudaMemset(c.workspaces[i].counters, 0, kSplitKCounters * sizeof(uint32_t)));
     }
-    c.stream_counter_count = 2 * (size_t)c.sm_count;   // a launch shares fewer than two tiles per SM
+    c.stream_counter_count = 3 * (size_t)c.sm_count;   // a launch shares fewer than two tiles per SM, of pairs of SMs fewer than one and three words a rank
     AFB_CUDA(allocate_stream_workspace(&c, &c.stream_workspaces[0], (size_t)2 * c.sm_count * kMaxStreamRows * 128 * sizeof(float)));   // the first stream's
     AFB_CUDA(cudaStreamCreateWithFlags(&c.clear_stream, cudaStreamNonBlocking));
     AFB_CUDA(cudaMalloc(&c.phase_ts, 8 * sizeof(unsigned long long)));
@@ -392,6 +394,8 @@ int afb_gemm_launch(const afb_gemm_args* args, void* stream) {
         }
         case AFB_VARIANT_PREFILL: {
             bool done = false;
+            rc = pair_if_faster(*args, ctx, s, nullptr, &done);
+            if (done) return rc;
             rc = stream_if_faster(*args, v, ctx, s, &done);
             if (done) return rc;
             // two implementations of the prefill variant; a flag or AFB_PREFILL_IMPL=ss|ts overrides the default
@@ -438,7 +442,9 @@ int afb_gemm_fused_launch(const afb_fused_args* f, void* stream) {
     if (!prefill_supports(a)) return AFB_ERR_UNSUPPORTED;   // [N,K] layout (plain or pre-packed), K % 64 == 0, aligned pointers and pitches
     DeviceCtx* ctx = current_ctx();
     if (!ctx) return AFB_ERR_NOT_INIT;
-    return launch_prefill_ts(a, ctx, (cudaStream_t)stream, f);
+    bool done = false;
+    rc = pair_if_faster(a, ctx, (cudaStream_t)stream, f, &done);
+    return done ? rc : launch_prefill_ts(a, ctx, (cudaStream_t)stream, f);
 }
 
 static size_t b_bytes(const afb_gemm_args& a) {
@@ -631,6 +637,7 @@ int afb_last_cuda_error(void) { return g_last_cuda_error.load(); }
 const char* afb_last_cuda_error_string(void) { return cudaGetErrorString((cudaError_t)g_last_cuda_error.load()); }
 unsigned long long afb_launch_count(void) { return g_launches.load(); }
 unsigned long long afb_stream_launch_count(void) { return g_stream_launches.load(); }
+unsigned long long afb_pair_launch_count(void) { return g_pair_launches.load(); }
 const char* afb_version(void) { return "afb 0.1 (sm_100a)"; }
 
 }  // extern "C"

@@ -137,6 +137,21 @@ __device__ __forceinline__ GroupUnpack group_unpack(int bits, uint16_t s, int ze
     return u;
 }
 
+// The folded constants of one group from those of all groups: a scale that folds is 0 or a positive normal number, so its products with
+// powers of two are integer additions to the exponent fields (6 instructions instead of 30).
+struct GroupFold { uint32_t mul0, mul1, add; };
+__device__ __forceinline__ GroupFold group_fold(int bits, const Nibbles& q) {
+    const uint32_t m0 = bits == 8 ? kMulByte : q.mul[0], m1 = bits == 8 ? kMulByte : q.mul[1];
+    const uint32_t sixteenth = 0x3F803F80u + 0x02000200u;   // the multipliers divided by 16, less the exponent of 1
+    return {m0 - sixteenth, m1 - sixteenth, 0x80008000u - (bits == 8 ? 0x01800180u : 0x03800380u)};   // -2^-3, -2^-7
+}
+__device__ __forceinline__ void group_folded(const GroupFold& f, uint16_t s, GroupUnpack& u) {
+    const uint32_t two = bf16_dup(s);
+    u.mul0 = s ? two + f.mul0 : 0u;
+    u.mul1 = s ? two + f.mul1 : 0u;
+    u.add = s ? two + f.add : 0x80008000u;
+}
+
 // Place of weight k inside its word in the pre-packed layout (int8: bytes [k0,k2,k1,k3]; int4: nibbles [k0,k2,k4,k6,k1,k3,k5,k7]).
 __host__ __device__ __forceinline__ uint32_t packed_pos(uint32_t bits, uint32_t k) {
     if (bits == 8) { const uint32_t i = k & 3u; return (k & ~3u) | ((i >> 1) | ((i & 1u) << 1)); }

@@ -781,10 +781,10 @@ int ts_tmap_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint6
 
 }  // namespace
 
-// Row tiles per group of the tile order, from a simple model of the HBM traffic.  One wave of CTAs covers g row tiles and
+// Row tiles per group of the tile order, from a simple model of the HBM traffic.  One wave of CTAs (or pairs of them: `sms`) covers g row tiles and
 // about sms / g channel tiles and re-reads both from HBM, unless the activations of the group (g * BMA * K * 2 bytes) are
 // small enough to stay in L2 over the whole group, in which case they are read once per group.
-uint32_t pick_group_m(const afb_gemm_args& a, uint32_t m_tiles, uint32_t n_tiles, uint32_t bma, int sms) {
+uint32_t pick_group_m(const afb_gemm_args& a, uint32_t m_tiles, uint32_t n_tiles, uint32_t bma, int sms, uint32_t channels) {
     const double k = a.k, wbytes = a.b_bits / 8.0;
     const double tiles = (double)m_tiles * n_tiles;
     const double w_total = (double)a.n * k * wbytes, a_total = (double)a.m * k * 2.0;
@@ -800,7 +800,7 @@ uint32_t pick_group_m(const afb_gemm_args& a, uint32_t m_tiles, uint32_t n_tiles
             bytes = a_total + groups * w_total;                       // activations once, weights once per group
         } else {
             const double ng = (double)sms / g < 1.0 ? 1.0 : ((double)sms / g > n_tiles ? (double)n_tiles : (double)sms / g);
-            const double per_wave = a_slice + ng * BNW * k * wbytes;
+            const double per_wave = a_slice + ng * channels * k * wbytes;
             bytes = tiles / ((double)g * ng) * per_wave;
         }
         if (bytes < best) { best = bytes; best_g = g; }

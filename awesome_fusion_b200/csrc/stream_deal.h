@@ -22,6 +22,7 @@ struct StreamDeal {
     uint32_t whole_waves;    // the tiles after them, `grid` per wave
     uint32_t grid;           // CTAs
     uint32_t dealers;        // CTAs [0, dealers) hold units of shared tiles
+    uint32_t tiles;          // all of them
 
     bool fits() const { return ((uint64_t)shared_tiles * blocks * (dealers + 1)) >> 32 == 0; }
     AFB_DEAL uint32_t units() const { return shared_tiles * blocks; }
@@ -41,6 +42,9 @@ struct Piece { uint32_t t, kb0, kb1; };
 struct Walk {
     uint32_t u, u_end, it;
     AFB_DEAL void start(const StreamDeal& d, uint32_t cta) { u = d.begin(cta); u_end = d.begin(cta + 1); it = 0; }
+    AFB_DEAL bool more(const StreamDeal& d, uint32_t cta) const { return u < u_end || (it < d.whole_waves && d.shared_tiles + cta + it * d.grid < d.tiles); }
+    // SHORT: the last wave may be short (deal_whole)
+    template <bool SHORT = false>
     AFB_DEAL bool next(const StreamDeal& d, uint32_t cta, Piece& x) {
         if (u < u_end) {
             x.t = u / d.blocks; x.kb0 = u - x.t * d.blocks;
@@ -50,6 +54,7 @@ struct Walk {
         }
         if (it >= d.whole_waves) return false;
         x.t = d.shared_tiles + cta + it * d.grid; x.kb0 = 0; x.kb1 = d.blocks;
+        if (SHORT && x.t >= d.tiles) return false;
         ++it;
         return true;
     }
@@ -57,18 +62,30 @@ struct Walk {
 
 // Tiles that fill whole waves stay whole; a short rest is shared together with the last full wave, so that no CTA gets less than
 // a quarter of a tile of it.
-inline StreamDeal deal_tiles(uint32_t tiles, uint32_t blocks, uint32_t sms) {
+// `least`: of a tile, in quarters.
+inline StreamDeal deal_tiles(uint32_t tiles, uint32_t blocks, uint32_t sms, uint32_t least = 1) {
     StreamDeal d;
     d.blocks = blocks;
     d.grid = sms;
+    d.tiles = tiles;
     const uint32_t waves = tiles / sms, rest = tiles - waves * sms;
     if (rest == 0) { d.shared_tiles = 0; d.whole_waves = waves; }
     else if (waves == 0) { d.shared_tiles = tiles; d.whole_waves = 0; }
-    else if (rest * 4 >= sms) { d.shared_tiles = rest; d.whole_waves = waves; }
+    else if (rest * 4 >= least * sms) { d.shared_tiles = rest; d.whole_waves = waves; }
     else { d.shared_tiles = sms + rest; d.whole_waves = waves - 1; }
     const uint64_t units = (uint64_t)d.shared_tiles * blocks;
     d.dealers = units < sms ? (uint32_t)units : sms;
     if (d.whole_waves == 0) d.grid = d.dealers;
+    return d;
+}
+
+// All tiles whole; the last wave may be short.
+inline StreamDeal deal_whole(uint32_t tiles, uint32_t blocks, uint32_t sms) {
+    StreamDeal d;
+    d.blocks = blocks; d.tiles = tiles;
+    d.shared_tiles = d.dealers = 0;
+    d.grid = tiles < sms ? tiles : sms;
+    d.whole_waves = (tiles + sms - 1) / sms;
     return d;
 }
 

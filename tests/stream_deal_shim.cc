@@ -4,9 +4,8 @@
 
 // 0, or which rule is broken: 1 a unit not dealt exactly once, 2 a contributor missing between the first and the last CTA of a tile (it
 // would be waited for), 3 two partial sums in one place, 4 more than two shared tiles to finish in one CTA, 5 a CTA with nothing to do,
-// 6 a run that is longer than another by more than one unit, 7 refused as too large
-extern "C" int check_deal(uint32_t tiles, uint32_t blocks, uint32_t sms) {
-    const afb::StreamDeal d = afb::deal_tiles(tiles, blocks, sms);
+// 6 a run that is longer than another by more than one unit, 7 refused as too large, 8 more() says otherwise than next()
+static int check(const afb::StreamDeal& d, uint32_t tiles, uint32_t blocks) {
     if (!d.fits()) return 7;
     std::vector<uint8_t> seen((size_t)tiles * blocks, 0);
     std::vector<uint32_t> arrivals(d.shared_tiles, 0);
@@ -21,9 +20,12 @@ extern "C" int check_deal(uint32_t tiles, uint32_t blocks, uint32_t sms) {
             longest = run > longest ? run : longest;
         }
         afb::Piece x;
+        bool more = true;
         uint32_t pieces = 0, parts = 0;
-        while (w.next(d, c, x)) {
+        while (w.next<true>(d, c, x)) {
             ++pieces;
+            if (!more) return 8;
+            more = w.more(d, c);
             if (x.t >= tiles || x.kb0 >= x.kb1 || x.kb1 > blocks) return 1;
             for (uint32_t kb = x.kb0; kb < x.kb1; ++kb)
                 if (seen[(size_t)x.t * blocks + kb]++) return 1;
@@ -34,11 +36,21 @@ extern "C" int check_deal(uint32_t tiles, uint32_t blocks, uint32_t sms) {
             if (slots[d.slot(c, x.t)]++) return 3;
         }
         if (!pieces) return 5;
+        if (more) return 8;
     }
     for (uint8_t s : seen) if (!s) return 1;
     for (uint32_t t = 0; t < d.shared_tiles; ++t)
         if (arrivals[t] && arrivals[t] != d.last_cta(t) - d.first_cta(t) + 1) return 2;
     if (d.shared_tiles && longest - shortest > 1) return 6;
+    return 0;
+}
+extern "C" int check_deal(uint32_t tiles, uint32_t blocks, uint32_t sms) { return check(afb::deal_tiles(tiles, blocks, sms), tiles, blocks); }
+// as the pair form deals: whatever does not fill whole waves shared, or nothing
+extern "C" uint32_t check_pair_range(uint32_t tiles_end, uint32_t blocks_end, uint32_t pairs, uint32_t* where) {
+    for (uint32_t t = 1; t < tiles_end; ++t)
+        for (uint32_t b = 1; b < blocks_end; ++b)
+            for (int share = 0; share < 2; ++share)
+                if (const int rc = check(share ? afb::deal_tiles(t, b, pairs, 0) : afb::deal_whole(t, b, pairs), t, b)) { where[0] = t; where[1] = b; return (uint32_t)rc; }
     return 0;
 }
 extern "C" uint32_t check_range(uint32_t tiles_end, uint32_t blocks_end, uint32_t sms, uint32_t* where) {

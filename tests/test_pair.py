@@ -1,0 +1,233 @@
+"""The pair form of the prefill variant and of the fused launches (csrc/pair.cu), forced onto small problems, against the CPU oracle.
+
+The sizes are those at which it can go wrong: activation rows around its tile heights (steps of 32 up to 256, halves in two CTAs), one to
+four stretches of K added up at the end, K that leaves raw blocks and steps incomplete, an odd number of 128-channel halves, channels that
+end inside one, tiles shared by many pairs (alone and next to whole waves) or not at all, more tiles than pairs."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import afb_testlib as T
+import awesome_fusion_b200 as pkg
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def _check(afb, oracle, case, what, rows=None, **kw):
+    from test_gpu_parity import check_close
+    before = afb.pair_launch_count()
+    got, _ = T.run_case(afb, case, variant=pkg.VARIANT_PREFILL, **kw)
+    again, _ = T.run_case(afb, case, variant=pkg.VARIANT_PREFILL, **kw)
+    assert afb.pair_launch_count() - before == 2, f"{what}: another form took the call"
+    assert np.array_equal(got, again), f"{what}: two runs differ"
+    assert afb.read_status()[0] == 0
+    rows = list(range(case.m)) if rows is None else rows
+    check_close(oracle, oracle.gemm(case, threads=8, round_w=bool(case.group), rows=rows), np.ascontiguousarray(got[rows]), what)
+    return got
+
+
+@pytest.fixture
+def forced(monkeypatch):
+    monkeypatch.setenv("AFB_PAIR", "1")
+    return monkeypatch
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("share", ["0", "1"])
+@pytest.mark.parametrize("m", [1, 32, 33, 65, 129, 160, 225, 256, 257, 385])
+@pytest.mark.parametrize("bits,group,n,k", [(8, 0, 264, 64), (8, 0, 1000, 960), (8, 0, 128, 4096), (4, 0, 392, 320), (4, 128, 520, 1152), (4, 256, 264, 2304),
+                                            (4, 64, 136, 704), (8, 128, 264, 640), (8, 64, 264, 448)])
+def test_rows_and_ragged_k(afb, oracle, forced, m, bits, group, n, k, share):
+    forced.setenv("AFB_PAIR_SHARE", share)
+    case = T.make_case(m, n, k, bits=bits, group=group, enc=m & 1, seed=m + k, scale_range=(0.005, 0.05))
+    _check(afb, oracle, case, f"int{bits} g{group} {m}x{n}x{k} share {share}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("most", ["64", "96", "128", "192", "224", "256"])
+@pytest.mark.parametrize("share", ["0", "1"])
+@pytest.mark.parametrize("m,n,k,bits,group", [(300, 10120, 640, 8, 0), (700, 6152, 512, 8, 0), (500, 4104, 1280, 4, 128)])
+def test_tile_heights_whole_waves_and_shared_tiles(afb, oracle, forced, m, n, k, bits, group, share, most):
+    forced.setenv("AFB_PAIR_ROWS", most)
+    forced.setenv("AFB_PAIR_SHARE", share)
+    case = T.make_case(m, n, k, bits=bits, group=group, seed=5, scale_range=(0.005, 0.05))
+    _check(afb, oracle, case, f"int{bits} g{group} {m}x{n}x{k} rows {most} share {share}", rows=list(range(0, m, 7)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("share", ["0", "1"])
+@pytest.mark.parametrize("m", [40, 200])
+@pytest.mark.parametrize("bits,group", [(8, 0), (8, 128), (4, 0), (4, 128), (4, 64)])
+def test_zero_points_and_packed_layout(afb, oracle, forced, m, bits, group, share):
+    forced.setenv("AFB_PAIR_SHARE", share)
+    case = T.make_case(m, 520, 1280, bits=bits, group=group, enc=1, seed=m + bits, zero_points=True, scale_range=(0.005, 0.05))
+    got = _check(afb, oracle, case, f"zero-points int{bits} g{group} m{m}")
+    assert np.array_equal(got, _check(afb, oracle, oracle.prepack(case), f"packed, zero-points int{bits} g{group} m{m}"))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scales", [[0.0, 0.03], [2.0 ** -110, 0.02], [17.0, 0.5], [-0.04, 0.04], [2.0 ** -99, 15.9]])
+def test_group_scales_at_the_edges_of_the_folding(afb, oracle, forced, scales):
+    """Scales that fold into the unpack next to ones that do not, in one warp: 0, below 2^-100, from 16 on, negative."""
+    case = T.make_case(70, 264, 1024, bits=4, group=128, seed=9, scale_range=(0.01, 0.02))
+    s = T.np_bf16_to_f32(case.scale)
+    s[:, ::3], s[:, 1::3] = scales[0], scales[1]
+    case.scale = T.np_bf16_rne(s)
+    _check(afb, oracle, case, f"scales {scales}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("share", ["0", "1"])
+@pytest.mark.parametrize("m,n,k,gated", [(1, 72, 512, True), (33, 136, 256, True), (257, 264, 1024, True), (300, 2056, 640, True), (70, 264, 320, False), (300, 4104, 512, False)])
+def test_fused_epilogue(afb, oracle, forced, m, n, k, gated, share):
+    """Bias, SiLU, gate * up and the residual, in place and with padded rows, in whole and in shared tiles."""
+    from test_fused import silu
+    from test_gpu_parity import check_close
+    forced.setenv("AFB_PAIR_SHARE", share)
+    rows = 2 * n if gated else n
+    case = T.make_case(m, rows, k, seed=m + n, scale_range=(0.002, 0.01))
+    rng = np.random.default_rng(11)
+    bias = rng.standard_normal(rows).astype(np.float32)
+    v = oracle.gemm(case, threads=8) + bias[None, :]
+    ldc = n + 24
+    before = T.np_bf16_rne(rng.standard_normal((m, ldc), dtype=np.float32))
+    want = (silu(v[:, 0::2]) * v[:, 1::2] if gated else silu(v)) + T.np_bf16_to_f32(before[:, :n])
+    held = [afb.to_device(x) for x in (case.a, case.b, case.scale, bias, before)]
+    d_a, d_b, d_s, d_bias, d_c = held
+    try:
+        count = afb.pair_launch_count()
+        args = afb.make_args(d_c, d_a, d_b, d_s, m, rows, k, ldc=ldc)
+        afb.gemm_fused_launch(afb.make_fused_args(args, gated=gated, activation=pkg.ACT_SILU, bias=d_bias, residual=d_c, ld_residual=ldc))
+        afb.device_sync()
+        got = afb.to_host(d_c, (m, ldc), np.uint16)
+        assert afb.pair_launch_count() == count + 1 and afb.read_status()[0] == 0
+    finally:
+        for p in held:
+            afb.free(p)
+    check_close(oracle, want, np.ascontiguousarray(got[:, :n]), f"fused gated={gated} {m}x{n}x{k}")
+    assert np.array_equal(got[:, n:], before[:, n:])
+
+
+@pytest.mark.gpu
+def test_silu_over_its_range(afb, forced):
+    """act(v) * 1 of values from -120 to 120, +-0, infinities and NaN against 64 bits.
+    (v below -88.7, where 1 + exp(-v) overflows fp32, gives -0.)"""
+    k, m = 64, 64
+    v = np.concatenate([np.linspace(-120, 120, 4073), [0.0, -0.0, np.inf, -np.inf, np.nan, 1e-30, -1e-30, 88.72, -88.72, -87.0, 1e30, -1e30]])
+    v = T.np_bf16_to_f32(T.np_bf16_rne(np.resize(v, 64 * 64).astype(np.float32))).reshape(64, 64)
+    a = np.zeros((m, k), np.float32)
+    a[:, :] = v                                   # a[i, j] = v[i, j]; channel 2j of B picks k = j, channel 2j + 1 nothing: up = bias = 1
+    q = np.zeros((2 * 64, k), np.int8)
+    q[2 * np.arange(64), np.arange(64)] = 1
+    finite = np.isfinite(v)
+    a[~finite] = 0.0
+    bias = np.zeros(128, np.float32)
+    bias[1::2] = 1.0
+    # infinities and NaN come in through the bias, one at a time, over a row of zeros
+    held = [afb.to_device(x) for x in (T.np_bf16_rne(a), q.view(np.uint8), np.ones(128, np.float32), bias)]
+    d_c = afb.malloc(m * 64 * 2)
+    try:
+        args = afb.make_args(d_c, held[0], held[1], held[2], m, 128, k, ldc=64)
+        afb.gemm_fused_launch(afb.make_fused_args(args, gated=True, activation=pkg.ACT_SILU, bias=held[3])); afb.device_sync()
+        got = T.np_bf16_to_f32(afb.to_host(d_c, (m, 64), np.uint16))
+        x = a.astype(np.float64)
+        want = np.where(x < -88.7, 0.0, x / (1 + np.exp(-np.maximum(x, -700.0))))
+        # 2^-22 from ex2.approx, 2^-23 from rcp.approx, four roundings of 2^-24: below 2^-20 of the value, next to half a unit of bf16, 2^-8
+        bad = np.abs(got - want) > np.abs(want) * (2.0 ** -8 + 2.0 ** -20) + 2.0 ** -126
+        assert not bad.any(), [(float(p), float(q), float(r)) for p, q, r in zip(x[bad], got[bad], want[bad])][:8]
+        for special, result in ((np.inf, np.inf), (-np.inf, np.nan), (np.nan, np.nan)):
+            bias[0::2] = special
+            b = afb.to_device(bias)
+            afb.gemm_fused_launch(afb.make_fused_args(args, gated=True, activation=pkg.ACT_SILU, bias=b)); afb.device_sync()
+            out = T.np_bf16_to_f32(afb.to_host(d_c, (m, 64), np.uint16))
+            afb.free(b)
+            assert np.all(np.isnan(out)) if np.isnan(result) else np.all(out == result), special
+    finally:
+        for p in held + [d_c]:
+            afb.free(p)
+
+
+@pytest.mark.gpu
+def test_shared_tiles_in_captured_graphs_and_on_streams(afb, oracle, forced):
+    """A shared launch per stream and per captured graph: workspaces of their own, counters back at zero for the next replay."""
+    import torch
+    from test_gpu_parity import check_close
+    forced.setenv("AFB_PAIR_SHARE", "1")
+    case = T.make_case(150, 1032, 1024, bits=4, group=128, seed=3, scale_range=(0.005, 0.05))
+    want = oracle.gemm(case, threads=8, round_w=True)
+    dcs = [T.DeviceCase(afb, case) for _ in range(3)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    try:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=streams[0]):
+            afb.gemm_launch(dcs[0].args(variant=pkg.VARIANT_PREFILL), torch.cuda.current_stream().cuda_stream)
+        for _ in range(3):
+            graph.replay()
+            for dc, s in zip(dcs[1:], streams):
+                afb.gemm_launch(dc.args(variant=pkg.VARIANT_PREFILL), s.cuda_stream)
+        torch.cuda.synchronize()
+        for dc in dcs:
+            check_close(oracle, want, dc.result()[0], "captured and on streams")
+    finally:
+        for dc in dcs:
+            dc.close()
+
+
+@pytest.mark.gpu
+def test_variables_and_flags_that_ask_for_another_form(afb, monkeypatch):
+    case = T.make_case(256, 8192, 1024, bits=4, group=128, seed=1)
+
+    def paired(**kw):
+        before = afb.pair_launch_count()
+        T.run_case(afb, case, **kw)
+        return afb.pair_launch_count() - before
+    assert paired() == 1 and paired(variant=pkg.VARIANT_PREFILL) == 1
+    for flags in (pkg.FLAG_PREFILL_TMEM_A, pkg.FLAG_PREFILL_SMEM_B, pkg.FLAG_GROUP_EXACT):
+        assert paired(flags=flags) == 0, flags
+    assert paired(c_f32=True) == 0
+    for name, value in (("AFB_PAIR", "0"), ("AFB_STREAM", "0"), ("AFB_STREAM", "1"), ("AFB_PREFILL_TILE_STORE", "0"), ("AFB_PREFILL_SPLIT_TAIL", "0")):
+        monkeypatch.setenv(name, value)
+        assert paired() == 0, name
+        monkeypatch.delenv(name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(512, 2048, 4096), (256, 8192, 8192), (120, 11008, 4096)])
+def test_stretches_of_k_do_not_drift(afb, monkeypatch, m, n, k):
+    """One tile per pair: K is added up in two (up to 128 rows per tile) or four (up to 64) accumulators, where the other forms cut it, too.
+    The tensor cores cut off what an addition shifts out, so sums of one sign come out low, the more the longer one accumulator adds: by
+    no more than in the other forms (the rounding to bf16 has a mean of zero: 2^-9 / sqrt(12) over the root of 10^6 results, 6e-7)."""
+    case = T.make_case(m, n, k, seed=m)
+    a, q = np.abs(T.np_bf16_to_f32(case.a)), np.abs(case.q)
+    case.a, case.b = T.np_bf16_rne(a), q.view(np.uint8)
+    exact = (a @ q.T.astype(np.float32)).astype(np.float64) if n * k > 3e7 else a.astype(np.float64) @ q.T.astype(np.float64)
+    exact *= case.scale.astype(np.float64)
+    off = []
+    for pair in ("1", "0"):
+        monkeypatch.setenv("AFB_PAIR", pair)
+        before = afb.pair_launch_count()
+        got, _ = T.run_case(afb, case, variant=pkg.VARIANT_PREFILL)
+        assert afb.pair_launch_count() - before == int(pair)
+        off.append(abs(((T.np_bf16_to_f32(got) - exact) / exact).mean()))
+    assert off[0] < off[1] + 6e-7, off
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("deal") / "libdeal.so")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I" + os.path.join(ROOT, "awesome_fusion_b200", "csrc"),
+                           "-o", out, os.path.join(ROOT, "tests", "stream_deal_shim.cc")])
+    lib = ctypes.CDLL(out)
+    lib.check_pair_range.argtypes = [ctypes.c_uint32] * 3 + [ctypes.POINTER(ctypes.c_uint32)]
+    return lib
+
+
+@pytest.mark.parametrize("pairs,tiles,blocks", [(74, 460, 17), (66, 210, 9), (3, 40, 12)])
+def test_dealing_over_pairs(shim, pairs, tiles, blocks):
+    """The tiles that do not fill whole waves shared, however few, and all tiles whole with a short last wave."""
+    where = (ctypes.c_uint32 * 2)()
+    rc = shim.check_pair_range(tiles, blocks, pairs, where)
+    assert rc == 0, f"rule {rc} broken at {where[0]} tiles of {where[1]} blocks on {pairs} pairs"
