@@ -47,7 +47,7 @@ constexpr uint32_t kSet = 4;            // kSums, kParts: sums handed to the epi
 // so a sum over all of K drifts: of 16 x 28672 x 8192 int8 results 15 in 10000 were not the correctly rounded ones (8 rows: 14), with
 // decode.cu, whose warps and CTAs each add a stretch of K, 10 (5), with sums over 1024 k 3 (3).
 constexpr uint32_t kPartSum = 1024;
-constexpr int kBars = 2 * (kMaxRaw + kMaxSlots + kMaxAcc) + kMaxSlots + 3;
+constexpr int kBars = 2 * (kMaxRaw + 2 * kMaxSlots + kMaxAcc) + kMaxSlots + 3;
 constexpr int kOffMisc = kBars * 8, kOffOut = 1024;
 constexpr int kOutBytes = 16 * 32 * 2;                    // one block of the result: 16 rows x 32 channels
 constexpr int kOffRaw = kOffOut + 4 * 2 * kOutBytes;      // two blocks per epilogue warp
@@ -104,15 +104,22 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
     auto bar = [&](uint32_t i) { return smem_base + 8u * i; };
     auto raw_full = [&](uint32_t s) { return bar(s); };
     auto raw_empty = [&](uint32_t s) { return bar(kMaxRaw + s); };
-    auto step_full = [&](uint32_t s) { return bar(2 * kMaxRaw + s); };                // converted weights in TMEM, activations in shared memory
-    auto step_empty = [&](uint32_t s) { return bar(2 * kMaxRaw + kMaxSlots + s); };   // the MMAs of the step are done with both
+    // Up to 16 rows a step's two parts are issued by two warps, each into sums of its own (`h`: which part): one warp, next to busy
+    // converters on its scheduler, needs 46 cycles per tcgen05.mma and 450 besides per step, the tensor cores 9 for 16 rows (5 x 28672 x
+    // 8192 int4 group-128: 1500 cycles per step of 256 k with one).
+    // A free slot then tells a converter group about one part of a step only, so the raw block that had its place in the raw ring before
+    // must have been this group's own: the ring is a multiple of the groups' turn, and a step takes the places of two int8 blocks even if
+    // it lacks the second (kPadded).
+    constexpr bool kDual = summed(MODE) && PAIR == 2, kPadded = kDual && SPB == 1;
+    auto step_full = [&](uint32_t s, uint32_t h = 0) { return bar(2 * kMaxRaw + h * kMaxSlots + s); };          // converted weights in TMEM, activations in shared memory
+    auto step_empty = [&](uint32_t s, uint32_t h = 0) { return bar(2 * kMaxRaw + (2 + h) * kMaxSlots + s); };   // the MMAs of the step are done with both
     // The arrival of a step's activations.  Where a step is two parts (few rows) a converter warp waits for it before it reports its part,
     // so that the issuing warp, whose own instructions set the pace there, has one thing to wait for that is usually complete (28672 x
     // 8192, 1 row: 43.3 -> 41.9 us int8); with more rows it counts into step_full (39 against 38 us on 333 x 11008 x 4096 otherwise).
     constexpr bool kActApart = PAIR == 2;
-    auto act_full = [&](uint32_t s) { return kActApart ? bar(2 * (kMaxRaw + kMaxSlots + kMaxAcc) + s) : step_full(s); };
-    auto acc_full = [&](uint32_t s) { return bar(2 * (kMaxRaw + kMaxSlots) + s); };
-    auto acc_empty = [&](uint32_t s) { return bar(2 * (kMaxRaw + kMaxSlots) + kMaxAcc + s); };
+    auto act_full = [&](uint32_t s) { return kActApart ? bar(2 * (kMaxRaw + 2 * kMaxSlots + kMaxAcc) + s) : step_full(s); };
+    auto acc_full = [&](uint32_t s) { return bar(2 * (kMaxRaw + 2 * kMaxSlots) + s); };
+    auto acc_empty = [&](uint32_t s) { return bar(2 * (kMaxRaw + 2 * kMaxSlots) + kMaxAcc + s); };
     // a shared tile: every epilogue warp has published its part; the count has been taken.  The end: the epilogue is through
     const uint32_t bar_stored = bar(kBars - 3), bar_verdict = bar(kBars - 2), bar_finish = bar(kBars - 1);
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + kOffMisc);   // TMEM base, abort flag, "arrived last", tiles to finish, their number
@@ -133,8 +140,9 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
     } else {
         if (warp == 1 && lane == 0) {
-            for (uint32_t s = 0; s < p.slots; ++s) { ptx::mbar_init(step_full(s), kActApart ? 4 * PAIR : 4 * PAIR + 1); ptx::mbar_init(step_empty(s), 1); if (kActApart) ptx::mbar_init(act_full(s), 1); }
-            for (uint32_t s = 0; s < p.accs; ++s) { ptx::mbar_init(acc_full(s), 1); ptx::mbar_init(acc_empty(s), 4); }
+            for (uint32_t s = 0; s < p.slots; ++s) { ptx::mbar_init(step_full(s), kDual ? 4 : kActApart ? 4 * PAIR : 4 * PAIR + 1); ptx::mbar_init(step_empty(s), 1); if (kActApart) ptx::mbar_init(act_full(s), 1); }
+            for (uint32_t s = 0; kDual && s < p.slots; ++s) { ptx::mbar_init(step_full(s, 1), 4); ptx::mbar_init(step_empty(s, 1), 1); }
+            for (uint32_t s = 0; s < p.accs; ++s) { ptx::mbar_init(acc_full(s), kDual ? 2 : 1); ptx::mbar_init(acc_empty(s), 4); }
             ptx::mbar_init(bar_stored, 4);
             ptx::mbar_init(bar_verdict, 1);
             ptx::mbar_init(bar_finish, 4);
@@ -238,6 +246,12 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                 issued |= 1u << r.i; parity = (parity & ~(1u << r.i)) | (r.phase << r.i);
                 r.step(1, p.raw_stages);
             }
+            if (kPadded && ok && ((x.kb1 - x.kb0) & 1u)) {
+                if (!warp_wait(raw_empty(r.i), r.phase ^ 1u, abort_flag)) { give_up(31, x.t, x.kb1); break; }
+                if (ptx::elect_one()) ptx::mbar_arrive(raw_full(r.i));
+                issued |= 1u << r.i; parity = (parity & ~(1u << r.i)) | (r.phase << r.i);
+                r.step(1, p.raw_stages);
+            }
         }
         for (uint32_t s = 0; s < p.raw_stages; ++s)   // never leave with a bulk copy still writing this CTA's shared memory
             if (issued & (1u << s)) ptx::mbar_wait(raw_full(s), (parity >> s) & 1u);
@@ -252,7 +266,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
             tile_origin(p, x.t, m0, n0);
             const uint32_t k0 = x.kb0 * SPB, ns = parts_of(x);
             for (uint32_t l = 0; l < ns; l += PAIR) {
-                if (!warp_wait(step_empty(r.i), r.phase ^ 1u, abort_flag)) { give_up(32, x.t, l); ok = false; break; }
+                if (!warp_wait(step_empty(r.i), r.phase ^ 1u, abort_flag) || (kDual && !warp_wait(step_empty(r.i, 1), r.phase ^ 1u, abort_flag))) { give_up(32, x.t, l); ok = false; break; }
                 if (ptx::elect_one()) {
                     ptx::mbar_arrive_expect_tx(act_full(r.i), l + PAIR <= ns ? act_bytes : part_bytes);
 #pragma unroll
@@ -266,6 +280,39 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
         }
         for (uint32_t s = 0; s < p.slots; ++s)
             if (issued & (1u << s)) ptx::mbar_wait(act_full(s), (parity >> s) & 1u);   // after an abort the converters' part may be missing: then the limit of the wait, far above the time of a copy
+    } else if (kDual && warp < kFirstEpi) {
+        // ======================= MMA issuers, one for each part of a step =======================
+        const uint32_t h = (uint32_t)warp - 2, idesc = ptx::umma_idesc_bf16_f32(kCh, p.rows);
+        const uint64_t desc0 = ptx::umma_desc_kmajor_sw128(smem_base + off_act) + h * (part_bytes >> 4);
+        const uint32_t slab_d = slab_bytes >> 4, act_d = act_bytes >> 4;   // in units of the descriptor's address field
+        Ring rs{0, 0}, rc{0, 0};
+        bool ok = true, ready = false;
+        while (ok && walk.next(p.deal, blockIdx.x, x)) {
+            const uint32_t ns = parts_of(x);
+            uint32_t in_sum = 0, sum = h;   // parts in this warp's current sum; which of the accumulator's sums (this warp's are h and h + 2)
+            for (uint32_t l = 0; l < ns; l += 2) {
+                if (in_sum == 0 && sum == h && !warp_wait(acc_empty(rc.i), rc.phase ^ 1u, abort_flag)) { give_up(33, x.t, l); ok = false; break; }
+                if (!__all_sync(0xffffffffu, ready) && !warp_wait(step_full(rs.i, h), rs.phase, abort_flag)) { give_up(34, x.t, l); ok = false; break; }
+                ptx::tc_fence_after_sync();
+                const uint64_t db = desc0 + rs.i * act_d;
+                const uint32_t ta = slot_base + rs.i * kSlotCols + h * kPartCols, td = tmem_base + rc.i * p.acc_cols + sum * 16, done = step_empty(rs.i, h), acc_done = acc_full(rc.i);
+                rs.step(1, p.slots);
+                ready = ptx::mbar_test_wait(step_full(rs.i, h), rs.phase);   // of the next step: the answer is back when this one has been issued
+                const bool there = l + h < ns, first = in_sum == 0;   // the last step of a piece may lack its second part
+                if (++in_sum == p.flush) { in_sum = 0; sum += 2; }
+                const bool last = l + 2 >= ns || sum >= kSet;
+                if (ptx::elect_one()) {
+                    if (there) {
+#pragma unroll
+                        for (int j = 0; j < KS / 16; ++j)
+                            ptx::umma_bf16_ts(td, ta + 8 * j, db + (uint32_t)(j / 4) * slab_d + 2u * (j % 4), idesc, !first || j > 0 ? 1u : 0u);
+                    }
+                    ptx::umma_commit(done);
+                    if (last) ptx::umma_commit(acc_done);
+                }
+                if (last) { rc.step(1, p.accs); in_sum = 0; sum = h; }
+            }
+        }
     } else if (warp == 2) {
         // ======================= MMA issuer =======================
         const uint32_t idesc = ptx::umma_idesc_bf16_f32(kCh, p.rows);
@@ -333,7 +380,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
             if (channel_scaled(MODE) && has_zero) up.add = unpack_add(BITS, zero_of(nn < p.n ? p.zero[nn] : 0u));
             uint32_t l = (g - steps_before * PAIR) & (kGroups - 1);
             Ring rr, rs;
-            rr.set(blocks_before + l / SPB, p.raw_stages);
+            rr.set((kPadded ? 2 * steps_before : blocks_before) + l / SPB, p.raw_stages);
             rs.set(steps_before + l / PAIR, p.slots);
             load_group(l, sc_nxt, zb_nxt);
             const uint32_t nv = (ns + PAIR - 1) / PAIR * PAIR;
@@ -341,13 +388,18 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                 if (PAIR > 1 && l == ns) {
                     // The part that the last step of this piece lacks: waited for and reported like the others.  A group that passed
                     // over it would next look at a slot two uses later, where the parity of the barrier no longer tells it anything.
-                    if (!warp_wait(step_empty(rs.i), rs.phase ^ 1u, abort_flag)) { give_up(36, x.t, l); ok = false; break; }
-                    if (lane == 0) ptx::mbar_arrive(step_full(rs.i));
+                    if (!warp_wait(step_empty(rs.i, kDual), rs.phase ^ 1u, abort_flag)) { give_up(36, x.t, l); ok = false; break; }
+                    if (kPadded && !warp_wait(raw_full(rr.i), rr.phase, abort_flag)) { give_up(35, x.t, l); ok = false; break; }
+                    // (with two issuing warps also for its activations: or their loader could find this barrier a phase ahead)
+                    if (kDual && quarter == 0 && !warp_wait(act_full(rs.i), rs.phase, abort_flag)) { give_up(39, x.t, l); ok = false; break; }
+                    if (lane == 0) ptx::mbar_arrive(step_full(rs.i, kDual));
+                    if (kPadded && lane == 0) ptx::mbar_arrive(raw_empty(rr.i));
                     continue;
                 }
+                const uint32_t which = kDual ? g & 1u : 0u;   // a group's parts are all first or all second ones
                 const uint32_t sub = l % SPB, left = ns - (l - sub);   // `left`: parts of this block and all after it
                 if (!channel_scaled(MODE)) { sc = sc_nxt; zb = zb_nxt; load_group(l + kGroups, sc_nxt, zb_nxt); }
-                if (p.slot_first && !warp_wait(step_empty(rs.i), rs.phase ^ 1u, abort_flag)) { give_up(36, x.t, l); ok = false; break; }
+                if (p.slot_first && !warp_wait(step_empty(rs.i, which), rs.phase ^ 1u, abort_flag)) { give_up(36, x.t, l); ok = false; break; }
                 if (!warp_wait(raw_full(rr.i), rr.phase, abort_flag)) { give_up(35, x.t, l); ok = false; break; }
                 const uint8_t* raw = smem_gen + kOffRaw + rr.i * kRawBytes + ch * 128;
                 constexpr int kWords = BITS == 8 ? 16 : 8;   // of 64 weights
@@ -381,7 +433,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                         for (int j = 0; j < 32; ++j) o[j] = bf16x2_mul(o[j], up.scale);
                     }
                     if (h == 0) {
-                        if (!p.slot_first && !warp_wait(step_empty(rs.i), rs.phase ^ 1u, abort_flag)) { give_up(36, x.t, l); ok = false; break; }
+                        if (!p.slot_first && !warp_wait(step_empty(rs.i, which), rs.phase ^ 1u, abort_flag)) { give_up(36, x.t, l); ok = false; break; }
                         ptx::tc_fence_after_sync();
                     }
                     ptx::tmem_st_32x32(slot_base + ((quarter * 32u) << 16) + rs.i * kSlotCols + (l % PAIR) * kPartCols + h * 32, o);
@@ -392,7 +444,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                 ptx::tc_fence_before_sync();
                 __syncwarp();   // every lane's weights are in tensor memory
                 if (lane == 0) {
-                    ptx::mbar_arrive(step_full(rs.i));
+                    ptx::mbar_arrive(step_full(rs.i, which));
                     ptx::mbar_arrive_count(raw_empty(rr.i), left < SPB && sub + 1 == left ? 1 + SPB - left : 1u);   // a short last block: for its missing parts, too
                 }
                 rr.step(kGroups / SPB, p.raw_stages);   // four parts on
@@ -467,18 +519,20 @@ stream_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constan
                     return p.scale_dtype == AFB_SCALE_BF16 ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(p.scale)[i] << 16)
                                                            : reinterpret_cast<const float*>(p.scale)[i];
                 };
+                // the part that sum i of a set begins with: with two issuing warps 0 and 1, and the next two 2 * flush parts on
+                auto begins = [&](uint32_t i) { return kDual ? (i >> 1) * 2 * p.flush + (i & 1u) : i * p.flush; };
                 float sc[kSet];
 #pragma unroll
-                for (uint32_t i = 0; i < kSet; ++i) sc[i] = group_scale(i * p.flush);
+                for (uint32_t i = 0; i < kSet; ++i) sc[i] = group_scale(begins(i));
                 for (uint32_t l = 0; l < ns; l += kSet * p.flush) {
                     float sc_nxt[kSet];
 #pragma unroll
-                    for (uint32_t i = 0; i < kSet; ++i) sc_nxt[i] = group_scale(l + (kSet + i) * p.flush);
+                    for (uint32_t i = 0; i < kSet; ++i) sc_nxt[i] = group_scale(l + kSet * p.flush + begins(i));
                     if (!warp_wait(acc_full(rc.i), rc.phase, abort_flag)) { give_up(37, x.t, l); ok = false; break; }
                     ptx::tc_fence_after_sync();
 #pragma unroll
                     for (uint32_t i = 0; i < kSet; ++i) {
-                        if (l + i * p.flush >= ns) break;
+                        if (l + begins(i) >= ns) break;
 #pragma unroll
                         for (int h = 0; h < 16; h += 8) {
                             uint32_t r[8];
@@ -722,10 +776,11 @@ int stream_if_faster(const afb_gemm_args& a, uint32_t variant, DeviceCtx* ctx, c
     const uint32_t spb = (a.b_bits == 8 ? 128 : 256) / ks;
     p.parts = a.k / ks;
     while (a.group_size && ks << p.group_shift < a.group_size) ++p.group_shift;
-    p.flush = mode == kParts ? kPartSum / ks : mode == kSums ? (1u << p.group_shift < spb ? 1u << p.group_shift : spb) : 0;
+    const uint32_t pair = ks == 128 && p.rows <= 64 ? 2 : 1;
+    const bool dual = pair == 2 && summed(mode);   // parts per sum are then those of one issuing warp, and two parts are never in one group's sum
+    p.flush = mode == kParts ? kPartSum / ks : mode == kSums ? (dual ? 1 : 1u << p.group_shift < spb ? 1u << p.group_shift : spb) : 0;
     p.acc_cols = summed(mode) ? kSet * 16 : p.rows;
     p.accs = p.rows <= 192 ? 2 : 1;
-    const uint32_t pair = ks == 128 && p.rows <= 64 ? 2 : 1;
     p.slots = (kTmemCols - p.accs * p.acc_cols) / (pair * ks / 2);
     if (p.slots > (uint32_t)kMaxSlots) p.slots = kMaxSlots;
     const uint32_t act_bytes = p.rows * ks * 2 * pair;
@@ -733,6 +788,8 @@ int stream_if_faster(const afb_gemm_args& a, uint32_t variant, DeviceCtx* ctx, c
     p.raw_stages = (kRingBudget - p.slots * act_bytes) / kRawBytes;
     if (p.raw_stages > (uint32_t)kMaxRaw) p.raw_stages = kMaxRaw;
 
+    if (dual)   // see kDual in the kernel
+        p.raw_stages -= p.raw_stages % (kGroups / spb);
     // A converter warp sees only every fourth part, and a wait for phase n of a raw stage means something only once phase n - 1 has
     // completed.  What tells it that is the MMA order: a free slot means that everything up to `slots` steps earlier has been
     // consumed.  With the slot wait of the PREVIOUS part behind it, up to 3 + slots * pair earlier parts may still be under way,
