@@ -7,8 +7,8 @@
 //
 //   warp 0                TMA: raw weight blocks, 128 channels x 128 bytes (128 k of int8, 256 k of int4), 128-byte swizzle
 //   warp 1                TMA: activation slabs [rows x 64] bf16, 128-byte swizzle
-//   warp 2                tcgen05.mma 128 x rows x 16, weights from TMEM, activations from shared memory
-//                         (warps 0 to 2 run as whole warps and elect a lane for the asynchronous instructions)
+//   warp 2 (and 3)        tcgen05.mma 128 x rows x 16, weights from TMEM, activations from shared memory; up to 16 rows two warps, one for
+//                         each part of a step (warps 0 to 3 run as whole warps and elect a lane for the asynchronous instructions)
 //   warps 4-7             epilogue, one lane quarter each: accumulator -> scale -> bf16 -> C, or fp32 partial sums -> workspace
 //   warps 8-23            converters: four groups of four warps (one per lane quarter); group g takes every fourth part of k,
 //                         64 or 128 wide, so that four parts are being unpacked at any time.  A warp's chain wait -> load ->
@@ -24,9 +24,9 @@
 // epilogue warps, while the next groups are being computed (per-channel sums are handed over every 1024 k); above that they are folded
 // into the bf16 weights.
 //
-// What bounds it: for few rows int8 the weight stream (28672 x 8192, 16 rows: 44.7 us = 5.3 TB/s of weights, 63.8 with decode.cu; the
-// stream, the hand-offs and the shared tiles alone, without unpack and MMAs, take 44.7 too), int4 the issue slots of the unpack and of
-// the hand-offs (50 against 63 us with decode.cu; 40 without unpack and MMAs); for 65 to 128 rows the activations through L2 (28672 x 8192 int4
+// What bounds it: for few rows int8 the weight stream (28672 x 8192, 16 rows: 44.7 us = 5.3 TB/s of weights, 63.8 with decode.cu), int4
+// the converters, which take 2400 cycles for a part of 128 k next to each other, and the issuing warps (5 rows with zero-points, caches cold: 53.6 us
+// with one issuing warp, 49.2 with two; 16 rows int8 47.0 and 45.9); for 65 to 128 rows the activations through L2 (28672 x 8192 int4
 // group-128, 128 rows: 66 us, 82 with prefill.cu); for many rows the pace of the issuing warp next to the unpack.
 #include <cstdlib>
 #include "afb_internal.h"
@@ -683,7 +683,7 @@ uint32_t tile_rows(const afb_gemm_args& a) {
     return ((a.m + tiles - 1) / tiles + 15) / 16 * 16;
 }
 
-// Where this form is the faster one, from times of both forms on one B200 (us, the other form / this one): 23 matrices from 1024 x 1024
+// Where this form is the faster one (of the forms with one SM per tile: pair.cu is asked before), from times of both forms on one B200 (us, the other form / this one): 23 matrices from 1024 x 1024
 // to 28672 x 8192, 35 row counts from 4 to 4096, int8, int4, int4 in groups of 128 and 64, int8 in groups of 128.  At none of those that it takes is this form more than 4 %
 // the slower one.
 bool is_faster(const afb_gemm_args& a, uint32_t sms) {

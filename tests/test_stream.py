@@ -44,6 +44,16 @@ def test_whole_waves_and_shared_tiles(afb, oracle, m, n, k, bits, group):
     _check(afb, oracle, case, f"int{bits} g{group} {m}x{n}x{k}")
 
 
+@pytest.mark.parametrize("m", [1, 16])
+@pytest.mark.parametrize("bits,group,n,k", [(8, 0, 264, 128), (8, 0, 264, 640), (8, 0, 20008, 1152), (8, 128, 19000, 384), (8, 256, 520, 2816), (4, 0, 392, 640), (4, 0, 300, 8320),
+                                            (4, 128, 19000, 640), (4, 512, 264, 2560)])
+def test_two_issuing_warps(afb, oracle, m, bits, group, n, k):
+    """Up to 16 rows the two parts of a step (128 k each) are issued by two warps: steps that lack the second part, in tiles and in the shares of
+    tiles, sums of several parts and sets of sums that are not full."""
+    case = T.make_case(m, n, k, bits=bits, group=group, enc=m & 1, seed=m + k, scale_range=(0.005, 0.05))
+    _check(afb, oracle, case, f"int{bits} g{group} {m}x{n}x{k}")
+
+
 @pytest.mark.parametrize("m", [7, 16, 100])
 @pytest.mark.parametrize("bits,group", [(8, 0), (8, 128), (4, 0), (4, 128), (4, 64)])
 def test_zero_points_and_packed_layout(afb, oracle, m, bits, group):
