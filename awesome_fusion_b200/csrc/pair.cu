@@ -747,6 +747,7 @@ int pair_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, const
     const char* env = getenv("AFB_PAIR");
     const int forced = env ? atoi(env) : -1;
     if (forced == 0 || a.flags & (AFB_FLAG_C_F32 | AFB_FLAG_PREFILL_SMEM_B | AFB_FLAG_PREFILL_TMEM_A)) return AFB_OK;
+    if (forced < 0 && !fused && a.m <= 64) return AFB_OK;   // is_faster says so, too: without the plan
     if (a.group_size && ((a.flags & AFB_FLAG_GROUP_EXACT) || a.group_size % kSlab || (a.group_size & (a.group_size - 1)))) return AFB_OK;
     const uint32_t pairs = (uint32_t)ctx->sm_count / 2;
     const uint32_t ks = a.k % 128 == 0 && a.group_size % 128 == 0 ? 128 : 64, spb = (a.b_bits == 8 ? 128 : 256) / ks;
