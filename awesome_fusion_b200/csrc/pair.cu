@@ -258,7 +258,9 @@ pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
             uint32_t* word = p.counters + (2 * t + rank) * kTileWords;   // contributions, chunks taken, warps that have left
             uint32_t seen = 0;
             if (lane == 0) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(word) : "memory");
-            if (__shfl_sync(0xffffffffu, seen, 0) == parts) {
+            const bool complete = __shfl_sync(0xffffffffu, seen, 0) == parts;
+            __syncwarp();   // the other lanes' loads of the partial sums are ordered after lane 0's acquire
+            if (complete) {
                 for (;;) {
                     uint32_t chunk = 0;
                     if (lane == 0) chunk = atomicAdd(word + 1, 1u);
