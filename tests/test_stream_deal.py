@@ -17,6 +17,8 @@ def shim(tmp_path_factory):
     lib = ctypes.CDLL(out)
     lib.check_deal.argtypes = [ctypes.c_uint32] * 3
     lib.fits.argtypes = [ctypes.c_uint32] * 3
+    lib.check_waves.argtypes = [ctypes.c_uint32] * 4
+    lib.tiles_past_the_end.argtypes = [ctypes.c_uint32] * 4 + [ctypes.c_int]
     lib.check_range.argtypes = [ctypes.c_uint32] * 3 + [ctypes.POINTER(ctypes.c_uint32)]
     return lib
 
@@ -34,6 +36,13 @@ def test_sizes_of_calls(shim, tiles, blocks):
     """24576 x 512 and 25600 x 512 int4 at 17 to 32 rows, 24576 x 768, 2048 rows of 38400 x 768 and of 19456 x 768 (fewer units than
     CTAs next to whole waves: such tiles were lost), and sizes with more units than CTAs."""
     assert shim.check_deal(tiles, blocks, 148) == 0
+
+
+@pytest.mark.parametrize("tiles,blocks,sms", [(300, 4, 148), (296, 4, 148), (40, 3, 148), (9, 5, 4)])
+def test_a_wave_too_many_is_seen(shim, tiles, blocks, sms):
+    """The streaming form's walk would take tiles past the end; the check walks as it does and says so.  (The pair form's walk stops there.)"""
+    assert shim.check_waves(tiles, blocks, sms, 0) == 0 and shim.check_waves(tiles, blocks, sms, 1) != 0
+    assert shim.tiles_past_the_end(tiles, blocks, sms, 1, 0) > 0 and shim.tiles_past_the_end(tiles, blocks, sms, 1, 1) == 0
 
 
 def test_the_limit_of_the_32_bit_arithmetic(shim):
