@@ -79,7 +79,7 @@ const DeviceCtx::Workspace* workspace_for(DeviceCtx* ctx, cudaStream_t s, int* r
 bool stream_workspace(DeviceCtx* ctx, cudaStream_t s, size_t bytes, float** ws, uint32_t** counters);
 int  cuda_fail(cudaError_t e);      // records e, returns AFB_ERR_CUDA
 void count_launch(unsigned n = 1);
-void count_stream_launch();          // of the streaming form, or of the pair form in its place (counted by count_launch as well)
+void count_stream_launch();          // of the streaming form (counted by count_launch as well)
 void count_pair_launch();            // of the pair form (likewise)
 
 // Driver entry point for tensor-map encoding, fetched once through the runtime.
@@ -104,7 +104,6 @@ uint32_t pick_group_m(const afb_gemm_args& a, uint32_t m_tiles, uint32_t n_tiles
 // arguments, is the faster one and no tuning variable asks for another (*done = true, its status returned); otherwise nothing happens
 // and the caller goes on to the other forms.
 int stream_if_faster(const afb_gemm_args& a, uint32_t variant, DeviceCtx* ctx, cudaStream_t s, bool* done);
-bool stream_is_faster(const afb_gemm_args& a, uint32_t sms);   // ... than the forms with one step for all converters; the pair form left aside
 // The pair form of the prefill variant (pair.cu), for a call that resolved to it or (`fused`) for a fused launch; otherwise as above.
 int pair_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, const afb_fused_args* fused, bool* done);
 int launch_prefill_ts_tiles(const afb_gemm_args& a, DeviceCtx* ctx, uint32_t* tile_done, cudaStream_t s);

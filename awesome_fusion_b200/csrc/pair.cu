@@ -798,7 +798,6 @@ int pair_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, const
         p.act = fused->activation;
     }
     *done = true;
-    if (!fused && stream_is_faster(a, (uint32_t)ctx->sm_count)) count_stream_launch();
     CUtensorMap ta, tw;
     int rc = tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.ptr_a, a.k, a.m, (uint64_t)a.lda * 2, kSlab, p.rows / 2, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;

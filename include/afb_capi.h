@@ -344,7 +344,7 @@ int afb_probe_launch(uint32_t kind, const void* src, size_t bytes, uint32_t ctas
 int afb_phase_timestamps(unsigned long long out[8]);
 /* Number of kernels this library launched since afb_init (all variants). */
 unsigned long long afb_launch_count(void);
-/* ... and how many of them were of the streaming form of the decode and prefill variants, or of the pair form in its place */
+/* ... and how many of them were of the streaming form of the decode and prefill variants */
 unsigned long long afb_stream_launch_count(void);
 /* ... and of the pair form of the prefill variant and the fused launches */
 unsigned long long afb_pair_launch_count(void);

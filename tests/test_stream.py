@@ -164,17 +164,17 @@ def test_group_sums_are_added_in_two_levels(afb):
     assert off < 2, off
 
 
-@pytest.mark.parametrize("m,n,k,bits,group,streamed", [
-    (3, 28672, 8192, 8, 0, 0), (4, 28672, 8192, 8, 0, 1), (4, 28672, 8192, 4, 128, 0), (5, 28672, 8192, 4, 128, 1), (16, 4096, 4096, 8, 0, 0),
-    (9, 12288, 4096, 8, 0, 1), (8, 8192, 8192, 4, 0, 0), (12, 8192, 8192, 4, 0, 1), (8, 4096, 11008, 4, 128, 1), (17, 12288, 1024, 4, 128, 0),
-    (40, 16384, 2048, 4, 128, 1), (24, 4096, 4096, 4, 0, 1), (40, 4096, 4096, 4, 0, 0), (40, 4096, 4096, 8, 0, 0), (64, 12288, 4096, 8, 0, 1),
-    (80, 12288, 4096, 8, 0, 0), (128, 8192, 8192, 8, 0, 1), (129, 8192, 8192, 8, 0, 1), (200, 8192, 8192, 8, 0, 0), (129, 12288, 4096, 8, 0, 0),
-    (333, 11000, 4096, 8, 0, 1), (333, 8192, 8192, 8, 0, 0), (777, 12288, 4096, 8, 0, 0), (777, 12288, 4096, 4, 128, 1), (4096, 1024, 11008, 4, 128, 0), (40, 28672, 2048, 4, 64, 0),
-    (40, 28672, 2048, 4, 128, 1), (777, 12288, 4096, 8, 128, 1), (40, 28672, 1024, 4, 128, 0)])
-def test_choice_of_the_form(afb, monkeypatch, m, n, k, bits, group, streamed):
-    """On both sides of the lines of the automatic choice (148 SMs)."""
+@pytest.mark.parametrize("m,n,k,bits,group,form", [
+    (3, 28672, 8192, 8, 0, "other"), (4, 28672, 8192, 8, 0, "stream"), (4, 28672, 8192, 4, 128, "other"), (5, 28672, 8192, 4, 128, "stream"), (16, 4096, 4096, 8, 0, "other"),
+    (9, 12288, 4096, 8, 0, "stream"), (8, 8192, 8192, 4, 0, "other"), (12, 8192, 8192, 4, 0, "stream"), (8, 4096, 11008, 4, 128, "stream"), (17, 12288, 1024, 4, 128, "other"),
+    (40, 16384, 2048, 4, 128, "stream"), (24, 4096, 4096, 4, 0, "stream"), (40, 4096, 4096, 4, 0, "other"), (40, 4096, 4096, 8, 0, "other"), (64, 12288, 4096, 8, 0, "stream"),
+    (80, 12288, 4096, 8, 0, "pair"), (128, 8192, 8192, 8, 0, "stream"), (129, 8192, 8192, 8, 0, "stream"), (200, 8192, 8192, 8, 0, "pair"), (129, 12288, 4096, 8, 0, "pair"),
+    (333, 11000, 4096, 8, 0, "pair"), (333, 8192, 8192, 8, 0, "pair"), (777, 12288, 4096, 8, 0, "pair"), (777, 12288, 4096, 4, 128, "pair"), (4096, 1024, 11008, 4, 128, "pair"), (40, 28672, 2048, 4, 64, "other"),
+    (40, 28672, 2048, 4, 128, "stream"), (777, 12288, 4096, 8, 128, "pair"), (40, 28672, 1024, 4, 128, "other")])
+def test_choice_of_the_form(afb, monkeypatch, m, n, k, bits, group, form):
+    """On both sides of the lines of the automatic choice (148 SMs): the streaming form, the pair form, or one of the others."""
     monkeypatch.delenv("AFB_STREAM")
-    before = afb.stream_launch_count()
+    before, paired = afb.stream_launch_count(), afb.pair_launch_count()
     a, b, s, c = (afb.malloc(size) for size in (m * k * 2, n * k * bits // 8, n * (k // group if group else 1) * 4, m * n * 2))
     try:
         for p, size in ((a, m * k * 2), (b, n * k * bits // 8), (s, n * (k // group if group else 1) * 4)):
@@ -184,7 +184,7 @@ def test_choice_of_the_form(afb, monkeypatch, m, n, k, bits, group, streamed):
     finally:
         for p in (a, b, s, c):
             afb.free(p)
-    assert afb.stream_launch_count() - before == streamed
+    assert (afb.stream_launch_count() - before, afb.pair_launch_count() - paired) == {"stream": (1, 0), "pair": (0, 1), "other": (0, 0)}[form]
 
 
 def test_dependent_launches_in_a_chain(afb):
