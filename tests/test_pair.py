@@ -81,7 +81,7 @@ def test_group_scales_at_the_edges_of_the_folding(afb, oracle, forced, scales):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("share", ["0", "1"])
-@pytest.mark.parametrize("m,n,k,gated", [(1, 72, 512, True), (33, 136, 256, True), (257, 264, 1024, True), (300, 2056, 640, True), (70, 264, 320, False), (300, 4104, 512, False)])
+@pytest.mark.parametrize("m,n,k,gated", [(1, 72, 512, True), (33, 136, 256, True), (257, 264, 1024, True), (300, 2056, 640, True), (70, 264, 320, False), (300, 4104, 512, False), (257, 264, 1024, False), (129, 1000, 960, False)])
 def test_fused_epilogue(afb, oracle, forced, m, n, k, gated, share):
     """Bias, SiLU, gate * up and the residual, in place and with padded rows, in whole and in shared tiles."""
     from test_fused import silu
