@@ -104,6 +104,7 @@ uint32_t pick_group_m(const afb_gemm_args& a, uint32_t m_tiles, uint32_t n_tiles
 // arguments, is the faster one and no tuning variable asks for another (*done = true, its status returned); otherwise nothing happens
 // and the caller goes on to the other forms.
 int stream_if_faster(const afb_gemm_args& a, uint32_t variant, DeviceCtx* ctx, cudaStream_t s, bool* done);
+bool stream_is_faster(const afb_gemm_args& a, uint32_t sms);   // than the forms with one step for all converters; the pair form left aside
 // The pair form of the prefill variant (pair.cu), for a call that resolved to it or (`fused`) for a fused launch; otherwise as above.
 int pair_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, const afb_fused_args* fused, bool* done);
 int launch_prefill_ts_tiles(const afb_gemm_args& a, DeviceCtx* ctx, uint32_t* tile_done, cudaStream_t s);

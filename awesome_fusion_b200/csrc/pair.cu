@@ -698,54 +698,80 @@ int launch_cfg(const CUtensorMap& ta, const CUtensorMap& tw, const PairParams& p
 // Rows per tile, and whether the tiles that do not fill whole waves are shared: the cheapest by a count of cycles.  Per step of 128 k
 // 4 per activation row (the tensor cores) or 820 (the issuing warp; of 64 k 700); per tile 3300 until its only accumulator has been drained
 // (up to 128 rows there are two); for sharing, that is partial sums written, read and added, 120 per row (2048 x 11008 x 4096 int8 with
-// 256 rows: 131 us shared, 119 not; 128 x 28672 x 8192 int4 group-128 with 128 rows: 62 and 70).
-struct Plan { uint32_t rows; bool shared; double cycles; };
+// 256 rows: 131 us shared, 119 not; 128 x 28672 x 8192 int4 group-128 with 128 rows: 62 and 70) and 1200 per pair that shares a tile: a
+// warp adds their sums one after the other (K = 8192 int8, 65 rows: 1 tile over a wave, 64 pairs on it, 116 us shared and 71 not; 3 tiles
+// 78 and 72; 10 tiles 65 and 71).
+// useful: the share of the pairs' cycles that goes into steps.
+struct Plan { uint32_t rows, waves; bool shared; double cycles, useful; };
 Plan plan(const afb_gemm_args& a, uint32_t ks, uint32_t pairs) {
-    Plan best{0, false, 0.};
-    const uint32_t n_tiles = (a.n + 2 * kCh - 1) / (2 * kCh), steps = a.k / ks;
+    Plan best{};
+    const uint32_t n_tiles = (a.n + 2 * kCh - 1) / (2 * kCh), steps = a.k / ks, blocks = (uint32_t)(((uint64_t)a.k * a.b_bits / 8 + 127) / 128);
     const uint32_t fewest = (a.m + 255) / 256, most = fewest + 8 < (a.m + 63) / 64 ? fewest + 8 : (a.m + 63) / 64;
     for (uint32_t row_tiles = fewest; row_tiles <= most; ++row_tiles) {
         const uint32_t rows = ((a.m + row_tiles - 1) / row_tiles + 31) / 32 * 32;   // for two SMs in steps of 32
         const uint32_t tiles = (a.m + rows - 1) / rows * n_tiles, waves = tiles / pairs, rest = tiles % pairs;
         const double hand_off = ks == 128 ? 820. : 700., mma = rows * (ks / 32.);
         const double work = steps * (mma > hand_off ? mma : hand_off), tile = work + (rows > 128 ? 3300. : 0.);
-        const double whole = (waves + (rest ? 1 : 0)) * tile, split = waves * tile + work * rest / pairs + 120. * rows;
+        const double sharers = !rest ? 0. : (double)pairs / rest < blocks ? (double)pairs / rest : blocks;
+        const double whole = (waves + (rest ? 1 : 0)) * tile, split = waves * tile + work * rest / pairs + 120. * rows + 1200. * sharers;
         const bool shared = rest && split < whole;
         const double cycles = (shared ? split : whole) + 25. * rows;   // ... and the last tile's way out
-        if (!best.rows || cycles < best.cycles) best = Plan{rows, shared, cycles};
+        if (!best.rows || cycles < best.cycles) best = Plan{rows, waves, shared, cycles, tiles * work / pairs / cycles};
     }
     return best;
 }
 
-// Where this form is the faster one, from times of both on one B200 (us, the best of the other forms / this one; 17 matrices from
-// 1024 x 1024 to 28672 x 8192, 20 row counts from 65 to 4096, int8, int4, int4 in groups of 128 and 64; fused: 9 matrices, 1 to 4096 rows).
-bool is_faster(const afb_gemm_args& a, const Plan& x, uint32_t sms, bool fused) {
-    // 1000 x 2*11008 x 4096 int8: 213 / 156;  1024 x 2*2048 x 2048: 37 / 31;  16 x 2*4096 x 11008 int4 group-128: 2.5 times;  but
-    // 64 x 2*2048 x 2048 int8: 28 / 33
-    if (fused) return a.group_size || a.m > 64 || (double)a.n * a.k >= 16e6;
+// Where this form is the faster one.  The lines are drawn through the times of this form and of the one that would take the call otherwise, on
+// one B200, caches cold: 21700 sizes, K from 512 to 28672, N from 1024 to 40960, 65 to 4096 rows, int8 and int4 per channel and in groups of
+// 128 and 64.  Of the 13950 that this form takes it is the slower one by more than 6 % at 9 (by 10 % at most) and 1.22 times as fast on
+// average.  Each line names sizes on its two sides (us, the other form / this one).
+// Fused (9 matrices and 15 more with K of 512, K = 64 modulo 128 or few channels; 1 to 4096 rows):
+//   1000 x 2*11008 x 4096 int8: 213 / 156;  1024 x 2*2048 x 2048: 37 / 31;  16 x 2*4096 x 11008 int4 group-128: 2.5 times;  but
+//   64 x 2*2048 x 2048 int8: 28 / 33 (65 rows: 30 / 27);  128 x 2*4096 x 4160 int8, in steps of 64 k: 40 / 49, 2*5504 x 2112: 0.92
+bool is_faster(const afb_gemm_args& a, const Plan& x, uint32_t ks, uint32_t sms, const afb_fused_args* fused) {
+    const double weights = (double)a.n * a.k;
+    const uint32_t pairs = sms / 2, n_tiles = (a.n + 2 * kCh - 1) / (2 * kCh), tiles = (a.m + x.rows - 1) / x.rows * n_tiles;
+    if (fused) {
+        if (a.group_size) return true;
+        if (fused->gated && ks == 64 && a.m > 64 && a.m <= 128 && a.k >= 2048 && n_tiles * 2 <= pairs) return false;
+        return a.m > 64 || weights >= 16e6;
+    }
     if (a.m <= 64) return false;
-    const uint32_t tiles = (a.m + x.rows - 1) / x.rows * ((a.n + 2 * kCh - 1) / (2 * kCh)), pairs = sms / 2;
     // All tiles shared: the other forms cut the same work into smaller pieces (128 x 8192 x 8192 int8: 36 / 49; 333 x 4096 x 11008: 51 / 57).
     if (x.shared && tiles < pairs) return false;
-    if (a.group_size % 128) {
-        // Steps of 64 k, so twice the hand-offs: 300 x 28672 x 8192: 0.94; 128 x 28672 x 1024: 22 / 25; 128 x 4096 x 4096: 0.93
-        if (a.m > 256 && a.m <= 384) return (double)a.n * a.k < 40e6;
-        if (a.m <= 128) return a.k > 1536 && tiles * 2 > pairs;
+    // The streaming form shares whatever is left over a wave evenly and has less to hand off per row; what decides is how much of this form's
+    // time is steps: 128 x 22528 x 8192 int8 (0.72) 60 / 66, 24576 (0.75) 69 / 67;  192 x 19200 x 8192 (0.46) 1.20, 160 x 20736 x 8192 (0.59) 74 / 72.
+    if (a.m <= 256 && stream_is_faster(a, sms)) {
+        if (x.shared && a.b_bits == 8 && a.m <= 96) return false;   // 65 x 28672 x 8192: 66 / 68, 40960: 96 / 100
+        const double least = ks == 64 ? (a.m <= 128 ? 0.8 : 0.7) : (a.m <= 128 ? 0.74 : 0.5);
+        return !x.waves || x.useful >= least;   // 128 x 14336 x 3072 int4 group-128, one wave: 0.80
     }
-    if (a.group_size && a.b_bits == 8 && a.m <= 128) return false;             // 72 x 20000 x 2048: 27 / 35
-    if (a.k <= 1536 && a.m <= 256 && x.rows >= 224) return false;              // 256 x 11000 x 1024: 18.4 / 20.5
-    if (!a.group_size) {
-        if (x.shared && a.b_bits == 8 && a.m < 96) return false;   // 65 x 28672 x 8192: 68 / 71
-        // The 256-row form (prefill_ts.cu) has one wave of whole tiles, too, and less to set up: 1024 x 4096 x 4096: 35 / 37;
-        // 512 x 7168 x 2048: 22.5 / 24.6;  128 x 16384 x 1152: 16.4 / 18.4;  4096 x 1024 x 1024: 18.4 / 20.5
-        const uint32_t there = (a.m + 255) / 256 * ((a.n + kCh - 1) / kCh);
-        if (there > sms / 2 && there <= sms) {
-            if (a.k <= 4096 && x.rows == 256) return false;
-            if (a.k <= 2304 && x.rows >= 224 && a.m <= 512) return false;
-            if (a.k <= 1536 && (a.m <= 256 || a.m >= 2560)) return false;
+    // Short rows leave too little to gain for the longer start and way out: K = 512: 1024 x 4096 int8: 15 / 20; 2048 x 28672: 1.33; K = 896: 1.03 on
+    // average from 513 rows on; groups of 64: 1.02 and 0.87.  With steps of 64 k and without groups up to K = 2047: 1088: 1.03, 1856: 0.98.
+    // Up to 128 rows the others need two waves from 19200 channels on: 0.65 to 0.8.
+    if (a.k < (a.group_size % 128 ? 768u : 1024u) || (ks == 64 && !a.group_size && a.k < 2048)) return !a.group_size && a.m <= 128 && n_tiles > pairs;
+    if (ks == 64) {   // twice the hand-offs
+        if (a.m > 256 && a.m <= 384) return weights < 40e6;   // 300 x 28672 x 4160 int8: 86 / 94; 28672 x 4096 in groups of 64: 1.03; 8192 x 4096: 0.68
+        if (a.m <= 128) {
+            // 128 x 8192 x 2112 int8: 1.12, 19200: 44 / 37;  groups of 64: 65 x 28672 x 2304: 1.12, 11008 x 2048: 0.82, 4096 x 2048 (32 tiles): 20 / 27
+            if (!a.group_size) return n_tiles > pairs;
+            return a.k > 1536 && tiles * 2 > pairs && (n_tiles <= pairs || a.k >= 4096);
         }
     }
-    return true;
+    if (a.m <= 128 && a.k >= 3072 && tiles * 8 <= pairs) return false;         // 65 x 1024 x 3072 int4: 1.10
+    if (a.m <= 256 && a.k <= 1536 && x.rows >= 224) return false;              // 256 x 11008 x 1280: 1.10
+    if (!a.group_size && a.m > 192 && a.m <= 256 && a.k >= 3072 && x.useful < 0.5) return false;   // 256 x 19200 x 8192: 89 / 101
+    if (a.group_size % 128) return true;
+    // The form with tiles of 256 x 128 (prefill_ts.cu) starts and ends sooner.  Where those fill one or two waves well, that decides for short K.
+    const uint32_t there = (a.m + 255) / 256 * ((a.n + kCh - 1) / kCh);
+    if (there <= sms / 2 || there > 2 * sms) return true;
+    const double full = (double)a.m * a.n / (256. * kCh * sms);   // waves of it, without padding
+    if (there > sms) return a.k >= 1536 || full < 1.6;            // 2048 x 4096 x 1024 int8 (1.73): 27 / 29;  1280 x 5504 (1.45): 0.86
+    if (a.k < 1536) return full <= 0.5 && (a.group_size || a.m > 128);   // 1024 x 4096 x 1024 (0.86): 18 / 22, 384 x 7168 (0.57): 1.0, 256 x 5504 (0.29): 0.72; 128 x 14336 int4: 1.08
+    if (a.group_size || a.m <= 128 || a.k > 4096) return true;
+    if (a.m <= 256 && x.rows >= 224) return false;                // 256 x 14336 x 2048: 1.04
+    // K = 1536: 1280 x 3072 (0.81) 1.08, 384 x 7168 (0.57) 0.97;  K = 2048: 450 x 7168 (0.67) 1.06, 777 x 4096 (0.66) 0.99, K = 2112: 450 (0.38) 1.03, 640 (0.54) 0.99;  1024 x 4096 x 4096 (0.86): 35 / 37
+    return full <= (a.k < 2048 ? 0.58 : a.k < 3072 ? (ks == 64 ? 0.6 : 0.66) : 0.84);
 }
 
 // A tuning variable that asks for one of the variant's other forms, or for a shape of theirs.
@@ -767,7 +793,7 @@ int pair_if_faster(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, const
     const uint32_t pairs = (uint32_t)ctx->sm_count / 2;
     const uint32_t ks = a.k % 128 == 0 && a.group_size % 128 == 0 ? 128 : 64, spb = (a.b_bits == 8 ? 128 : 256) / ks;
     Plan chosen = plan(a, ks, pairs);
-    if (forced < 0 && (!is_faster(a, chosen, (uint32_t)ctx->sm_count, fused != nullptr) || other_form_asked())) return AFB_OK;
+    if (forced < 0 && (!is_faster(a, chosen, ks, (uint32_t)ctx->sm_count, fused) || other_form_asked())) return AFB_OK;
     if (const char* e = getenv("AFB_PAIR_ROWS")) {   // tuning aids: the most rows per tile, shared tiles or none
         const uint32_t most = (uint32_t)atoi(e), t = most >= 32 && most <= 256 ? (a.m + most - 1) / most : 0;
         if (t) chosen.rows = ((a.m + t - 1) / t + 31) / 32 * 32;

@@ -742,6 +742,8 @@ bool is_faster(const afb_gemm_args& a, uint32_t sms) {
 
 }  // namespace
 
+bool stream_is_faster(const afb_gemm_args& a, uint32_t sms) { return stream_supports(a) && is_faster(a, sms); }
+
 // A tuning variable that asks for one of the variant's other forms, or for a shape of theirs.
 static bool other_form_asked(uint32_t variant) {
     if (variant == AFB_VARIANT_PREFILL) return getenv("AFB_PREFILL_IMPL") != nullptr;

@@ -195,6 +195,64 @@ def test_variables_and_flags_that_ask_for_another_form(afb, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,bits,group,form", [
+    # up to 64 rows, all tiles shared
+    (64, 28672, 8192, 8, 0, "stream"), (65, 12288, 4096, 8, 0, "pair"), (128, 8192, 8192, 8, 0, "stream"), (333, 4096, 11008, 8, 0, "other"),
+    # against the streaming form: the share of this form's time that is steps; few rows of int8 in shared tiles
+    (128, 22528, 8192, 8, 0, "stream"), (128, 24576, 8192, 8, 0, "pair"), (192, 19200, 8192, 8, 0, "stream"), (160, 20736, 8192, 8, 0, "pair"),
+    (65, 19200, 8192, 8, 64, "stream"), (96, 28672, 8192, 8, 0, "stream"), (97, 28672, 8192, 8, 0, "pair"), (128, 14336, 3072, 4, 128, "pair"),
+    # short rows
+    (512, 1024, 896, 8, 0, "other"), (512, 1024, 1024, 8, 0, "pair"), (512, 4096, 512, 4, 64, "other"), (512, 4096, 768, 4, 64, "pair"),
+    (2048, 28672, 512, 8, 0, "other"), (128, 19200, 512, 8, 0, "pair"), (128, 18688, 512, 8, 0, "other"),
+    # steps of 64 k
+    (256, 8192, 1984, 8, 0, "other"), (256, 8192, 2112, 8, 0, "pair"), (300, 28672, 4160, 8, 0, "stream"), (300, 8192, 4160, 8, 0, "pair"),
+    (128, 8192, 2112, 8, 0, "other"), (128, 19200, 2112, 8, 0, "pair"), (128, 28672, 2048, 4, 64, "other"), (128, 11008, 2048, 4, 64, "pair"),
+    (65, 4096, 2048, 4, 64, "other"), (300, 28672, 4096, 4, 64, "stream"), (300, 8192, 4096, 4, 64, "pair"),
+    # few rows and few channels, 256 rows
+    (65, 1024, 3072, 4, 0, "other"), (65, 1024, 2048, 4, 0, "pair"), (256, 11008, 1280, 8, 0, "other"), (192, 11008, 1280, 8, 0, "pair"), (256, 19200, 8192, 8, 0, "other"),
+    # one or two waves of the 256-row form, nearly full or not
+    (2048, 4096, 1024, 8, 0, "other"), (1280, 5504, 1024, 8, 0, "pair"), (1024, 4096, 1024, 8, 0, "other"), (1024, 4096, 1024, 4, 128, "other"),
+    (512, 4096, 1024, 8, 0, "pair"), (128, 14336, 1024, 4, 0, "other"), (128, 8192, 1024, 4, 0, "pair"), (400, 7168, 1536, 8, 0, "other"),
+    (384, 7168, 1536, 8, 0, "pair"), (450, 7168, 2048, 8, 0, "other"), (777, 4096, 2048, 8, 0, "pair"), (777, 4096, 2112, 8, 0, "other"),
+    (640, 4096, 2112, 8, 0, "pair"), (1024, 4096, 4096, 8, 0, "other"), (900, 4096, 4096, 8, 0, "pair"), (256, 14336, 2048, 8, 0, "other"),
+    (1024, 4096, 4096, 4, 128, "pair")])
+def test_choice_of_the_form(afb, m, n, k, bits, group, form):
+    """On both sides of each line of the automatic choice (148 SMs)."""
+    streamed, paired = afb.stream_launch_count(), afb.pair_launch_count()
+    args, held = _zero_args(afb, m, n, k, bits, group)
+    afb.gemm_launch(args)
+    afb.device_sync()
+    for p in held:
+        afb.free(p)
+    assert (afb.stream_launch_count() - streamed, afb.pair_launch_count() - paired) == {"stream": (1, 0), "pair": (0, 1), "other": (0, 0)}[form]
+
+
+def _zero_args(afb, m, n, k, bits, group, n_out=None):
+    sizes = (m * k * 2, n * k * bits // 8, n * (k // group if group else 1) * 4, m * n * 2)
+    held = [afb.malloc(size) for size in sizes]
+    for p, size in zip(held, sizes):
+        afb.memset(p, 0, size)
+    a, b, s, c = held
+    return afb.make_args(c, a, b, s, m, n, k, ldc=n_out, bits=bits, group=group, scale_dtype=pkg.SCALE_BF16 if group else pkg.SCALE_F32), held
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,bits,group,gated,paired", [
+    (64, 2048, 2048, 8, 0, True, 0), (65, 2048, 2048, 8, 0, True, 1), (64, 2048, 2048, 4, 128, True, 1), (8, 2048, 2048, 8, 64, True, 1), (1, 11008, 4096, 8, 0, True, 1),
+    (1, 2048, 4096, 8, 0, False, 0), (1, 4096, 4096, 8, 0, False, 1), (128, 4096, 4160, 8, 0, True, 0), (129, 4096, 4160, 8, 0, True, 1),
+    (128, 5504, 2112, 8, 0, True, 1), (128, 4096, 1984, 8, 0, True, 1), (128, 4096, 4160, 8, 0, False, 1), (256, 512, 512, 8, 32, True, 0)])
+def test_choice_of_the_fused_form(afb, m, n, k, bits, group, gated, paired):
+    """The same for fused launches: this form or the tensor-memory form."""
+    before = afb.pair_launch_count()
+    args, held = _zero_args(afb, m, 2 * n if gated else n, k, bits, group, n)
+    afb.gemm_fused_launch(afb.make_fused_args(args, gated=gated, activation=pkg.ACT_SILU))
+    afb.device_sync()
+    for p in held:
+        afb.free(p)
+    assert afb.pair_launch_count() - before == paired
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k", [(512, 2048, 4096), (256, 8192, 8192), (120, 11008, 4096)])
 def test_stretches_of_k_do_not_drift(afb, monkeypatch, m, n, k):
     """One tile per pair: K is added up in two (up to 128 rows per tile) or four (up to 64) accumulators, where the other forms cut it, too.
