@@ -20,11 +20,13 @@ constexpr size_t kSplitKWorkspaceBytes = 32u << 20;
 constexpr size_t kSplitKCounters = 4096;
 constexpr int kPreallocatedWorkspaces = 8;
 constexpr size_t kMinStreamWorkspace = 4u << 20;       // of a captured graph: a power of two from here on
-constexpr size_t kMaxStreamWorkspaceTotal = 2048u << 20;   // beyond this, and beyond kMaxStreamWorkspaces, launches take another form
+constexpr size_t kMaxStreamWorkspaceTotal = 3072u << 20;   // 79 streams of 148 SMs; beyond this, and beyond kMaxStreamWorkspaces, launches take another form
 // Captured graphs whose workspaces stay theirs until afb_finalize, as streams' do.  Those of further graphs go back to the pool when the
 // graph is gone; the user object that says so costs each replay of the graph 2.5 us (16 x 22016 x 4096 int4, captured: 30.9 / 33.9 us).
 constexpr int kKeptGraphWorkspaces = 32;
-constexpr uint32_t kMaxStreamRows = 192;              // tile height of the streaming form
+// Of a stream: two partial sums per SM of a tile of 256 rows (the pair form's highest, the streaming form's is 192) x 128 channels.  A stream
+// takes it once and for both forms, so that its later launches allocate nothing.
+size_t stream_workspace_bytes(int sm_count) { return (size_t)2 * sm_count * 256 * 128 * sizeof(float); }
 constexpr uint32_t kPrefillTsMinM = 128;   // measured: above 128 activation rows the tensor-memory form is 1.3x faster, at 128 it is slower
 }  // namespace
 
@@ -121,9 +123,10 @@ bool stream_workspace(DeviceCtx* ctx, cudaStream_t s, size_t bytes, float** ws, 
     if (!capturing) id = 0;
     std::lock_guard<std::mutex> lock(g_mutex);
     // a stream's own workspace serves all its launches to come, a graph's the one at hand and those no larger
-    size_t want = (size_t)2 * ctx->sm_count * kMaxStreamRows * 128 * sizeof(float);
-    if (capturing) for (want = kMinStreamWorkspace; want < bytes;) want *= 2;
-    else if (want < bytes) want = bytes;
+    const size_t whole = stream_workspace_bytes(ctx->sm_count);
+    if (bytes > whole) return false;
+    size_t want = whole;
+    if (capturing) for (want = kMinStreamWorkspace; want < bytes;) want = want * 2 < whole ? want * 2 : whole;
     DeviceCtx::StreamWorkspace* spare = nullptr;   // smallest one with memory that is large enough
     DeviceCtx::StreamWorkspace* empty = nullptr;
     for (auto& w : ctx->stream_workspaces) {
@@ -280,7 +283,7 @@ int afb_init(int device) {
         AFB_CUDA(cudaMemset(c.workspaces[i].counters, 0, kSplitKCounters * sizeof(uint32_t)));
     }
     c.stream_counter_count = 3 * (size_t)c.sm_count;   // a launch shares fewer than two tiles per SM, of pairs of SMs fewer than one and three words a rank
-    AFB_CUDA(allocate_stream_workspace(&c, &c.stream_workspaces[0], (size_t)2 * c.sm_count * kMaxStreamRows * 128 * sizeof(float)));   // the first stream's
+    AFB_CUDA(allocate_stream_workspace(&c, &c.stream_workspaces[0], stream_workspace_bytes(c.sm_count)));   // the first stream's
     AFB_CUDA(cudaStreamCreateWithFlags(&c.clear_stream, cudaStreamNonBlocking));
     AFB_CUDA(cudaMalloc(&c.phase_ts, 8 * sizeof(unsigned long long)));
     AFB_CUDA(cudaMemset(c.phase_ts, 0, 8 * sizeof(unsigned long long)));

@@ -45,7 +45,7 @@ extern "C" {
 
 #define AFB_VARIANT_AUTO    0u /* decode for M <= 16, prefill above, naive where neither applies */
 #define AFB_VARIANT_DECODE  1u /* memory-bound small-M kernels (decode.cu or, where faster, stream.cu) */
-#define AFB_VARIANT_PREFILL 2u /* TMA + tcgen05/TMEM kernels (prefill.cu, prefill_ts.cu or stream.cu)  */
+#define AFB_VARIANT_PREFILL 2u /* TMA + tcgen05/TMEM kernels (prefill.cu, prefill_ts.cu, stream.cu or pair.cu) */
 #define AFB_VARIANT_NAIVE   3u /* one thread per output element, fp32, order of host_ref.hpp:15-24 */
 
 #define AFB_FLAG_C_F32 1u /* C is fp32 [M,N] instead of bf16: prefill variant (partial sums of a K-split) and naive variant */
@@ -134,13 +134,13 @@ int afb_device_sync(void);
  * launch, which then must not happen inside a stream capture; at most 64 streams per device, after
  * that AFB_ERR_TOO_LARGE.  A captured graph keeps using the workspace of the stream it was captured on,
  * so it must not run next to launches on that stream or to other graphs captured on it.
- * The streaming form of both variants (M >= 4 on large matrices, 17 and more rows, group-scaled int4; see
- * stream.cu) has workspaces of its own: one per stream (30 MB; afb_init allocates the first) and one per captured
- * graph (4 to 32 MB, by need): such graphs may run next to each other and to their capture stream.  The first 32 captured graphs
+ * The streaming form of both variants (stream.cu: mostly 4 to 128 rows of large matrices) and the pair form (pair.cu: mostly from 65 rows,
+ * and the fused launches) have workspaces of their own: one per stream for both (39 MB; afb_init allocates the first) and one per captured
+ * graph (4 to 39 MB, by need): such graphs may run next to each other and to their capture stream.  The first 32 captured graphs
  * keep theirs until afb_finalize; a further graph's goes back to the library when the graph and its executables are destroyed,
  * which costs its replays 2.5 us each.  (Two executables of ONE graph share its workspace; an executable
  * updated from another graph uses that graph's, which must then outlive it.)  They are allocated when first needed, also
- * inside a capture.  At most 256 and 2 GB of them per device; launches beyond that, and launches on cudaStreamPerThread, take a
+ * inside a capture.  At most 256 and 3 GB of them per device; launches beyond that, and launches on cudaStreamPerThread, take a
  * form without, whose results may differ in the order of the fp32 additions. */
 int afb_gemm_launch(const afb_gemm_args* args, void* stream);
 /* Which variant AFB_VARIANT_AUTO resolves to for these args (no launch). */

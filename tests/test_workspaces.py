@@ -197,3 +197,37 @@ def test_first_streaming_launch_next_to_a_capture_and_on_the_per_thread_stream(a
     torch.cuda.synchronize()
     assert afb.stream_launch_count() - before == 6
     assert ((g.c.float() - g.want.float()).norm() / g.want.float().norm()).item() < 1e-3   # another order of addition: a few roundings
+
+
+def test_a_stream_takes_one_workspace_for_both_forms(afb, monkeypatch):
+    """The streaming form, and the pair form with tiles of 224 and of 256 rows, its highest, share tiles on one stream: its first such launch takes
+    a workspace for all of them; the first stream finds the one that afb_init allocated."""
+    monkeypatch.setenv("AFB_PAIR_SHARE", "1")
+    monkeypatch.setenv("AFB_PAIR_ROWS", "256")
+    gemms = {}
+
+    def form_of(rows):
+        monkeypatch.setenv("AFB_PAIR", "0" if rows == 40 else "1")
+
+    for rows in (40, 224, 256):
+        form_of(rows)
+        gemms[rows] = Gemm(afb, rows, 8192, 8192, seed=rows)   # (loads the kernels, too)
+    torch.cuda.synchronize()
+    afb.finalize()
+    afb.init(0)
+
+    def taken(stream, order):
+        out = []
+        for rows in order:
+            form_of(rows)
+            streamed, paired, free = afb.stream_launch_count(), afb.pair_launch_count(), torch.cuda.mem_get_info()[0]
+            gemms[rows].launch(stream)
+            torch.cuda.synchronize()
+            out.append(free - torch.cuda.mem_get_info()[0])
+            assert (afb.stream_launch_count() - streamed, afb.pair_launch_count() - paired) == ((1, 0) if rows == 40 else (0, 1))
+            gemms[rows].check(f"{rows} rows")
+        return out
+
+    assert taken(torch.cuda.current_stream().cuda_stream, (40, 224, 256)) == [0, 0, 0]
+    first, *later = taken(_new_streams(afb, 1)[0], (40, 224, 256, 224, 40))
+    assert 0 < first <= 40 << 20 and later == [0] * 4, (first, later)
