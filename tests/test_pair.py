@@ -112,6 +112,40 @@ def test_fused_epilogue(afb, oracle, forced, m, n, k, gated, share):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,gated,share", [(33, 136, 512, True, "0"), (300, 264, 896, True, "1"), (200, 520, 640, False, "0"), (200, 520, 640, False, "1")])
+@pytest.mark.parametrize("zero_points,packed", [(False, False), (True, True)])
+@pytest.mark.parametrize("bits,group", [(8, 0), (4, 0), (4, 128), (4, 64), (8, 128), (8, 64)])
+def test_fused_epilogue_of_the_weight_formats(afb, oracle, forced, bits, group, zero_points, packed, m, n, k, gated, share):
+    """Fused launches in both steps of k (groups of 64: 64 wide), with group scales folded into the weights, zero-points and pre-packed weights."""
+    from test_fused import silu
+    from test_gpu_parity import check_close
+    forced.setenv("AFB_PAIR_SHARE", share)
+    rows = 2 * n if gated else n
+    case = T.make_case(m, rows, k, bits=bits, group=group, enc=m & 1, seed=m + bits + group, zero_points=zero_points,
+                       scale_range=(0.002, 0.01) if bits == 8 else (0.01, 0.05))
+    rng = np.random.default_rng(7)
+    bias = rng.standard_normal(rows).astype(np.float32)
+    residual = T.np_bf16_rne(rng.standard_normal((m, n), dtype=np.float32))
+    v = oracle.gemm(case, threads=8, round_w=bool(group)) + bias[None, :]
+    want = (silu(v[:, 0::2]) * v[:, 1::2] if gated else silu(v)) + T.np_bf16_to_f32(residual)
+    dc = T.DeviceCase(afb, oracle.prepack(case) if packed else case)
+    held = [afb.to_device(bias), afb.to_device(residual), afb.malloc(m * n * 2)]
+    try:
+        count = afb.pair_launch_count()
+        args = dc.args()
+        args.ptr_c, args.ldc = held[2], n
+        afb.gemm_fused_launch(afb.make_fused_args(args, gated=gated, activation=pkg.ACT_SILU, bias=held[0], residual=held[1], ld_residual=n))
+        afb.device_sync()
+        got = afb.to_host(held[2], (m, n), np.uint16)
+        assert afb.pair_launch_count() == count + 1 and afb.read_status()[0] == 0
+    finally:
+        dc.close()
+        for p in held:
+            afb.free(p)
+    check_close(oracle, want, got, f"fused int{bits} g{group} zero-points {zero_points} packed {packed} gated {gated} {m}x{n}x{k}")
+
+
+@pytest.mark.gpu
 def test_silu_over_its_range(afb, forced):
     """act(v) * 1 of values from -120 to 120, +-0, infinities and NaN against 64 bits.
     (v below -88.7, where 1 + exp(-v) overflows fp32, gives -0.)"""
