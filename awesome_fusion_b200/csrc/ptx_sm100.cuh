@@ -216,7 +216,10 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Arrives on the barrier at the same offset in the shared memory of CTA `rank` of this cluster.  What it reports is complete when it is
-// issued (tcgen05.wait, or a barrier that has been waited for), so it needs no release at cluster scope, which takes 1000 cycles.
+// issued (tcgen05.wait, or a barrier that has been waited for), and is read by tcgen05.mma in the CTA that it arrives at.  Without qualifiers
+// an arrival is a release at CTA scope; the memory model as written orders such reads only after one at cluster scope, which takes 1000
+// cycles.  This relies on what the two-SM pipelines of CUTLASS rely on: their remote arrival (ClusterBarrier::arrive with a CTA's id) is this
+// instruction, next to the same waits.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t rank) {
     asm volatile(
         "{\n\t.reg .b32 r;\n\t"
