@@ -712,7 +712,8 @@ Plan plan(const afb_gemm_args& a, uint32_t ks, uint32_t pairs) {
         const uint32_t tiles = (a.m + rows - 1) / rows * n_tiles, waves = tiles / pairs, rest = tiles % pairs;
         const double hand_off = ks == 128 ? 820. : 700., mma = rows * (ks / 32.);
         const double work = steps * (mma > hand_off ? mma : hand_off), tile = work + (rows > 128 ? 3300. : 0.);
-        const double sharers = !rest ? 0. : (double)pairs / rest < blocks ? (double)pairs / rest : blocks;
+        // (Short of a wave, whole tiles of more than 128 rows add up all of K in one accumulator; there sharing stays as cheap as its rows.)
+        const double sharers = !rest || (!waves && rows > 128) ? 0. : (double)pairs / rest < blocks ? (double)pairs / rest : blocks;
         const double whole = (waves + (rest ? 1 : 0)) * tile, split = waves * tile + work * rest / pairs + 120. * rows + 1200. * sharers;
         const bool shared = rest && split < whole;
         const double cycles = (shared ? split : whole) + 25. * rows;   // ... and the last tile's way out
@@ -723,8 +724,8 @@ Plan plan(const afb_gemm_args& a, uint32_t ks, uint32_t pairs) {
 
 // Where this form is the faster one.  The lines are drawn through the times of this form and of the one that would take the call otherwise, on
 // one B200, caches cold: 21700 sizes, K from 512 to 28672, N from 1024 to 40960, 65 to 4096 rows, int8 and int4 per channel and in groups of
-// 128 and 64.  Of the 13950 that this form takes it is the slower one by more than 6 % at 9 (by 10 % at most) and 1.22 times as fast on
-// average.  Each line names sizes on its two sides (us, the other form / this one).
+// 128 and 64.  Of the 13400 that this form takes it is the slower one by more than 6 % at 6 (by 10 % at most) and 1.23 times as fast on
+// average (with nothing to write back in L2 before: at 1 in 200, by 13 % at most, and 1.20).  Each line names sizes on its two sides (us, the other form / this one).
 // Fused (9 matrices and 15 more with K of 512, K = 64 modulo 128 or few channels; 1 to 4096 rows):
 //   1000 x 2*11008 x 4096 int8: 213 / 156;  1024 x 2*2048 x 2048: 37 / 31;  16 x 2*4096 x 11008 int4 group-128: 2.5 times;  but
 //   64 x 2*2048 x 2048 int8: 28 / 33 (65 rows: 30 / 27);  128 x 2*4096 x 4160 int8, in steps of 64 k: 40 / 49, 2*5504 x 2112: 0.92
@@ -739,6 +740,7 @@ bool is_faster(const afb_gemm_args& a, const Plan& x, uint32_t ks, uint32_t sms,
     if (a.m <= 64) return false;
     // All tiles shared: the other forms cut the same work into smaller pieces (128 x 8192 x 8192 int8: 36 / 49; 333 x 4096 x 11008: 51 / 57).
     if (x.shared && tiles < pairs) return false;
+    if (a.group_size && a.b_bits == 8 && a.m <= 128) return false;   // 65 x 19200 x 8192 in groups of 64: 1.81; 72 x 20000 x 2048: 27 / 35
     // The streaming form shares whatever is left over a wave evenly and has less to hand off per row; what decides is how much of this form's
     // time is steps: 128 x 22528 x 8192 int8 (0.72) 60 / 66, 24576 (0.75) 69 / 67;  192 x 19200 x 8192 (0.46) 1.20, 160 x 20736 x 8192 (0.59) 74 / 72.
     if (a.m <= 256 && stream_is_faster(a, sms)) {
@@ -766,12 +768,12 @@ bool is_faster(const afb_gemm_args& a, const Plan& x, uint32_t ks, uint32_t sms,
     const uint32_t there = (a.m + 255) / 256 * ((a.n + kCh - 1) / kCh);
     if (there <= sms / 2 || there > 2 * sms) return true;
     const double full = (double)a.m * a.n / (256. * kCh * sms);   // waves of it, without padding
-    if (there > sms) return a.k >= 1536 || full < 1.6;            // 2048 x 4096 x 1024 int8 (1.73): 27 / 29;  1280 x 5504 (1.45): 0.86
-    if (a.k < 1536) return full <= 0.5 && (a.group_size || a.m > 128);   // 1024 x 4096 x 1024 (0.86): 18 / 22, 384 x 7168 (0.57): 1.0, 256 x 5504 (0.29): 0.72; 128 x 14336 int4: 1.08
+    if (there > sms) return a.k >= 1536 || full < 1.5;            // 2048 x 4096 x 1024 int8 (1.73): 27 / 29, 512 x 14336 (1.51): 27 / 30;  1280 x 5504 (1.45): 0.86
+    if (a.k < 1536) return full <= 0.5 && (a.group_size || a.m > 256);   // 1024 x 4096 x 1024 (0.86): 18 / 22, 384 x 7168 (0.57): 1.0, 512 x 4096 (0.43): 0.76; 128 x 14336 int4: 1.08, 192 x 11008: 1.0
     if (a.group_size || a.m <= 128 || a.k > 4096) return true;
-    if (a.m <= 256 && x.rows >= 224) return false;                // 256 x 14336 x 2048: 1.04
-    // K = 1536: 1280 x 3072 (0.81) 1.08, 384 x 7168 (0.57) 0.97;  K = 2048: 450 x 7168 (0.67) 1.06, 777 x 4096 (0.66) 0.99, K = 2112: 450 (0.38) 1.03, 640 (0.54) 0.99;  1024 x 4096 x 4096 (0.86): 35 / 37
-    return full <= (a.k < 2048 ? 0.58 : a.k < 3072 ? (ks == 64 ? 0.6 : 0.66) : 0.84);
+    if (x.rows == 256 || (a.m <= 256 && x.rows >= 224)) return false;   // 1024 x 4096 x 4096: 35 / 37, 512 x 8192 x 3072: 1.02;  224 x 14336 x 2048: 1.01
+    // K = 1536: 1280 x 3072 (0.81) 1.08, 384 x 7168 (0.57) 0.97;  K = 2048: 450 x 7168 (0.67) 1.06, 777 x 4096 (0.66) 0.99, K = 2112: 450 (0.38) 1.03, 640 (0.54) 0.99
+    return a.k >= 3072 || full <= (a.k < 2048 ? 0.58 : ks == 64 ? 0.6 : 0.66);
 }
 
 // A tuning variable that asks for one of the variant's other forms, or for a shape of theirs.

@@ -243,12 +243,12 @@ def test_variables_and_flags_that_ask_for_another_form(afb, monkeypatch):
     (128, 8192, 2112, 8, 0, "other"), (128, 19200, 2112, 8, 0, "pair"), (128, 28672, 2048, 4, 64, "other"), (128, 11008, 2048, 4, 64, "pair"),
     (65, 4096, 2048, 4, 64, "other"), (300, 28672, 4096, 4, 64, "stream"), (300, 8192, 4096, 4, 64, "pair"),
     # few rows and few channels, 256 rows
-    (65, 1024, 3072, 4, 0, "other"), (65, 1024, 2048, 4, 0, "pair"), (256, 11008, 1280, 8, 0, "other"), (192, 11008, 1280, 8, 0, "pair"), (256, 19200, 8192, 8, 0, "other"),
+    (65, 1024, 3072, 4, 0, "other"), (65, 1024, 2048, 4, 0, "pair"), (256, 11008, 1536, 8, 0, "other"), (192, 11008, 1536, 8, 0, "pair"), (256, 19200, 8192, 8, 0, "other"),
     # one or two waves of the 256-row form, nearly full or not
-    (2048, 4096, 1024, 8, 0, "other"), (1280, 5504, 1024, 8, 0, "pair"), (1024, 4096, 1024, 8, 0, "other"), (1024, 4096, 1024, 4, 128, "other"),
+    (2048, 4096, 1024, 8, 0, "other"), (512, 14336, 1024, 8, 0, "other"), (1280, 5504, 1024, 8, 0, "pair"), (1024, 4096, 1024, 8, 0, "other"), (1024, 4096, 1024, 4, 128, "other"),
     (512, 4096, 1024, 8, 0, "pair"), (128, 14336, 1024, 4, 0, "other"), (128, 8192, 1024, 4, 0, "pair"), (400, 7168, 1536, 8, 0, "other"),
     (384, 7168, 1536, 8, 0, "pair"), (450, 7168, 2048, 8, 0, "other"), (777, 4096, 2048, 8, 0, "pair"), (777, 4096, 2112, 8, 0, "other"),
-    (640, 4096, 2112, 8, 0, "pair"), (1024, 4096, 4096, 8, 0, "other"), (900, 4096, 4096, 8, 0, "pair"), (256, 14336, 2048, 8, 0, "other"),
+    (640, 4096, 2112, 8, 0, "pair"), (1024, 4096, 4096, 8, 0, "other"), (777, 4096, 4096, 8, 0, "pair"), (256, 14336, 2048, 8, 0, "other"),
     (1024, 4096, 4096, 4, 128, "pair")])
 def test_choice_of_the_form(afb, m, n, k, bits, group, form):
     """On both sides of each line of the automatic choice (148 SMs)."""
