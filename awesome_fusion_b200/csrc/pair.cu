@@ -27,6 +27,8 @@
 // Measured (one B200, caches cold between passes, the forms before / this one): 4096 x 28672 x 8192 int4 group-128 1909 / 1380 us, 2048 x
 // 11008 x 4096 int8 165 / 150, 128 x 28672 x 8192 int4 79 / 71, gated 1000 x 2*11008 x 4096 int8 224 / 179.  The tensor pipe is now fed as fast as
 // it goes in the main loop of 256-row tiles (1036 cycles per 128 k); the clock (1.5 to 1.6 GHz under the power limit) and the last wave set the rest.
+// ptxas spills 96 to 140 bytes in the instances without fused epilogue, whose epilogue holds 64 registers of results once per tile, and 24 to
+// 132 in the others.
 #include <cstdlib>
 #include "dequant.cuh"
 #include "stream_common.cuh"

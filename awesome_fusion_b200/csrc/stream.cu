@@ -683,21 +683,24 @@ uint32_t tile_rows(const afb_gemm_args& a) {
     return ((a.m + tiles - 1) / tiles + 15) / 16 * 16;
 }
 
-// Where this form is the faster one (of the forms with one SM per tile: pair.cu is asked before), from times of both forms on one B200 (us, the other form / this one): 23 matrices from 1024 x 1024
-// to 28672 x 8192, 35 row counts from 4 to 4096, int8, int4, int4 in groups of 128 and 64, int8 in groups of 128.  At none of those that it takes is this form more than 4 %
-// the slower one.
+// Where this form is the faster one (of the forms with one SM per tile: pair.cu is asked before), from times of both forms on one B200 (us, the
+// other form / this one): 23 matrices from 1024 x 1024 to 28672 x 8192, 35 row counts from 4 to 4096, int8, int4, int4 in groups of 128 and 64,
+// int8 in groups of 128.  At none of those that it takes is this form more than 4 % the slower one (20 matrices again up to 16 rows, caches cold,
+// with two issuing warps; of int4 in groups of 256 at one: 8 x 8192 x 8192, 25 / 27).
 bool is_faster(const afb_gemm_args& a, uint32_t sms) {
     const double weights = (double)a.n * a.k, mbytes = weights * a.b_bits / 8 / 1e6;
     const uint32_t n_tiles = (a.n + kCh - 1) / kCh;
     if (a.m <= 16) {
         // The decode kernel has about 9 us less to set up and finish, and its arithmetic grows with M; this form's does not.
-        //   28672 x 8192 int8   M = 2: 44 / 44   4: 51 / 44    8: 68 / 44   16: 64 / 45
-        //   28672 x 8192 int4   M = 4: 53 / 50   5: 57 / 50    8: 64 / 50   16: 63 / 50    (group 128; without groups 4: 45 / 50   5: 50 / 50)
-        //   12288 x 4096 int8   M = 8: 21 / 22  16: 27 / 22;   4096 x 4096: never
+        //   28672 x 8192 int8   M = 2: 49 / 47   4: 56 / 46    8: 72 / 46   16: 69 / 47
+        //   28672 x 8192 int4   M = 4: 60 / 49   5: 66 / 50    8: 68 / 50   16: 69 / 51    (group 128; without groups 4: 43 / 43   5: 45 / 43)
+        //   12288 x 4096 int8   M = 4: 23 / 23   9: 29 / 23   16: 32 / 24;   4096 x 4096   M = 4: 12 / 19   16: 16 / 19
+        // The lines date from when one warp issued both parts of a step; with two this form is the faster one below some of them, too (12288 x
+        // 4096 int8 M = 8: 28 / 24;  4096 x 11008 int8 M = 5: 23 / 23;  1024 x 11008 int8 M = 9: 43 / 19).
         if (mbytes >= 100) return a.m >= (a.b_bits == 8 ? 4u : 5u);
         // Long rows: the decode kernel stages the activations in several passes.  Without groups its int4 arithmetic is so much
         // cheaper that this must cost it more, more than 192 KiB of activations:
-        //   4096 x 11008 int4   M = 8: 30 / 21 (group 128)   8: 20 / 22   9: 34 / 22 (no groups);   8192 x 8192 int4   M = 9: 20 / 22   12: 25 / 22
+        //   4096 x 11008 int4   M = 8: 43 / 24 (group 128)   8: 31 / 23   9: 49 / 23 (no groups);   8192 x 8192 int4   M = 8: 21 / 25   12: 39 / 25
         if (a.k >= 8192 && mbytes >= 20) return a.m >= 8 && (a.b_bits == 8 || a.group_size || a.m * a.k >= 98304);
         return mbytes >= 40 && a.m >= 9;
     }
