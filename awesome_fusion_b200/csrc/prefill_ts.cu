@@ -832,7 +832,8 @@ int launch_ts_cfg(const afb_gemm_args& a, DeviceCtx* ctx, cudaStream_t s, uint32
     {
         const char* e = getenv("AFB_PREFILL_TILE_STORE");   // tuning aid: 0 switches it off
         const bool wanted = !(e && atoi(e) == 0);
-        if (wanted && !(a.flags & AFB_FLAG_C_F32) && !tile_done && !push && a.ldc % 8 == 0 && (uintptr_t)a.ptr_c % 16 == 0 &&
+        // A tile store is clipped at the edge of C to whole 16 bytes: a gated result of 4 modulo 8 columns would overwrite 4 behind each row.
+        if (wanted && !(a.flags & AFB_FLAG_C_F32) && !tile_done && !push && a.ldc % 8 == 0 && (uintptr_t)a.ptr_c % 16 == 0 && (gated ? a.n / 2 : a.n) % 8 == 0 &&
             ts_tmap_2d(&tc, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.ptr_c, gated ? a.n / 2 : a.n, a.m, (uint64_t)a.ldc * 2, gated ? 16 : 32, 32, CU_TENSOR_MAP_SWIZZLE_NONE) == AFB_OK)
             p.c_tma = 1;
     }

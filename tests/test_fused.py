@@ -127,3 +127,28 @@ def test_in_place_residual_and_padded_rows(afb, oracle, monkeypatch, m, n, gated
             afb.free(p)
     check_close(oracle, want, np.ascontiguousarray(got[:, :n]), f"in-place residual gated={gated} {m}x{n}")
     assert np.array_equal(got[:, n:], before[:, n:])
+
+
+@pytest.mark.parametrize("m,n", [(257, 132), (64, 76), (1, 4), (300, 260)])
+@pytest.mark.parametrize("pair", ["0", "1"])
+def test_gated_results_that_end_inside_16_bytes(afb, oracle, monkeypatch, m, n, pair):
+    """A number of columns that is 4 modulo 8: what lies behind each row of C, and behind its last, stays as it was.  Both forms."""
+    monkeypatch.setenv("AFB_PAIR", pair)
+    case = T.make_case(m, 2 * n, 512, seed=m + n, scale_range=(0.002, 0.01))
+    v = oracle.gemm(case, threads=8)
+    ldc = n + 12
+    before = T.np_bf16_rne(np.random.default_rng(9).standard_normal((m + 1, ldc), dtype=np.float32))
+    want = silu(v[:, 0::2]) * v[:, 1::2] + T.np_bf16_to_f32(before[:m, :n])
+    d_a, d_b, d_s, d_c = (afb.to_device(x) for x in (case.a, case.b, case.scale, before))
+    try:
+        count = afb.pair_launch_count()
+        args = afb.make_args(d_c, d_a, d_b, d_s, m, 2 * n, 512, ldc=ldc)
+        afb.gemm_fused_launch(afb.make_fused_args(args, gated=True, activation=pkg.ACT_SILU, residual=d_c, ld_residual=ldc))
+        afb.device_sync()
+        got = afb.to_host(d_c, (m + 1, ldc), np.uint16)
+        assert afb.pair_launch_count() - count == int(pair)
+    finally:
+        for p in (d_a, d_b, d_s, d_c):
+            afb.free(p)
+    check_close(oracle, want, np.ascontiguousarray(got[:m, :n]), f"gated {m}x{n} AFB_PAIR={pair}")
+    assert np.array_equal(got[:m, n:], before[:m, n:]) and np.array_equal(got[m], before[m])
